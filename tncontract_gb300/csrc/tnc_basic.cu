@@ -300,33 +300,89 @@ __global__ void trunc_rank_kernel(int64_t n, const R* __restrict__ s, int64_t ch
   if (threadIdx.x == 0) { *kout = k; *disc = acc; }
 }
 
-// out = sum_p A[p][l][r] * W[po][p][wl][wr] with the fused bond layout
-template <typename T>
-__global__ void mps_mpo_site_kernel(int64_t din, int64_t dout, int64_t chl, int64_t chr, int64_t Dl,
-                                    int64_t Dr, const T* __restrict__ A, const T* __restrict__ W,
-                                    T* __restrict__ out, int layout) {
-  const int64_t L = chl * Dl, Rr = chr * Dr;
-  const int64_t total = dout * L * Rr;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t po, li, ri;
-    if (layout == 1) {  // (phys, left, right)
-      po = e / (L * Rr);
-      int64_t rem = e - po * L * Rr;
-      li = rem / Rr;
-      ri = rem - li * Rr;
-    } else {            // (left, physout, right)
-      li = e / (dout * Rr);
-      int64_t rem = e - li * dout * Rr;
-      po = rem / Rr;
-      ri = rem - po * Rr;
-    }
-    const int64_t l = li / Dl, wl = li - l * Dl;
-    const int64_t r = ri / Dr, wr = ri - r * Dr;
-    T acc = zero_<T>();
-    for (int64_t p = 0; p < din; ++p)
-      fma_(acc, A[(p * chl + l) * chr + r], W[((po * din + p) * Dl + wl) * Dr + wr]);
-    out[e] = acc;
+// out = sum_p A[p][l][r] * W[po][p][wl][wr] with the fused bond layout.
+// Bound by HBM: every A element becomes dout Dl Dr outputs, written once.  A
+// CTA takes one left index l and a range of output columns c = r Dr + wr; a
+// thread keeps its column's din values of A in registers, splits c once (one
+// 32-bit division) and writes the column's element of all dout Dl output rows,
+// so stores stay coalesced along c and W is read from shared memory.  (One
+// thread per output element spent its time in three 64-bit divisions each:
+// float32, chi = 512, D = 5, d = 2, 52 MB out a site: 118 us, now 22.)
+// W beyond kSiteSmem is read through the cache instead; DIN = 0 keeps A's
+// values out of registers for din > 4.
+constexpr size_t kSiteSmem = 32 * 1024;
+constexpr int kSiteThreads = 128;
+constexpr int64_t kSiteCtas = 152 * 16;  // a full chip; a CTA then takes several left indices with W staged once
+
+template <typename T, int DIN>
+__global__ void __launch_bounds__(kSiteThreads)
+mps_mpo_site_kernel(int din_, int dout, int64_t chl, int64_t chr, int Dl, int Dr, const T* __restrict__ A,
+                    const T* __restrict__ W, T* __restrict__ out, int layout, int stage) {
+  extern __shared__ __align__(16) unsigned char site_smem[];
+  const int din = DIN ? DIN : din_;
+  const int64_t Rr = chr * Dr, rows = chl * Dl;
+  const T* w = W;
+  if (stage) {
+    T* sw = reinterpret_cast<T*>(site_smem);
+    const int nw = dout * din * Dl * Dr;
+    for (int i = threadIdx.x; i < nw; i += kSiteThreads) sw[i] = W[i];
+    __syncthreads();
+    w = sw;
   }
+  const int64_t plane = chl * chr;
+  for (int64_t l = blockIdx.y; l < chl; l += gridDim.y) {
+    for (int64_t c = (int64_t)blockIdx.x * kSiteThreads + threadIdx.x; c < Rr; c += (int64_t)gridDim.x * kSiteThreads) {
+      const int64_t r = Rr <= 0xffffffffLL ? (int64_t)((unsigned)c / (unsigned)Dr) : c / Dr;
+      const int wr = (int)(c - r * Dr);
+      const T* a = A + l * chr + r;
+      T av[DIN ? DIN : 1];
+      if (DIN) {
+#pragma unroll
+        for (int p = 0; p < DIN; ++p) av[p] = a[p * plane];
+      }
+      for (int po = 0; po < dout; ++po) {
+        const T* wp = w + (int64_t)po * din * Dl * Dr + wr;
+        // row of (left, wl, po): layout 0 (left, physout, right), layout 1 (phys, left, right)
+        T* o = out + (layout == 1 ? (int64_t)po * rows + l * Dl : l * Dl * dout + po) * Rr + c;
+        const int64_t step = (layout == 1 ? 1 : dout) * Rr;
+#pragma unroll 4
+        for (int wl = 0; wl < Dl; ++wl) {
+          T acc = zero_<T>();
+          if (DIN) {
+#pragma unroll
+            for (int p = 0; p < DIN; ++p) fma_(acc, av[p], wp[((int64_t)p * Dl + wl) * Dr]);
+          } else {
+            for (int p = 0; p < din; ++p) fma_(acc, a[p * plane], wp[((int64_t)p * Dl + wl) * Dr]);
+          }
+          o[wl * step] = acc;
+        }
+      }
+    }
+  }
+}
+
+template <typename T>
+static int mps_mpo_site_launch(int64_t din, int64_t dout, int64_t chl, int64_t chr, int64_t Dl, int64_t Dr, const T* A,
+                               const T* W, T* out, int layout, cudaStream_t st) {
+  if (din > 0x7fffffff || dout > 0x7fffffff || Dl > 0x7fffffff || Dr > 0x7fffffff) return TNC_ERR_ARG;
+  const double nw = (double)dout * din * Dl * Dr;
+  const size_t bytes = nw * sizeof(T) <= (double)kSiteSmem ? (size_t)nw * sizeof(T) : 0;
+  const int64_t Rr = chr * Dr;
+  // columns across x, left indices across y; both strided, so any size fits
+  int64_t gx = (Rr + kSiteThreads - 1) / kSiteThreads;
+  if (gx > 4096) gx = 4096;
+  int64_t gy = (kSiteCtas + gx - 1) / gx;
+  if (gy > chl) gy = chl;
+  const dim3 grid((unsigned)gx, (unsigned)gy);
+#define TNC_SITE(D)                                                                                                \
+  mps_mpo_site_kernel<T, D><<<grid, kSiteThreads, bytes, st>>>((int)din, (int)dout, chl, chr, (int)Dl, (int)Dr, A, \
+                                                                W, out, layout, bytes ? 1 : 0)
+  if (din == 2) TNC_SITE(2);
+  else if (din == 3) TNC_SITE(3);
+  else if (din == 4) TNC_SITE(4);
+  else TNC_SITE(0);
+#undef TNC_SITE
+  return launch_status();
 }
 
 template <typename T>
@@ -510,10 +566,9 @@ int tnc_mps_mpo_site(int dtype, int64_t din, int64_t dout, int64_t chl, int64_t 
   if (din <= 0 || dout <= 0 || chl <= 0 || chr <= 0 || Dl <= 0 || Dr <= 0 || (layout != 0 && layout != 1))
     return TNC_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  int64_t total = dout * chl * Dl * chr * Dr;
-  TNC_DISPATCH(dtype, T, mps_mpo_site_kernel<T><<<grid1d(total, 256), 256, 0, st>>>(
-                             din, dout, chl, chr, Dl, Dr, (const T*)A, (const T*)W, (T*)out, layout));
-  return launch_status();
+  TNC_DISPATCH(dtype, T,
+               return mps_mpo_site_launch<T>(din, dout, chl, chr, Dl, Dr, (const T*)A, (const T*)W, (T*)out, layout, st));
+  return TNC_ERR_ARG;
 }
 
 }  // extern "C"
