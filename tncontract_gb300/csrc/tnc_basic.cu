@@ -16,7 +16,8 @@ struct PermParams {
   int64_t in_stride_of_out[8];  // input stride of output axis i
 };
 
-// Generic gather: one thread per output element (coalesced writes).
+// Generic gather: one thread per output element (coalesced writes).  Only for
+// tensors of 2^31 elements or more; below, permute_blocked moves them.
 template <typename T, bool CONJ>
 __global__ void permute_gather(const T* __restrict__ src, T* __restrict__ dst,
                                PermParams p, int64_t total) {
@@ -33,6 +34,178 @@ __global__ void permute_gather(const T* __restrict__ src, T* __restrict__ dst,
     T v = src[off];
     dst[o] = CONJ ? conj_(v) : v;
   }
+}
+
+// Blocked permute for small inner axes (a fused MPO bond of 2 or 3 next to a
+// long one), where a 32 x 32 tile of two axes would be mostly empty, and for
+// kept inner axes.  A block is a box of the tensor that holds at least kRun
+// elements contiguous in the input and at least kRun contiguous in the output
+// (as many whole fast axes of each side as that takes, the last one cut): it
+// is read along the input's order into shared memory and written along the
+// output's.  Bound by HBM; indices are 32-bit, split by multiply-high.
+// complex64 (256, 3, 256, 2)-like moves of an environment update: 200 us each
+// as 32 x 32 tiles with two lanes in 32 at work, 6 us here.
+struct FastDiv {
+  unsigned d, m, s;  // q = (umulhi(n, m) + n) >> s for n < 2^31 (Granlund and Montgomery 1994)
+};
+static FastDiv fast_div(unsigned d) {
+  FastDiv f;
+  f.d = d;
+  unsigned s = 0;
+  while ((1ull << s) < d) ++s;
+  f.s = s;
+  f.m = (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+  return f;
+}
+__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) {
+  return (unsigned)(((unsigned long long)__umulhi(n, f.m) + n) >> f.s);
+}
+
+struct BlockParams {
+  int rank;                // axes in output order, slowest first
+  int dims[8];             // their sizes
+  unsigned istr[8], ostr[8];  // input / output strides
+  int blk[8];              // box sizes
+  FastDiv tiles[8];        // boxes along each axis
+  int nin, nout;           // axes of the box (size > 1), fastest first in input / output order
+  int in_axis[8], out_axis[8];
+  FastDiv in_div[8], out_div[8];
+  int pitch[8];            // shared-memory stride of every axis
+  int count;               // elements of a box
+};
+
+template <typename T, bool CONJ>
+__global__ void __launch_bounds__(256) permute_blocked(const T* __restrict__ src, T* __restrict__ dst,
+                                                       const __grid_constant__ BlockParams p) {
+  extern __shared__ __align__(16) unsigned char perm_smem[];
+  T* box = reinterpret_cast<T*>(perm_smem);
+  int lo[8];
+  unsigned in0 = 0, out0 = 0, rem = blockIdx.x;
+#pragma unroll
+  for (int i = 7; i >= 0; --i) {
+    lo[i] = 0;
+    if (i < p.rank) {
+      const unsigned q = fdiv(rem, p.tiles[i]);
+      lo[i] = (int)(rem - q * p.tiles[i].d) * p.blk[i];
+      rem = q;
+      in0 += lo[i] * p.istr[i];
+      out0 += lo[i] * p.ostr[i];
+    }
+  }
+  __shared__ int left[8];  // of each axis, from the box's corner
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i < p.rank) left[i] = p.dims[i] - lo[i];
+  }
+  __syncthreads();
+  for (unsigned e = threadIdx.x; e < (unsigned)p.count; e += 256) {
+    unsigned r = e, off = in0, at = 0;
+    bool ok = true;
+    for (int j = 0; j < p.nin; ++j) {
+      const int a = p.in_axis[j];
+      const unsigned q = fdiv(r, p.in_div[j]);
+      const unsigned c = r - q * p.in_div[j].d;
+      r = q;
+      ok = ok && (int)c < left[a];
+      off += c * p.istr[a];
+      at += c * p.pitch[a];
+    }
+    if (ok) box[at] = src[off];
+  }
+  __syncthreads();
+  for (unsigned e = threadIdx.x; e < (unsigned)p.count; e += 256) {
+    unsigned r = e, off = out0, at = 0;
+    bool ok = true;
+    for (int j = 0; j < p.nout; ++j) {
+      const int a = p.out_axis[j];
+      const unsigned q = fdiv(r, p.out_div[j]);
+      const unsigned c = r - q * p.out_div[j].d;
+      r = q;
+      ok = ok && (int)c < left[a];
+      off += c * p.ostr[a];
+      at += c * p.pitch[a];
+    }
+    if (ok) {
+      const T v = box[at];
+      dst[off] = CONJ ? conj_(v) : v;
+    }
+  }
+}
+
+// od / os: output axes' sizes and input strides (merged, rank r >= 1), total
+// below 2^31 elements.
+template <typename T>
+static int permute_blocked_launch(const T* src, T* dst, int r, const int64_t* od, const int64_t* os, int conj,
+                                  cudaStream_t st) {
+  constexpr int kRun = sizeof(T) >= 16 ? 16 : 32;
+  BlockParams p;
+  p.rank = r;
+  int64_t s = 1;
+  int by_input[8];  // axes by input stride, fastest first
+  for (int i = r - 1; i >= 0; --i) {
+    p.dims[i] = (int)od[i];
+    p.istr[i] = (unsigned)os[i];
+    p.ostr[i] = (unsigned)s;
+    s *= od[i];
+    p.blk[i] = 1;
+    by_input[i] = i;
+  }
+  for (int i = 0; i < r; ++i)
+    for (int j = i + 1; j < r; ++j)
+      if (os[by_input[j]] < os[by_input[i]]) { const int t = by_input[i]; by_input[i] = by_input[j]; by_input[j] = t; }
+  auto grow = [&](const int* order, int first, int step, int want) {
+    int n = 1;
+    for (int k = 0; k < r && n < want; ++k) {
+      const int a = order ? order[k] : first + step * k;
+      int b = (want + n - 1) / n;
+      if (b > p.dims[a]) b = p.dims[a];
+      if (p.blk[a] < b) p.blk[a] = b;
+      n *= p.blk[a];
+      if (p.blk[a] < p.dims[a]) break;  // a cut axis ends the contiguous run
+    }
+  };
+  grow(by_input, 0, 0, kRun);
+  grow(nullptr, r - 1, -1, kRun);
+  // a box of few elements (an inner axis that both sides share) takes more of
+  // the output's run: 256 threads, a few elements each
+  p.count = 1;
+  for (int i = 0; i < r; ++i) p.count *= p.blk[i];
+  for (int i = r - 1; i >= 0 && p.count < 1024; --i) {
+    int b = 1024 / (p.count / p.blk[i]);
+    if (b > p.dims[i]) b = p.dims[i];
+    if (b > p.blk[i]) { p.count = p.count / p.blk[i] * b; p.blk[i] = b; }
+  }
+  int64_t boxes = 1;
+  for (int i = 0; i < r; ++i) {
+    const int64_t t = (p.dims[i] + p.blk[i] - 1) / p.blk[i];
+    p.tiles[i] = fast_div((unsigned)t);
+    boxes *= t;
+  }
+  // shared layout: input order, the rows after the input's contiguous run on
+  // an odd pitch, so a column read hits distinct banks
+  p.nin = p.nout = 0;
+  int pitch = 1;
+  bool padded = false;
+  for (int k = 0; k < r; ++k) {
+    const int a = by_input[k];
+    p.pitch[a] = pitch;
+    if (p.blk[a] == 1) continue;
+    p.in_axis[p.nin] = a;
+    p.in_div[p.nin++] = fast_div((unsigned)p.blk[a]);
+    pitch *= p.blk[a];
+    if (!padded && pitch >= 16) { pitch |= 1; padded = true; }
+  }
+  for (int i = r - 1; i >= 0; --i) {
+    if (p.blk[i] == 1) continue;
+    p.out_axis[p.nout] = i;
+    p.out_div[p.nout++] = fast_div((unsigned)p.blk[i]);
+  }
+  const size_t smem = (size_t)pitch * sizeof(T);
+  if (smem > 48 * 1024 || boxes > 0x7fffffff) return TNC_ERR_TOO_LARGE;
+  if (conj) permute_blocked<T, true><<<(unsigned)boxes, 256, smem, st>>>(src, dst, p);
+  else permute_blocked<T, false><<<(unsigned)boxes, 256, smem, st>>>(src, dst, p);
+  return launch_status();
 }
 
 // Tiled transpose for permutations that move the input's innermost axis:
@@ -134,7 +307,17 @@ static int permute_impl(const T* src, T* dst, int rank, const int64_t* shape,
                  ? TNC_OK : TNC_ERR_CUDA;
     }
   }
-  if (inner_kept || r == 1) {
+  int pb = -1;  // the output axis that is the input's innermost
+  for (int i = 0; i < r; ++i) if (os[i] == 1) pb = i;
+  if (pb < 0) return TNC_ERR_ARG;
+  // A kept inner axis, or a transposed pair of which one is short (the 32 x 32
+  // tile wastes half its lanes below 17), moves in boxes
+  const bool narrow = inner_kept || od[r - 1] <= 16 || od[pb] <= 16;
+  if (narrow && total < (1LL << 31)) {
+    const int rc = permute_blocked_launch<T>(src, dst, r, od, os, conj && traits<T>::is_complex, st);
+    if (rc != TNC_ERR_TOO_LARGE) return rc;
+  }
+  if (inner_kept) {
     PermParams p;
     p.rank = r;
     for (int i = 0; i < r; ++i) { p.out_dims[i] = od[i]; p.in_stride_of_out[i] = os[i]; }
@@ -145,9 +328,6 @@ static int permute_impl(const T* src, T* dst, int rank, const int64_t* shape,
   }
   // tiled transpose: output axis r-1 (input stride os[r-1]) and the output
   // axis whose input stride is 1
-  int pb = -1;
-  for (int i = 0; i < r; ++i) if (os[i] == 1) pb = i;
-  if (pb < 0) return TNC_ERR_ARG;
   int64_t ostr[8];
   {
     int64_t s = 1;
