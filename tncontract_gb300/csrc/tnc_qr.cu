@@ -1,45 +1,29 @@
 // Reduced QR (np.linalg.qr(mode="reduced") in tensor_qr, tncontract/tensor.py:1044).
 //
 // Householder QR in LAPACK's convention (geqrf + ungqr: Q = H_0 ... H_{k-1},
-// H_c = I - tau_c v_c v_c^H, v_c[c] = 1, R's diagonal real for complex input),
-// run as ONE cooperative persistent launch organised as a column-owner
-// dataflow: every column of A is owned by one warp; reflector c is published
-// (with a flag) by the owner of column c as soon as reflectors 0..c-1 have
-// been applied to that column, and each warp applies the published
-// reflectors to its own columns in order.  The owner of column c+1 applies
-// reflector c to that column first and publishes reflector c+1 before
-// touching its other columns (look-ahead), which keeps the critical path at
-// one column update + one reflector per step.  No grid-wide barrier is needed.
+// H_c = I - tau_c v_c v_c^H, v_c[c] = 1, R's diagonal real for complex input).
+// Up to kQrPanelRows rows it runs in panels (tnc_qr_block.cuh): one cluster
+// factors a panel and forms its block reflector's T, one launch applies it to
+// the remaining columns, and Q is formed by the same block reflectors in
+// reverse.  Longer matrices run the general kernels below: a cooperative
+// column-owner dataflow, where every column of A is owned by one warp;
+// reflector c is published (with a flag) by the owner of column c as soon as
+// reflectors 0..c-1 have been applied to that column, and each warp applies
+// the published reflectors to its own columns in order, the owner of column
+// c+1 first (look-ahead).
 //
 // Working layout: Bt = A^T (row c of Bt is column c of A, contiguous), so
 // every warp streams its own column and the published reflector with
-// coalesced loads.  Q is formed by backward accumulation, each warp applying
-// H_{min(j,k-1)} ... H_0 to its own column e_j -- independent across warps.
+// coalesced loads.
 #include "tnc_persist.cuh"
+#include "tnc_qr_block.cuh"
 
 #include <atomic>
+#include <type_traits>
 
 namespace tnc {
 
 constexpr int kQrWarps = 4;  // warps per CTA
-
-template <typename T>
-__device__ __forceinline__ T div_(T a, T b);
-template <> __device__ __forceinline__ float div_(float a, float b) { return a / b; }
-template <> __device__ __forceinline__ double div_(double a, double b) { return a / b; }
-template <typename R>
-__device__ __forceinline__ cplx<R> div_c(cplx<R> a, cplx<R> b) {
-  R d = b.re * b.re + b.im * b.im;
-  return cplx<R>((a.re * b.re + a.im * b.im) / d, (a.im * b.re - a.re * b.im) / d);
-}
-template <> __device__ __forceinline__ c64 div_(c64 a, c64 b) { return div_c(a, b); }
-template <> __device__ __forceinline__ c128 div_(c128 a, c128 b) { return div_c(a, b); }
-
-// CTA-local barrier over the first `count` threads' warps (count a multiple of
-// 32), id 1..15 (0 is __syncthreads)
-__device__ __forceinline__ void named_barrier(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
 
 template <typename T> __device__ __forceinline__ typename traits<T>::real imag_(T v) {
   if constexpr (traits<T>::is_complex) return v.im; else return 0;
@@ -59,8 +43,8 @@ __device__ void make_reflector(T* col, int64_t c, int64_t m, T* tau_out) {
     R ar = real_(alpha);
     R beta = -copysign(sqrt(abs2_(alpha) + xn), ar);
     T betaT = from_real<T>(beta);
-    tau = div_(betaT - alpha, betaT);
-    T scal = div_(one_<T>(), alpha - betaT);
+    tau = qr_div<T>(betaT - alpha, betaT);
+    T scal = qr_div<T>(one_<T>(), alpha - betaT);
     for (int64_t i = c + 1 + lane; i < m; i += 32) col[i] = scal * col[i];
     __syncwarp();
     if (lane == 0) col[c] = betaT;
@@ -143,377 +127,28 @@ __global__ void qr_extract_r(const T* __restrict__ Bt, int64_t m, int64_t n, int
   }
 }
 
-// ---------------------------------------------------------------------------
-// Register-resident panel variant (columns of up to 32*E rows).
-//
-// Each warp keeps its column in registers (element i at lane i%32, slot i/32);
-// a CTA of kPanel warps owns kPanel consecutive columns (a panel).  Inside a
-// panel, reflector c is made by its owner warp, written to shared memory and
-// applied by the panel's later columns after a CTA barrier -- no global
-// round trip.  Each reflector is also published to global memory with a
-// flag; warps of later panels wait on the flag (bounded) and apply it from
-// registers loaded in one burst.  The critical path is the in-panel chain,
-// one CTA barrier per column.
-constexpr int kPanel = 8;
-
-template <typename T>
-__device__ __forceinline__ T shfl_T(T v, int src) {
-  if constexpr (traits<T>::is_complex) {
-    v.re = __shfl_sync(0xffffffffu, v.re, src);
-    v.im = __shfl_sync(0xffffffffu, v.im, src);
-    return v;
-  } else {
-    return __shfl_sync(0xffffffffu, v, src);
-  }
-}
-
-// value at row i of a register-resident column, broadcast to the warp
-template <typename T, int E>
-__device__ __forceinline__ T reg_get(const T (&x)[E], int i) {
-  const int slot = i >> 5;
-  T a = zero_<T>();
-#pragma unroll
-  for (int u = 0; u < E; ++u)
-    if (u == slot) a = x[u];
-  return shfl_T(a, (int)(i & 31));
-}
-
-// larfg on the register column: entries > c scaled to v, entry c = beta.
-// Norm with four independent partial sums (short dependency chains).
-template <typename T, int E>
-__device__ __forceinline__ T make_reflector_reg(T (&x)[E], int c, int m) {
-  typedef typename traits<T>::real R;
-  const int lane = threadIdx.x & 31;
-  R xn0 = 0, xn1 = 0, xn2 = 0, xn3 = 0;
-#pragma unroll
-  for (int u = 0; u < E; ++u) {
-    const int i = lane + 32 * u;
-    const R a = (i > c && i < m) ? abs2_(x[u]) : R(0);
-    if ((u & 3) == 0) xn0 += a; else if ((u & 3) == 1) xn1 += a; else if ((u & 3) == 2) xn2 += a; else xn3 += a;
-  }
-  const R xn = warp_sum((xn0 + xn1) + (xn2 + xn3));
-  const T alpha = reg_get(x, c);
-  T tau = zero_<T>();
-  if (!(xn == R(0) && imag_(alpha) == R(0))) {
-    const R beta = -copysign(sqrt(abs2_(alpha) + xn), real_(alpha));
-    const T betaT = from_real<T>(beta);
-    tau = div_(betaT - alpha, betaT);
-    const T scal = div_(one_<T>(), alpha - betaT);
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-      const int i = lane + 32 * u;
-      if (i > c && i < m) x[u] = scal * x[u];
-      else if (i == c) x[u] = betaT;
-    }
-  }
-  return tau;
-}
-
-// x <- H_c^H x, v read twice from `v` (entries i > c; v_c = 1 implied):
-// shared memory for the panel's own reflectors, L2 for earlier panels'.  Each
-// pass fetches v in chunks of C independent loads before using them (keeps
-// the L2 latency overlapped without a full register copy of v); the dot
-// product runs four independent partial sums.
-template <typename T, int E, bool GLOBAL>
-__device__ __forceinline__ void apply_stream(T (&x)[E], const T* v, T tau, int c, int m) {
-  constexpr int C = (E % 16 == 0 && E < 48) ? 16 : 8;
-  const int lane = threadIdx.x & 31;
-  T w0 = zero_<T>(), w1 = zero_<T>(), w2 = zero_<T>(), w3 = zero_<T>();
-#pragma unroll
-  for (int u0 = 0; u0 < E; u0 += C) {
-    T vc[C];
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int i = lane + 32 * (u0 + q);
-      vc[q] = (i > c && i < m) ? (GLOBAL ? ldcg(v + i) : v[i]) : zero_<T>();
-    }
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int u = u0 + q;
-      const int i = lane + 32 * u;
-      if (i == c) w0 += x[u];
-      else if ((q & 3) == 0) fma_(w0, conj_(vc[q]), x[u]);
-      else if ((q & 3) == 1) fma_(w1, conj_(vc[q]), x[u]);
-      else if ((q & 3) == 2) fma_(w2, conj_(vc[q]), x[u]);
-      else fma_(w3, conj_(vc[q]), x[u]);
-    }
-  }
-  const T w = warp_sum((w0 + w1) + (w2 + w3));
-  const T f = conj_(tau) * w;
-#pragma unroll
-  for (int u0 = 0; u0 < E; u0 += C) {
-    T vc[C];
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int i = lane + 32 * (u0 + q);
-      vc[q] = (i > c && i < m) ? (GLOBAL ? ldcg(v + i) : v[i]) : zero_<T>();
-    }
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int u = u0 + q;
-      const int i = lane + 32 * u;
-      if (i == c) x[u] = x[u] - f;
-      else x[u] = x[u] - f * vc[q];  // vc is 0 outside (c, m)
-    }
-  }
-}
-
-// The look-ahead step of the owner of column c+1: x <- H_c^H x (v from shared
-// memory) and then the reflector of x at row c+1, in three passes over the
-// register column instead of six: (1) the dot product; (2) the update, the
-// norm of rows > c+1 and row c+1 itself (one shuffle, no select chain);
-// (3) the scaling, written straight to `out` (the next shared buffer).
-template <typename T, int E>
-__device__ __forceinline__ T apply_and_reflect(T (&x)[E], const T* v, T tau, int c, int m, T* out) {
-  typedef typename traits<T>::real R;
-  constexpr int C = (E % 16 == 0 && E < 48) ? 16 : 8;
-  const int lane = threadIdx.x & 31;
-  T w0 = zero_<T>(), w1 = zero_<T>(), w2 = zero_<T>(), w3 = zero_<T>();
-#pragma unroll
-  for (int u0 = 0; u0 < E; u0 += C) {
-    T vc[C];
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int i = lane + 32 * (u0 + q);
-      vc[q] = (i > c && i < m) ? v[i] : zero_<T>();
-    }
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int u = u0 + q;
-      const int i = lane + 32 * u;
-      if (i == c) w0 += x[u];
-      else if ((q & 3) == 0) fma_(w0, conj_(vc[q]), x[u]);
-      else if ((q & 3) == 1) fma_(w1, conj_(vc[q]), x[u]);
-      else if ((q & 3) == 2) fma_(w2, conj_(vc[q]), x[u]);
-      else fma_(w3, conj_(vc[q]), x[u]);
-    }
-  }
-  const T f = conj_(tau) * warp_sum((w0 + w1) + (w2 + w3));
-  const int c1 = c + 1;
-  R n0 = 0, n1 = 0, n2 = 0, n3 = 0;
-  T a_l = zero_<T>();
-#pragma unroll
-  for (int u0 = 0; u0 < E; u0 += C) {
-    T vc[C];
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int i = lane + 32 * (u0 + q);
-      vc[q] = (i > c && i < m) ? v[i] : zero_<T>();
-    }
-#pragma unroll
-    for (int q = 0; q < C; ++q) {
-      const int u = u0 + q;
-      const int i = lane + 32 * u;
-      x[u] = (i == c) ? x[u] - f : x[u] - f * vc[q];
-      const R a = (i > c1 && i < m) ? abs2_(x[u]) : R(0);
-      if ((q & 3) == 0) n0 += a; else if ((q & 3) == 1) n1 += a; else if ((q & 3) == 2) n2 += a; else n3 += a;
-      if (i == c1) a_l = x[u];
-    }
-  }
-  const R xn = warp_sum((n0 + n1) + (n2 + n3));
-  const T alpha = shfl_T(a_l, c1 & 31);
-  T t = zero_<T>();
-  T scal = one_<T>(), betaT = alpha;
-  if (!(xn == R(0) && imag_(alpha) == R(0))) {
-    const R beta = -copysign(sqrt(abs2_(alpha) + xn), real_(alpha));
-    betaT = from_real<T>(beta);
-    t = div_(betaT - alpha, betaT);
-    scal = div_(one_<T>(), alpha - betaT);
-  }
-#pragma unroll
-  for (int u = 0; u < E; ++u) {
-    const int i = lane + 32 * u;
-    if (i > c1 && i < m) x[u] = scal * x[u];
-    else if (i == c1) x[u] = betaT;
-    if (i < m) out[i] = x[u];
-  }
-  return t;
-}
-
-// x <- H_c^H x with v held in registers vv (v_c = 1 implied); used by the
-// Q formation kernel below
-template <typename T, int E>
-__device__ __forceinline__ void apply_reg(T (&x)[E], const T (&vv)[E], T tau, int c, int m) {
-  const int lane = threadIdx.x & 31;
-  T w0 = zero_<T>(), w1 = zero_<T>();
-#pragma unroll
-  for (int u = 0; u < E; ++u) {
-    const int i = lane + 32 * u;
-    if (i == c) w0 += x[u];
-    else if (i > c && i < m) {
-      if (u & 1) fma_(w1, conj_(vv[u]), x[u]);
-      else fma_(w0, conj_(vv[u]), x[u]);
-    }
-  }
-  const T w = warp_sum(w0 + w1);
-  const T f = conj_(tau) * w;
-#pragma unroll
-  for (int u = 0; u < E; ++u) {
-    const int i = lane + 32 * u;
-    if (i == c) x[u] = x[u] - f;
-    else if (i > c && i < m) x[u] = x[u] - f * vv[u];
-  }
-}
-
-template <typename T, int E>
-__global__ void __launch_bounds__(kPanel * 32)
-qr_panel_kernel(T* Bt, int64_t m, int64_t n, int64_t ld, T* tau, int* flags, SyncWords* sw) {
-  __shared__ T sv[2 * 32 * E];
-  __shared__ T stau[2];
-  extern __shared__ __align__(16) unsigned char qr_panel_dyn[];  // kPanel staging rows of 32 * E
-  const int64_t k = m < n ? m : n;
-  const int mi = (int)m;  // rows <= 32 * E
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t p0 = (int64_t)blockIdx.x * kPanel;  // first column of the panel
-  const int64_t j = p0 + warp;                      // my column
-  const bool has = j < n;
-  T x[E];
-  if (has) {
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-      const int i = lane + 32 * u;
-      x[u] = (i < mi) ? Bt[j * ld + i] : zero_<T>();
-    }
-  }
-  // reflectors of earlier panels, as they are published: each is staged from
-  // L2 into this warp's shared-memory row (16 independent loads a lane in
-  // flight), then applied from there in two passes
-  const int64_t cend = p0 < k ? p0 : k;
-  if (has) {
-    T* stage = reinterpret_cast<T*>(qr_panel_dyn) + warp * (32 * E);
-    for (int64_t c = 0; c < cend; ++c) {
-      if (!warp_wait_flag(&flags[c], sw)) break;
-      const T* src = Bt + c * ld;
-      const int ci = (int)c;
-      constexpr int CH = 16;
-#pragma unroll
-      for (int u0 = 0; u0 < E; u0 += CH) {
-        T vc[CH];
-#pragma unroll
-        for (int q = 0; q < CH && u0 + q < E; ++q) {
-          const int i = lane + 32 * (u0 + q);
-          vc[q] = (i > ci && i < mi) ? ldcg(src + i) : zero_<T>();
-        }
-#pragma unroll
-        for (int q = 0; q < CH && u0 + q < E; ++q) stage[lane + 32 * (u0 + q)] = vc[q];
-      }
-      __syncwarp();
-      apply_stream<T, E, false>(x, stage, ldcg(tau + c), ci, mi);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  if (ld_volatile(&sw->err)) return;  // uniform: every warp sees the same error word after the barrier
-  // this panel's reflectors.  Reflector c is written to shared memory buffer
-  // (c & 1) by its owner; after one barrier the later columns apply it, and
-  // the owner of column c+1 builds reflector c+1 into the other buffer right
-  // after applying c (look-ahead).  The owner of c is then done: it
-  // publishes c to global memory (stores, fence, flag) and leaves the loop,
-  // so the barrier of step w counts only warps w..kPanel-1 (a named barrier
-  // with a shrinking count) and no fence sits on the column chain.  The
-  // owner keeps its tau in a register (the shared slot is reused two steps
-  // later, possibly before a departed owner has read it).
-  const int64_t nw = (k - p0) < kPanel ? (k - p0) : kPanel;
-  T my_tau = zero_<T>();
-  if (nw > 0 && warp == 0) {
-    my_tau = make_reflector_reg(x, (int)p0, mi);
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-      const int i = lane + 32 * u;
-      if (i < mi) sv[i] = x[u];
-    }
-    if (lane == 0) stau[0] = my_tau;
-  }
-  for (int w = 0; w < nw; ++w) {
-    const int64_t c = p0 + w;
-    const int b = w & 1;
-    named_barrier(1, (kPanel - w) * 32);
-    if (warp == w) {
-#pragma unroll
-      for (int u = 0; u < E; ++u) {
-        const int i = lane + 32 * u;
-        if (i >= (int)c && i < mi) stcg(Bt + c * ld + i, x[u]);
-      }
-      if (lane == 0) stcg(tau + c, my_tau);
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) atomicExch(&flags[c], 1);
-      break;
-    }
-    if (has) {  // warp > w
-      if (warp == w + 1 && w + 1 < nw) {
-        my_tau = apply_and_reflect<T, E>(x, sv + b * (32 * E), stau[b], (int)c, mi, sv + (b ^ 1) * (32 * E));
-        if (lane == 0) stau[b ^ 1] = my_tau;
-      } else {
-        apply_stream<T, E, false>(x, sv + b * (32 * E), stau[b], (int)c, mi);
-      }
-    }
-  }
-  if (has) {
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-      const int i = lane + 32 * u;
-      if (i < mi) Bt[j * ld + i] = x[u];
-    }
-  }
-}
-
-// Qt[j] = H_{min(j,k-1)} ... H_0 e_j with the column in registers
-template <typename T, int E>
-__global__ void __launch_bounds__(kPanel * 32)
-qr_form_q_reg_kernel(const T* __restrict__ Bt, int64_t m, int64_t k, const T* __restrict__ tau, T* __restrict__ Qt) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = (int64_t)gridDim.x * kPanel;
-  for (int64_t j = (int64_t)blockIdx.x * kPanel + (threadIdx.x >> 5); j < k; j += nwarps) {
-    T x[E], vv[E];
-#pragma unroll
-    for (int u = 0; u < E; ++u) x[u] = (lane + 32 * u == j) ? one_<T>() : zero_<T>();
-    for (int64_t c = j; c >= 0; --c) {
-#pragma unroll
-      for (int u = 0; u < E; ++u) {
-        const int64_t i = lane + 32 * u;
-        vv[u] = (i > c && i < m) ? Bt[c * m + i] : zero_<T>();
-      }
-      // H_c (not conjugated): x -= tau (v^H x) v
-      apply_reg(x, vv, conj_(tau[c]), (int)c, (int)m);
-    }
-#pragma unroll
-    for (int u = 0; u < E; ++u) {
-      const int64_t i = lane + 32 * u;
-      if (i < m) Qt[j * m + i] = x[u];
-    }
-  }
-}
-
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // ---------------------------------------------------------------------------
-// Blocked factorisation (the geqrf / ungqr structure with compact-WY block
-// reflectors, Schreiber & Van Loan 1989).  Panels of kQrNB columns are factored
-// by the dataflow kernels above on the panel's sub-matrix; then, with
-//   H_c0 ... H_c0+nb-1 = I - V T V^H        (T upper triangular, larft),
-// the trailing columns get A2 <- (I - V T^H V^H) A2 and Q is formed backwards,
-// Q <- (I - V T V^H) Q for the panels in reverse order.  In the transposed
-// working layout (rows of Bt / Qt are columns of A / Q) each update is
-//   Wt = X2t conj(V) ,  W2t = Wt op(T) ,  X2t -= W2t Vt
-// with the long dimension as GEMM rows, all on the CUDA-core GEMM (the
-// products have K = 64 or a narrow output; FP32 rounding keeps the
-// reflectors orthogonal to FP32 accuracy).
+// Workspace.  `blocked` (k >= kQrBlockedMin) has room for the general path's
+// products; the panels' T factors (nb x nb each) lie in its `sm` area, or in an
+// area of their own for a smaller k.
 template <typename T>
 static int dtype_of() {
   return sizeof(T) == 4 ? TNC_F32 : (sizeof(T) == 8 ? (traits<T>::is_complex ? TNC_C64 : TNC_F64) : TNC_C128);
 }
 
-constexpr int64_t kQrNB = 64;
-constexpr int64_t kQrBlockedMin = 2 * kQrNB;  // k below this: unblocked dataflow only
+constexpr int64_t kQrNB = 64;                 // panel width of the general path
+constexpr int64_t kQrBlockedMin = 2 * kQrNB;  // k below this: its unblocked dataflow only
 
 constexpr int64_t kQrSplitK = 128;  // K chunk of the split-K products
 
 struct QrLayout {
-  size_t bt, tau, flags, sync, qt, vt, sm, wt, w2t, part, total;
+  size_t bt, tau, flags, sync, qt, vt, sm, wt, w2t, part, tf, total;
   bool blocked;
 };
-static QrLayout qr_layout(int64_t m, int64_t n, int dt) {
+// t_area = false: the caller keeps the T factors (at most k x k elements) elsewhere.
+static QrLayout qr_layout(int64_t m, int64_t n, int dt, bool t_area = true) {
   const size_t es = (size_t)elem_size(dt);
   int64_t k = m < n ? m : n;
   QrLayout L;
@@ -533,6 +168,10 @@ static QrLayout qr_layout(int64_t m, int64_t n, int dt) {
     L.wt = off; off = align256(off + (size_t)rows * kQrNB * es);
     L.w2t = off; off = align256(off + (size_t)rows * kQrNB * es);
     L.part = off; off = align256(off + (size_t)((m + kQrSplitK - 1) / kQrSplitK) * rows * kQrNB * es);
+    L.tf = L.sm;
+  } else {
+    L.tf = off;
+    if (t_area) off = align256(off + (size_t)k * (k < kQrNB ? k : kQrNB) * es);
   }
   L.total = off;
   return L;
@@ -675,63 +314,12 @@ static int qr_gemm_splitk(int opA, int opB, int64_t M, int64_t N, int64_t K, con
   return launch_status(1);
 }
 
-// Dynamic shared memory of the panel kernel (kPanel staging rows of 32 * E
-// elements, up to 96 KB): the attribute is raised once per device.
-template <typename T, int E>
-static int ensure_panel_smem() {
-  constexpr size_t bytes = (size_t)kPanel * 32 * E * sizeof(T);
-  if constexpr (bytes <= 48 * 1024) {
-    return TNC_OK;
-  } else {
-    static std::atomic<unsigned long long> done{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return TNC_ERR_CUDA;
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (done.load() & bit) return TNC_OK;
-    if (cudaFuncSetAttribute((const void*)qr_panel_kernel<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bytes) != cudaSuccess)
-      return TNC_ERR_CUDA;
-    done.fetch_or(bit);
-    return TNC_OK;
-  }
-}
-
 // Unblocked dataflow factorisation of the m x n matrix whose transpose is at
 // Bt (row stride ld): reflectors in place, tau, per-column flags (zeroed by
-// the caller), errors in sw.  Returns the register width E of the panel
-// kernel used (0: the general kernel).
+// the caller), errors in sw.
 template <typename T>
-static int qr_dataflow(int64_t m, int64_t n, int64_t ld, T* Bt, T* tau, int* flags, SyncWords* sw, cudaStream_t st,
-                       int* E_used) {
+static int qr_dataflow(int64_t m, int64_t n, int64_t ld, T* Bt, T* tau, int* flags, SyncWords* sw, cudaStream_t st) {
   void* args[] = {(void*)&Bt, (void*)&m, (void*)&n, (void*)&ld, (void*)&tau, (void*)&flags, (void*)&sw};
-  // register-resident panels when the column fits (E slots of 32 rows)
-  const void* panel_fn = nullptr;
-  int E = 0;
-  int attr_rc = TNC_OK;
-  const int64_t slots = (m + 31) / 32;
-  const int64_t maxE = sizeof(T) >= 16 ? 16 : 48;
-  if (slots <= 8) { panel_fn = (const void*)qr_panel_kernel<T, 8>; E = 8; attr_rc = ensure_panel_smem<T, 8>(); }
-  else if (slots <= 16) { panel_fn = (const void*)qr_panel_kernel<T, 16>; E = 16; attr_rc = ensure_panel_smem<T, 16>(); }
-  else if constexpr (sizeof(T) < 16) {
-    if (slots <= 32 && maxE >= 32) {
-      panel_fn = (const void*)qr_panel_kernel<T, 32>; E = 32; attr_rc = ensure_panel_smem<T, 32>();
-    } else if (slots <= 48 && maxE >= 48) {
-      panel_fn = (const void*)qr_panel_kernel<T, 48>; E = 48; attr_rc = ensure_panel_smem<T, 48>();
-    }
-  }
-  if (attr_rc) return attr_rc;
-  if (panel_fn != nullptr) {
-    const int64_t want = (n + kPanel - 1) / kPanel;
-    const size_t dyn = (size_t)kPanel * 32 * E * sizeof(T);
-    const int cap = coop_capacity(panel_fn, kPanel * 32, dyn);
-    if (cap > 0 && want <= cap) {
-      if (cudaLaunchCooperativeKernel(panel_fn, dim3((unsigned)want), dim3(kPanel * 32), args, dyn, st) != cudaSuccess)
-        return TNC_ERR_CUDA;
-      *E_used = E;
-      return launch_status(1);
-    }
-  }
-  *E_used = 0;
   const int threads = kQrWarps * 32;
   int cap = coop_capacity((const void*)qr_factor_kernel<T>, threads, 0);
   if (cap <= 0) return TNC_ERR_CUDA;
@@ -743,12 +331,104 @@ static int qr_dataflow(int64_t m, int64_t n, int64_t ld, T* Bt, T* tau, int* fla
   return launch_status(1);
 }
 
+// A kernel's dynamic shared memory (and cluster sizes above 8), once per device.
+static int cluster_attrs(const void* fn, size_t smem, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return TNC_ERR_CUDA;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done.load() & bit) return TNC_OK;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return TNC_ERR_CUDA;
+  done.fetch_or(bit);
+  return TNC_OK;
+}
+
+static cudaLaunchConfig_t cluster_config(unsigned ctas, unsigned cluster, int threads, size_t smem, cudaStream_t st,
+                                         cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = cluster;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+static int pow2_at_least(int64_t v) {
+  int p = 1;
+  while (p < v) p *= 2;
+  return p;
+}
+
+template <typename T, int R>
+static int launch_panel(T* P, int64_t ld, int m, int nb, T* tau, T* Tout, int* info, cudaStream_t st) {
+  static std::atomic<unsigned long long> done{0};
+  const size_t smem = qr_panel_smem<T>(R);
+  if (int rc = cluster_attrs((const void*)qr_panel_kernel<T, R>, smem, done)) return rc;
+  const int cs = pow2_at_least((m + 32 * R - 1) / (32 * R));
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config(cs, cs, QrShape<T>::NW * 32, smem, st, &attr);
+  return cudaLaunchKernelEx(&cfg, qr_panel_kernel<T, R>, P, ld, m, nb, tau, Tout, cs, info) == cudaSuccess ? TNC_OK
+                                                                                                         : TNC_ERR_CUDA;
+}
+
+// Rows of a CTA by the panel's length: FP32 panels stay within the portable
+// cluster of 8 as long as they can (a step's barrier and reduction take 1160
+// cycles over 8 CTAs and 1700 over 16, measured); FP64 panels spread over 16
+// as soon as possible, their arithmetic being the longer part.
+template <typename T>
+static int qr_panel(T* P, int64_t ld, int64_t m, int64_t nb, T* tau, T* Tout, int* info, cudaStream_t st) {
+  const int rows = (int)m, n = (int)nb;
+  if constexpr (sizeof(typename traits<T>::real) == 4) {
+    if (m <= 512) return launch_panel<T, 2>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 1024) return launch_panel<T, 4>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 1536) return launch_panel<T, 6>(P, ld, rows, n, tau, Tout, info, st);
+  } else {
+    if (m <= 512) return launch_panel<T, 1>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 1024) return launch_panel<T, 2>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 2048) return launch_panel<T, 4>(P, ld, rows, n, tau, Tout, info, st);
+  }
+  return launch_panel<T, 8>(P, ld, rows, n, tau, Tout, info, st);
+}
+
+// X (nc columns, ms rows) <- (I - V op(T) V^H) X.  Clusters of up to 8 CTAs of
+// 64 rows or more, 32 where that leaves SMs idle, as many as shared memory
+// holds at most.
+template <typename T>
+static int qr_apply(const T* V, int64_t ldv, int64_t nb, int64_t ms, const T* Tm, T* X, int64_t ldx, int64_t nc,
+                    int adjoint, cudaStream_t st) {
+  constexpr int kRows = std::is_same<T, c64>::value ? 192 : 256;
+  static std::atomic<unsigned long long> done{0};
+  if (int rc = cluster_attrs((const void*)qr_apply_kernel<T>, qr_apply_smem<T>(kRows), done)) return rc;
+  const int64_t blocks = (nc + QrShape<T>::NC - 1) / QrShape<T>::NC;
+  int cs = pow2_at_least((ms + 63) / 64);
+  if (cs > 8) cs = 8;
+  while (cs < 8 && 32 * cs < ms && blocks * cs < 152) cs *= 2;
+  int64_t rows = ((ms + cs - 1) / cs + 31) / 32 * 32;
+  if (rows < QrShape<T>::NB) rows = QrShape<T>::NB;
+  if (rows > kRows) rows = kRows;
+  if (blocks * cs > 0x7fffffff) return TNC_ERR_ARG;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config((unsigned)(blocks * cs), cs, QrShape<T>::ATHR,
+                                                qr_apply_smem<T>((int)rows), st, &attr);
+  return cudaLaunchKernelEx(&cfg, qr_apply_kernel<T>, V, ldv, (int)nb, ms, Tm, X, ldx, nc, (int)rows, cs, adjoint) ==
+                 cudaSuccess
+             ? TNC_OK
+             : TNC_ERR_CUDA;
+}
+
 // Householder factorisation of the m x n matrix X whose transpose is already
 // in Bt (n x m, dense).  R (k x n) is always extracted; the rows of Q^T
 // (k x m, in the workspace at L.qt) are formed when want_qt or Q is set, and
 // Q = (Q^T)^T (m x k) is written when Q is not null.
 template <typename T>
-static int qr_factor_bt(int64_t m, int64_t n, T* Q, bool want_qt, T* R, const QrLayout& L, char* w, int* info,
+static int qr_factor_bt(int64_t m, int64_t n, T* Q, bool want_qt, T* R, const QrLayout& L, char* w, T* tf, int* info,
                         cudaStream_t st) {
   const int64_t k = m < n ? m : n;
   T* Bt = (T*)(w + L.bt);
@@ -757,31 +437,49 @@ static int qr_factor_bt(int64_t m, int64_t n, T* Q, bool want_qt, T* R, const Qr
   SyncWords* sw = (SyncWords*)(w + L.sync);
   T* Qt = (T*)(w + L.qt);
   const bool form_q = (Q != nullptr || want_qt);
+  if (m <= kQrPanelRows) {
+    constexpr int64_t NB = QrShape<T>::NB;
+    if (cudaMemsetAsync(info, 0, sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
+    int launches = 1;  // extract R
+    for (int64_t c0 = 0; c0 < k; c0 += NB) {
+      const int64_t nb = (k - c0) < NB ? (k - c0) : NB, ms = m - c0, n2 = n - c0 - nb;
+      T* panel = Bt + c0 * m + c0;
+      if (int rc = qr_panel<T>(panel, m, ms, nb, tau + c0, tf + c0 * NB, info, st)) return rc;
+      ++launches;
+      if (n2 > 0) {
+        if (int rc = qr_apply<T>(panel, m, nb, ms, tf + c0 * NB, panel + nb * m, m, n2, 1, st)) return rc;
+        ++launches;
+      }
+    }
+    qr_extract_r<T><<<grid1d(k * n, 256), 256, 0, st>>>(Bt, m, n, k, R);
+    if (form_q) {
+      qr_eye_rows<T><<<grid1d(k * m, 256), 256, 0, st>>>(Qt, k, m);
+      ++launches;
+      for (int64_t c0 = (k - 1) / NB * NB; c0 >= 0; c0 -= NB) {
+        const int64_t nb = (k - c0) < NB ? (k - c0) : NB;
+        if (int rc = qr_apply<T>(Bt + c0 * m + c0, m, nb, m - c0, tf + c0 * NB, Qt + c0 * m + c0, m, k - c0, 0, st))
+          return rc;
+        ++launches;
+      }
+    }
+    if (launch_status(launches)) return TNC_ERR_CUDA;
+    if (Q == nullptr) return TNC_OK;
+    const int64_t shp[2] = {k, m};
+    const int perm[2] = {1, 0};
+    return tnc_permute(dtype_of<T>(), Qt, Q, 2, shp, perm, 0, st);
+  }
   if (cudaMemsetAsync(flags, 0, (size_t)k * sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(sw, 0, sizeof(SyncWords), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(info, 0, sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (!L.blocked) {
-    int E = 0;
-    if (int rc = qr_dataflow<T>(m, n, m, Bt, tau, flags, sw, st, &E)) return rc;
+    if (int rc = qr_dataflow<T>(m, n, m, Bt, tau, flags, sw, st)) return rc;
     copy_sync_error<<<1, 1, 0, st>>>(sw, info);
     int launches = 2;  // error copy, extract R
     if (form_q) {
-      void (*formq_fn)(const T*, int64_t, int64_t, const T*, T*) = nullptr;
-      if (E == 8) formq_fn = qr_form_q_reg_kernel<T, 8>;
-      else if (E == 16) formq_fn = qr_form_q_reg_kernel<T, 16>;
-      else if constexpr (sizeof(T) < 16) {
-        if (E == 32) formq_fn = qr_form_q_reg_kernel<T, 32>;
-        else if (E == 48) formq_fn = qr_form_q_reg_kernel<T, 48>;
-      }
-      if (formq_fn != nullptr) {
-        int64_t gq = (k + kPanel - 1) / kPanel;
-        formq_fn<<<(unsigned)gq, kPanel * 32, 0, st>>>(Bt, m, k, tau, Qt);
-      } else {
-        const int threads = kQrWarps * 32;
-        int64_t gq = (k + kQrWarps - 1) / kQrWarps;
-        if (gq > 152 * 16) gq = 152 * 16;
-        qr_form_q_kernel<T><<<(unsigned)gq, threads, 0, st>>>(Bt, m, k, tau, Qt);
-      }
+      const int threads = kQrWarps * 32;
+      int64_t gq = (k + kQrWarps - 1) / kQrWarps;
+      if (gq > 152 * 16) gq = 152 * 16;
+      qr_form_q_kernel<T><<<(unsigned)gq, threads, 0, st>>>(Bt, m, k, tau, Qt);
       ++launches;
     }
     qr_extract_r<T><<<grid1d(k * n, 256), 256, 0, st>>>(Bt, m, n, k, R);
@@ -801,8 +499,7 @@ static int qr_factor_bt(int64_t m, int64_t n, T* Q, bool want_qt, T* R, const Qr
       const int64_t nbb = (k - c0) < kQrNB ? (k - c0) : kQrNB;
       const int64_t ms = m - c0;
       T* panel = Bt + c0 * m + c0;
-      int E = 0;
-      if (int rc = qr_dataflow<T>(ms, nbb, m, panel, tau + c0, flags + c0, sw, st, &E)) return rc;
+      if (int rc = qr_dataflow<T>(ms, nbb, m, panel, tau + c0, flags + c0, sw, st)) return rc;
       const int64_t n2 = n - c0 - nbb;
       const bool need_t = form_q || n2 > 0;
       if (!need_t) continue;
@@ -865,7 +562,7 @@ static int qr_impl(int64_t m, int64_t n, const T* A, int64_t lda, T* Q, T* R, vo
   int64_t shp[2] = {m, n};
   int perm[2] = {1, 0};
   if (int s = tnc_permute(dtype_of<T>(), A, (T*)(w + L.bt), 2, shp, perm, 0, st)) return s;
-  return qr_factor_bt<T>(m, n, Q, false, R, L, w, info, st);
+  return qr_factor_bt<T>(m, n, Q, false, R, L, w, (T*)(w + L.tf), info, st);
 }
 
 // R factor only, of A (m x n) or, with adjoint, of A^H (n x m).  For A^H the
@@ -889,20 +586,20 @@ static int qr_r_impl(int64_t m, int64_t n, const T* A, int adjoint, T* R, void* 
     int perm[2] = {1, 0};
     if (int s = tnc_permute(dtype_of<T>(), A, (T*)(w + L.bt), 2, shp, perm, 0, st)) return s;
   }
-  return qr_factor_bt<T>(fm, fn, (T*)nullptr, false, R, L, w, info, st);
+  return qr_factor_bt<T>(fm, fn, (T*)nullptr, false, R, L, w, (T*)(w + L.tf), info, st);
 }
 
 }  // namespace tnc
 
 namespace tnc {
 
-size_t qr_qt_workspace(int64_t fm, int64_t fn, int dt) { return qr_layout(fm, fn, dt).total; }
+size_t qr_qt_workspace(int64_t fm, int64_t fn, int dt) { return qr_layout(fm, fn, dt, false).total; }
 
 template <typename T>
-int qr_qt(int64_t fm, int64_t fn, const T* A, int adjoint, bool want_qt, T* R, void* work, size_t wb, int* info,
+int qr_qt(int64_t fm, int64_t fn, const T* A, int adjoint, bool want_qt, T* R, void* work, size_t wb, T* tf, int* info,
           cudaStream_t st, T** qt) {
   if (fm <= 0 || fn <= 0 || !A || !R || !work || !info) return TNC_ERR_ARG;
-  QrLayout L = qr_layout(fm, fn, dtype_of<T>());
+  QrLayout L = qr_layout(fm, fn, dtype_of<T>(), false);
   if (wb < L.total) return TNC_ERR_WORKSPACE;
   char* w = (char*)work;
   // Bt = X^T: for X = A^H that is conj(A) as stored (A is fn x fm)
@@ -912,14 +609,13 @@ int qr_qt(int64_t fm, int64_t fn, const T* A, int adjoint, bool want_qt, T* R, v
                           (adjoint && traits<T>::is_complex) ? 1 : 0, st))
     return s;
   if (qt) *qt = (T*)(w + L.qt);
-  return qr_factor_bt<T>(fm, fn, (T*)nullptr, want_qt, R, L, w, info, st);
+  return qr_factor_bt<T>(fm, fn, (T*)nullptr, want_qt, R, L, w, L.blocked ? (T*)(w + L.tf) : tf, info, st);
 }
 
-template int qr_qt<float>(int64_t, int64_t, const float*, int, bool, float*, void*, size_t, int*, cudaStream_t, float**);
-template int qr_qt<double>(int64_t, int64_t, const double*, int, bool, double*, void*, size_t, int*, cudaStream_t,
-                           double**);
-template int qr_qt<c64>(int64_t, int64_t, const c64*, int, bool, c64*, void*, size_t, int*, cudaStream_t, c64**);
-template int qr_qt<c128>(int64_t, int64_t, const c128*, int, bool, c128*, void*, size_t, int*, cudaStream_t, c128**);
+template int qr_qt<float>(int64_t, int64_t, const float*, int, bool, float*, void*, size_t, float*, int*, cudaStream_t, float**);
+template int qr_qt<double>(int64_t, int64_t, const double*, int, bool, double*, void*, size_t, double*, int*, cudaStream_t, double**);
+template int qr_qt<c64>(int64_t, int64_t, const c64*, int, bool, c64*, void*, size_t, c64*, int*, cudaStream_t, c64**);
+template int qr_qt<c128>(int64_t, int64_t, const c128*, int, bool, c128*, void*, size_t, c128*, int*, cudaStream_t, c128**);
 
 TNC_DEFINE_SPIN_SETTER(spin_limit_set_qr)
 

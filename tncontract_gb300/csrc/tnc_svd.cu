@@ -222,7 +222,8 @@ static int svd_impl(int64_t m, int64_t n, const T* A, int64_t lda, T* U, typenam
   double* frob2 = (double*)(w + Ly.frob2);
   T* Qt = nullptr;
   // X = A^H (wide) or A (tall); R of X into W, Q^T (nr x L) kept in the QR workspace
-  int s = qr_qt<T>(L, nr, A, tall ? 0 : 1, true, W, w + Ly.qr, qr_qt_workspace(L, nr, dtype_of<T>()), info, st, &Qt);
+  int s = qr_qt<T>(L, nr, A, tall ? 0 : 1, true, W, w + Ly.qr, qr_qt_workspace(L, nr, dtype_of<T>()), J, info,
+                   st, &Qt);
   if (s) return s;
   T* small = (T*)(w + Ly.qr);  // the QR's transposed copy (nr * L >= nr * nr elements) is free now
   eye_kernel<T><<<grid1d(nr * nr, 256), 256, 0, st>>>(J, nr);
