@@ -1,18 +1,18 @@
 // Batched GEMM on row-major operands with transpose / conjugate options
 // (the product inside np.tensordot, tncontract/tensor.py:735).
 //
-// CUDA-core tiled kernel: a 64x64 output tile per 256-thread CTA, 4x4
-// register micro-tile per thread, K in slices of BK staged in shared memory
-// k-major (so a thread reads its 4 consecutive values of each operand with
-// 16-byte loads).  Two shared-memory buffers: the next slice is fetched into
-// registers while the current one is multiplied, then stored to the other
-// buffer -- one CTA barrier per slice and the global-load latency hidden
-// behind the FMAs.  Whether an operand's contiguous axis is K (A: N/R,
-// B: T/C) or M/N (A: T/C, B: N/R) is a template parameter, so each tile load
-// is a coalesced, branch-free pattern.  This is the FP64 / complex128 path
-// (GB300 runs FP64 on the CUDA cores), the FP32-accurate path of the blocked
-// QR's products, and the general path for small or odd shapes; FP32-class
-// products that tolerate TF32-split accuracy can use the tcgen05 kernel.
+// CUDA-core tiled kernel: an output tile per CTA (64 x 64 with a 4x4 register
+// micro-tile per thread in FP32, smaller ones in FP64), K in slices of BK
+// staged in shared memory k-major (so an FP32 thread reads its 4 consecutive
+// values of each operand with 16-byte loads).  Two shared-memory buffers: the
+// next slice is fetched into registers while the current one is multiplied,
+// then stored to the other buffer -- one CTA barrier per slice and the
+// global-load latency hidden behind the FMAs.  Whether an operand's contiguous
+// axis is K (A: N/R, B: T/C) or M/N (A: T/C, B: N/R) is a template parameter,
+// so each tile load is a coalesced, branch-free pattern.  This is the FP64 /
+// complex128 path (GB300 runs FP64 on the CUDA cores) and the general path for
+// small or odd shapes; FP32-class products that tolerate its digit split can
+// use the tcgen05 kernel.
 #include "tnc_common.cuh"
 
 namespace tnc {
@@ -25,68 +25,68 @@ __device__ __forceinline__ void lds4(const float* p, float (&v)[4]) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
-__device__ __forceinline__ void lds4(const double* p, double (&v)[4]) {
-  const double2 q0 = reinterpret_cast<const double2*>(p)[0], q1 = reinterpret_cast<const double2*>(p)[1];
-  v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-}
 __device__ __forceinline__ void lds4(const c64* p, c64 (&v)[4]) {
   const float4 q0 = reinterpret_cast<const float4*>(p)[0], q1 = reinterpret_cast<const float4*>(p)[1];
   v[0] = c64(q0.x, q0.y); v[1] = c64(q0.z, q0.w); v[2] = c64(q1.x, q1.y); v[3] = c64(q1.z, q1.w);
 }
-__device__ __forceinline__ void lds4(const c128* p, c128 (&v)[4]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = p[i];
-}
 
-template <typename T>
+// Output tile BM x BN of a CTA, TM x TN of it a thread, K slices of BK.
+// FP32 threads take 4 x 4 consecutive outputs (16-byte shared-memory loads feed
+// the FMAs).  FP64 ones take outputs BM / TM rows and BN / TN columns apart: an
+// FP64 instruction holds a scheduler for 64 cycles, so loads are free beside it
+// and any tile runs at the pipe's rate; only the balance over the SMs counts.
+template <typename T, int BM_, int BN_, int TM_, int TN_>
 struct GemmTile {
-  static constexpr int BM = 64, BN = 64;
-  static constexpr int BK = sizeof(T) >= 16 ? 8 : 16;
-  static constexpr int PAD = sizeof(T) >= 16 ? 1 : 16 / (int)sizeof(T);  // rows stay 16-byte aligned
-  static constexpr int LD = BM + PAD;
-  static constexpr int PER = BM * BK / 256;  // tile elements each thread moves
+  static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_;
+  static constexpr int THR = (BM / TM) * (BN / TN);
+  static constexpr bool WIDE = sizeof(typename traits<T>::real) == 8;
+  static constexpr int BK = 16;
+  static constexpr int PAD = WIDE ? 1 : 16 / (int)sizeof(T);  // FP32 rows stay 16-byte aligned
+  static constexpr int LDA = BM + PAD, LDB = BN + PAD;
+  static constexpr int PA = BM * BK / THR, PB = BN * BK / THR;  // tile elements each thread moves
 };
+template <typename T> using Tile64 = GemmTile<T, 64, 64, 4, 4>;  // FP32
+template <typename T> using TileL = GemmTile<T, 32, 32, 4, 2>;   // FP64, 128 threads each
+template <typename T> using TileM = GemmTile<T, 16, 16, 2, 1>;
+template <typename T> using TileS = GemmTile<T, 8, 16, 1, 1>;
 
-// Fetch the BK-slice at k0 of a 64-row operand tile into registers.
+// Fetch the BK-slice at k0 of a BR-row operand tile into registers.
 // KMAJOR: element (r, k) at X[r * ld + k] (lanes run along k);
 // else:   element (r, k) at X[k * ld + r] (lanes run along r).
-template <typename T, bool KMAJOR>
+template <typename T, int BR, int BK, int THR, bool KMAJOR, int PER>
 __device__ __forceinline__ void tile_fetch(const T* __restrict__ X, int64_t ld, int64_t r0, int64_t R, int64_t k0,
-                                           int64_t K, T (&v)[GemmTile<T>::PER]) {
-  constexpr int BK = GemmTile<T>::BK;
+                                           int64_t K, T (&v)[PER]) {
   const int t = threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < GemmTile<T>::PER; ++j) {
+  for (int j = 0; j < PER; ++j) {
     int r, k;
-    if (KMAJOR) { k = t % BK; r = t / BK + (256 / BK) * j; }
-    else { r = t & 63; k = (t >> 6) + 4 * j; }
+    if (KMAJOR) { k = t % BK; r = t / BK + (THR / BK) * j; }
+    else { r = t % BR; k = t / BR + (THR / BR) * j; }
     const int64_t gr = r0 + r, gk = k0 + k;
     v[j] = (gr < R && gk < K) ? (KMAJOR ? X[gr * ld + gk] : X[gk * ld + gr]) : zero_<T>();
   }
 }
 
-template <typename T, bool KMAJOR>
-__device__ __forceinline__ void tile_store(T* s, const T (&v)[GemmTile<T>::PER], bool cj) {
-  constexpr int BK = GemmTile<T>::BK, LD = GemmTile<T>::LD;
+template <typename T, int BR, int BK, int LD, int THR, bool KMAJOR, int PER>
+__device__ __forceinline__ void tile_store(T* s, const T (&v)[PER], bool cj) {
   const int t = threadIdx.x;
 #pragma unroll
-  for (int j = 0; j < GemmTile<T>::PER; ++j) {
+  for (int j = 0; j < PER; ++j) {
     int r, k;
-    if (KMAJOR) { k = t % BK; r = t / BK + (256 / BK) * j; }
-    else { r = t & 63; k = (t >> 6) + 4 * j; }
+    if (KMAJOR) { k = t % BK; r = t / BK + (THR / BK) * j; }
+    else { r = t % BR; k = t / BR + (THR / BR) * j; }
     s[k * LD + r] = maybe_conj(v[j], cj);
   }
 }
 
-// One 64 x 64 output tile (rows m0.., columns n0..) of C = alpha op(A) op(B) + beta C.
-template <typename T, bool AK, bool BKM>
+// One output tile (rows m0.., columns n0..) of C = alpha op(A) op(B) + beta C.
+// The terms of an output are added in the order of k by every tile shape.
+template <typename T, typename G, bool AK, bool BKM>
 __device__ __forceinline__ void gemm_tile(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha,
                                           const T* __restrict__ Ab, int64_t lda, const T* __restrict__ Bb,
                                           int64_t ldb, T beta, T* __restrict__ Cb, int64_t ldc, int64_t m0,
-                                          int64_t n0, T (*As)[GemmTile<T>::BK * GemmTile<T>::LD],
-                                          T (*Bs)[GemmTile<T>::BK * GemmTile<T>::LD]) {
-  typedef GemmTile<T> G;
-  constexpr int TM = 4, TN = 4;
+                                          int64_t n0, T (*As)[G::BK * G::LDA], T (*Bs)[G::BK * G::LDB]) {
+  constexpr int TM = G::TM, TN = G::TN, BK = G::BK;
   const int tid = threadIdx.x;
   const int tx = tid % (G::BN / TN), ty = tid / (G::BN / TN);
   const bool beta_zero = (abs2_(beta) == 0);
@@ -96,45 +96,58 @@ __device__ __forceinline__ void gemm_tile(int64_t M, int64_t N, int64_t K, bool 
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = zero_<T>();
 
-  T va[G::PER], vb[G::PER];
-  tile_fetch<T, AK>(Ab, lda, m0, M, 0, K, va);
-  tile_fetch<T, BKM>(Bb, ldb, n0, N, 0, K, vb);
-  tile_store<T, AK>(As[0], va, aC);
-  tile_store<T, BKM>(Bs[0], vb, bC);
+  T va[G::PA], vb[G::PB];
+  auto fetch = [&](int64_t k0) {
+    tile_fetch<T, G::BM, BK, G::THR, AK>(Ab, lda, m0, M, k0, K, va);
+    tile_fetch<T, G::BN, BK, G::THR, BKM>(Bb, ldb, n0, N, k0, K, vb);
+  };
+  auto store = [&](int buf) {
+    tile_store<T, G::BM, BK, G::LDA, G::THR, AK>(As[buf], va, aC);
+    tile_store<T, G::BN, BK, G::LDB, G::THR, BKM>(Bs[buf], vb, bC);
+  };
+  fetch(0);
+  store(0);
   __syncthreads();
   int buf = 0;
-  for (int64_t k0 = 0; k0 < K; k0 += G::BK) {
-    const bool more = k0 + G::BK < K;
-    if (more) {
-      tile_fetch<T, AK>(Ab, lda, m0, M, k0 + G::BK, K, va);
-      tile_fetch<T, BKM>(Bb, ldb, n0, N, k0 + G::BK, K, vb);
-    }
+  for (int64_t k0 = 0; k0 < K; k0 += BK) {
+    const bool more = k0 + BK < K;
+    if (more) fetch(k0 + BK);
     const T* as = As[buf];
     const T* bs = Bs[buf];
-#pragma unroll
-    for (int kk = 0; kk < G::BK; ++kk) {
+    auto step = [&](int kk) {
       T a[TM], b[TN];
-      lds4(as + kk * G::LD + ty * TM, a);
-      lds4(bs + kk * G::LD + tx * TN, b);
+      if constexpr (G::WIDE) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = as[kk * G::LDA + ty + (G::BM / TM) * i];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[j] = bs[kk * G::LDB + tx + (G::BN / TN) * j];
+      } else {
+        lds4(as + kk * G::LDA + ty * TM, a);
+        lds4(bs + kk * G::LDB + tx * TN, b);
+      }
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) fma_(acc[i][j], a[i], b[j]);
+    };
+    const int kn = (K - k0) < BK ? (int)(K - k0) : BK;
+    if (!G::WIDE || kn == BK) {
+#pragma unroll
+      for (int kk = 0; kk < BK; ++kk) step(kk);
+    } else {  // no FP64 products with the padding
+      for (int kk = 0; kk < kn; ++kk) step(kk);
     }
-    if (more) {
-      tile_store<T, AK>(As[buf ^ 1], va, aC);
-      tile_store<T, BKM>(Bs[buf ^ 1], vb, bC);
-    }
+    if (more) store(buf ^ 1);
     __syncthreads();
     buf ^= 1;
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int64_t gm = m0 + ty * TM + i;
+    const int64_t gm = m0 + (G::WIDE ? ty + (G::BM / TM) * i : ty * TM + i);
     if (gm >= M) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int64_t gn = n0 + tx * TN + j;
+      const int64_t gn = n0 + (G::WIDE ? tx + (G::BN / TN) * j : tx * TN + j);
       if (gn >= N) continue;
       T v = alpha * acc[i][j];
       if (!beta_zero) v += beta * Cb[gm * ldc + gn];
@@ -143,20 +156,35 @@ __device__ __forceinline__ void gemm_tile(int64_t M, int64_t N, int64_t K, bool 
   }
 }
 
-template <typename T, bool AK, bool BKM>
-__global__ void __launch_bounds__(256)
+template <typename T, typename G, bool AK, bool BKM>
+__global__ void __launch_bounds__(G::THR)
 gemm_simt_kernel(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, const T* __restrict__ A, int64_t lda,
                  int64_t sA, const T* __restrict__ B, int64_t ldb, int64_t sB, T beta, T* __restrict__ C,
                  int64_t ldc, int64_t sC, int64_t batch) {
-  typedef GemmTile<T> G;
-  __shared__ __align__(16) T As[2][G::BK * G::LD];
-  __shared__ __align__(16) T Bs[2][G::BK * G::LD];
-  const int64_t m0 = (int64_t)blockIdx.y * G::BM, n0 = (int64_t)blockIdx.x * G::BN;
-  for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z) {
-    gemm_tile<T, AK, BKM>(M, N, K, aC, bC, alpha, A + bz * sA, lda, B + bz * sB, ldb, beta, C + bz * sC, ldc, m0,
-                          n0, As, Bs);
-    __syncthreads();  // the next batch entry reuses the shared tiles
-  }
+  __shared__ __align__(16) T As[2][G::BK * G::LDA];
+  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
+  const int64_t n0 = (int64_t)blockIdx.x * G::BN;
+  for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z)
+    for (int64_t m0 = (int64_t)blockIdx.y * G::BM; m0 < M; m0 += (int64_t)gridDim.y * G::BM) {
+      gemm_tile<T, G, AK, BKM>(M, N, K, aC, bC, alpha, A + bz * sA, lda, B + bz * sB, ldb, beta, C + bz * sC, ldc, m0,
+                               n0, As, Bs);
+      __syncthreads();  // the next tile reuses the shared tiles
+    }
+}
+
+// FP64 tile of a set of products by the time of the busiest SM: tiles are dealt
+// to 152 SMs and a tile takes BM BN K / 2 cycles of its SM (four times that in
+// complex), so the cost is ceil(tiles / 152) BM BN; the larger tile among equals
+// (fewer loads).  One 64 x 64 tile shape left most SMs without work: a 32 x 16 x
+// 32 complex128 product took 70 us in one CTA, a 513 x 203 x 291 float64 one 220
+// in 45.  ``tiles`` counts the tiles of a shape.
+enum { kTileS, kTileM, kTileL };
+template <typename Count>
+static int wide_tile(Count tiles) {
+  const int64_t cl = (tiles(32, 32) + 151) / 152 * 1024, cm = (tiles(16, 16) + 151) / 152 * 256,
+                cs = (tiles(8, 16) + 151) / 152 * 128;
+  if (cl <= cm && cl <= cs) return kTileL;
+  return cm <= cs ? kTileM : kTileS;
 }
 
 // Independent products of different shapes in one launch: the CTAs of the
@@ -176,11 +204,10 @@ struct GemmGroup {
   GroupProblem p[kGroupMax];
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_grouped_kernel(const __grid_constant__ GemmGroup g) {
-  typedef GemmTile<T> G;
-  __shared__ __align__(16) T As[2][G::BK * G::LD];
-  __shared__ __align__(16) T Bs[2][G::BK * G::LD];
+template <typename T, typename G>
+__global__ void __launch_bounds__(G::THR) gemm_grouped_kernel(const __grid_constant__ GemmGroup g) {
+  __shared__ __align__(16) T As[2][G::BK * G::LDA];
+  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
   int q = 0;
   while (q + 1 < g.count && (int64_t)blockIdx.x >= g.p[q + 1].tile0) ++q;
   const GroupProblem& P = g.p[q];
@@ -192,10 +219,24 @@ __global__ void __launch_bounds__(256) gemm_grouped_kernel(const __grid_constant
   const T* A = (const T*)P.A;
   const T* B = (const T*)P.B;
   T* C = (T*)P.C;
-  if (aK && bK) gemm_tile<T, true, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
-  else if (aK) gemm_tile<T, true, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
-  else if (bK) gemm_tile<T, false, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
-  else gemm_tile<T, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
+  if (aK && bK) gemm_tile<T, G, true, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
+  else if (aK) gemm_tile<T, G, true, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
+  else if (bK) gemm_tile<T, G, false, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
+  else gemm_tile<T, G, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
+}
+
+template <typename T, typename G>
+static int grouped_launch(GemmGroup& g, cudaStream_t st) {
+  int64_t tiles = 0;
+  for (int i = 0; i < g.count; ++i) {
+    GroupProblem& q = g.p[i];
+    q.tiles_n = (q.n + G::BN - 1) / G::BN;
+    q.tile0 = tiles;
+    tiles += q.tiles_n * ((q.m + G::BM - 1) / G::BM);
+  }
+  if (tiles > 0x7fffffff) return TNC_ERR_ARG;
+  gemm_grouped_kernel<T, G><<<(unsigned)tiles, G::THR, 0, st>>>(g);
+  return launch_status();
 }
 
 template <typename T>
@@ -203,7 +244,6 @@ int gemm_grouped_launch(int count, const tnc_gemm_problem* probs, cudaStream_t s
   if (count <= 0 || count > kGroupMax || !probs) return TNC_ERR_ARG;
   GemmGroup g;
   g.count = 0;
-  int64_t tiles = 0;
   for (int i = 0; i < count; ++i) {
     const tnc_gemm_problem& p = probs[i];
     if (p.m < 0 || p.n < 0 || p.k <= 0 || p.opA < 0 || p.opA > 3 || p.opB < 0 || p.opB > 3 || p.ldc < p.n)
@@ -214,14 +254,22 @@ int gemm_grouped_launch(int count, const tnc_gemm_problem* probs, cudaStream_t s
     q.m = p.m; q.n = p.n; q.k = p.k; q.lda = p.lda; q.ldb = p.ldb; q.ldc = p.ldc;
     q.A = p.A; q.B = p.B; q.C = p.C; q.opA = p.opA; q.opB = p.opB;
     q.alpha[0] = p.alpha[0]; q.alpha[1] = p.alpha[1]; q.beta[0] = p.beta[0]; q.beta[1] = p.beta[1];
-    q.tiles_n = (p.n + GemmTile<T>::BN - 1) / GemmTile<T>::BN;
-    q.tile0 = tiles;
-    tiles += q.tiles_n * ((p.m + GemmTile<T>::BM - 1) / GemmTile<T>::BM);
   }
   if (g.count == 0) return TNC_OK;
-  if (tiles > 0x7fffffff) return TNC_ERR_ARG;
-  gemm_grouped_kernel<T><<<(unsigned)tiles, 256, 0, st>>>(g);
-  return launch_status();
+  if constexpr (Tile64<T>::WIDE) {
+    auto count_tiles = [&](int bm, int bn) {
+      int64_t t = 0;
+      for (int i = 0; i < g.count; ++i) t += ((g.p[i].m + bm - 1) / bm) * ((g.p[i].n + bn - 1) / bn);
+      return t;
+    };
+    switch (wide_tile(count_tiles)) {
+      case kTileS: return grouped_launch<T, TileS<T>>(g, st);
+      case kTileM: return grouped_launch<T, TileM<T>>(g, st);
+      default: return grouped_launch<T, TileL<T>>(g, st);
+    }
+  } else {
+    return grouped_launch<T, Tile64<T>>(g, st);
+  }
 }
 
 // C = beta*C when K == 0 (np.tensordot over no axes still has the outer
@@ -237,6 +285,27 @@ __global__ void gemm_scale_c(int64_t M, int64_t N, T beta, T* C, int64_t ldc, in
   }
 }
 
+template <typename T, typename G>
+static int simt_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, const T* A, int64_t lda, int64_t sA,
+                       const T* B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC, int64_t batch,
+                       cudaStream_t st) {
+  const int64_t gy = (m + G::BM - 1) / G::BM, gx = (n + G::BN - 1) / G::BN;
+  if (gx > 0x7fffffff) return TNC_ERR_ARG;
+  const dim3 grid((unsigned)gx, (unsigned)(gy < 65535 ? gy : 65535), (unsigned)(batch < 65535 ? batch : 65535));
+  // A is K-contiguous for N / R, B for T / C
+  const bool aK = (opA == TNC_OP_N || opA == TNC_OP_R), bK = (opB == TNC_OP_T || opB == TNC_OP_C);
+  const bool aC = (opA == TNC_OP_C || opA == TNC_OP_R), bC = (opB == TNC_OP_C || opB == TNC_OP_R);
+#define TNC_GEMM_LAUNCH(AKV, BKV)                                                                                  \
+  gemm_simt_kernel<T, G, AKV, BKV><<<grid, G::THR, 0, st>>>(m, n, k, aC, bC, alpha, A, lda, sA, B, ldb, sB, beta, C, \
+                                                            ldc, sC, batch)
+  if (aK && bK) TNC_GEMM_LAUNCH(true, true);
+  else if (aK) TNC_GEMM_LAUNCH(true, false);
+  else if (bK) TNC_GEMM_LAUNCH(false, true);
+  else TNC_GEMM_LAUNCH(false, false);
+#undef TNC_GEMM_LAUNCH
+  return launch_status();
+}
+
 template <typename T>
 int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, const T* A, int64_t lda,
                 int64_t sA, const T* B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC,
@@ -248,24 +317,17 @@ int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, cons
     gemm_scale_c<T><<<grid1d(m * n * batch, 256), 256, 0, st>>>(m, n, beta, C, ldc, sC, batch);
     return launch_status();
   }
-  constexpr int BM = GemmTile<T>::BM, BN = GemmTile<T>::BN;
-  int64_t gy = (m + BM - 1) / BM, gx = (n + BN - 1) / BN;
-  if (gy > 65535) return TNC_ERR_ARG;
-  if (gx > 0x7fffffff) return TNC_ERR_ARG;
-  unsigned gz = (unsigned)(batch < 65535 ? batch : 65535);
-  dim3 grid((unsigned)gx, (unsigned)gy, gz);
-  // A is K-contiguous for N / R, B for T / C
-  const bool aK = (opA == TNC_OP_N || opA == TNC_OP_R), bK = (opB == TNC_OP_T || opB == TNC_OP_C);
-  const bool aC = (opA == TNC_OP_C || opA == TNC_OP_R), bC = (opB == TNC_OP_C || opB == TNC_OP_R);
-#define TNC_GEMM_LAUNCH(AKV, BKV)                                                                              \
-  gemm_simt_kernel<T, AKV, BKV><<<grid, 256, 0, st>>>(m, n, k, aC, bC, alpha, A, lda, sA, B, ldb, sB, beta, C, \
-                                                      ldc, sC, batch)
-  if (aK && bK) TNC_GEMM_LAUNCH(true, true);
-  else if (aK) TNC_GEMM_LAUNCH(true, false);
-  else if (bK) TNC_GEMM_LAUNCH(false, true);
-  else TNC_GEMM_LAUNCH(false, false);
-#undef TNC_GEMM_LAUNCH
-  return launch_status();
+  if ((m + 63) / 64 > 65535) return TNC_ERR_ARG;
+  if constexpr (Tile64<T>::WIDE) {
+    auto tiles = [&](int bm, int bn) { return ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch; };
+    switch (wide_tile(tiles)) {
+      case kTileS: return simt_launch<T, TileS<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+      case kTileM: return simt_launch<T, TileM<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+      default: return simt_launch<T, TileL<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+    }
+  } else {
+    return simt_launch<T, Tile64<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+  }
 }
 
 template int gemm_launch<float>(int, int, int64_t, int64_t, int64_t, float, const float*, int64_t, int64_t,
