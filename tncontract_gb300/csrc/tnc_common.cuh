@@ -21,6 +21,7 @@ constexpr long long kSpinLimitDefault = 1LL << 24;
 int spin_limit_set_qr(long long polls);
 int spin_limit_set_svd(long long polls);
 int spin_limit_set_rows(long long polls);
+int spin_limit_set_j32(long long polls);
 int spin_limit_set_tc(long long polls);
 
 // ---------------------------------------------------------------- complex

@@ -260,4 +260,13 @@ inline int coop_capacity(const void* kernel, int threads, size_t smem) {
   return cap;
 }
 
+// Single-precision block Jacobi (tnc_jacobi32.cu) of the nr rows of W (length L
+// >= nr, at most 1024), with the rotations accumulated in J's rows of the same
+// length unless J is null (L <= 512 then).  Counters: 2 x 100 + nr words and the
+// SyncWords, zeroed by the caller; Dn: nr floats; frob2: the rows' squared norm.
+template <typename T>
+int jacobi32_rows(T* W, T* J, int64_t nr, int64_t L, int h, int max_sweeps, double tol, double stop_tol,
+                  const double* frob2, float* Dn, unsigned* counters, SyncWords* sw, int* info, int64_t nkeep,
+                  cudaStream_t st);
+
 }  // namespace tnc

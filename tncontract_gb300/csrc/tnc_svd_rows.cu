@@ -14,19 +14,20 @@
 //   phase 0 -- every half-block is loaded into shared memory by one CTA and
 //              all pairs inside it are rotated (an h-point round-robin);
 //   rounds  -- a round-robin tournament over the half-blocks; in each round a
-//              CTA takes a half-block pair (P, Q), keeps the rows of P in
-//              registers (warp i owns row i of P) and the rows of Q in shared
-//              memory, and rotates every (P_i, Q_j) pair in h steps (step s:
-//              warp i pairs with Q_{(i+s) mod h}).
+//              CTA takes a half-block pair (P, Q) into shared memory and rotates
+//              every (P_i, Q_j) pair in h steps (step s: warp i pairs P_i with
+//              Q_{(i+s) mod h}).
+// This kernel runs FP64 and double-float rows; single-precision ones have their
+// own (tnc_jacobi32.cuh).
 // A task of one step (phase 0 or a round) waits only for the tasks of the
 // previous step that wrote its two half-blocks (a step counter per
 // half-block); one grid barrier per sweep closes it for the convergence test.
 // That is 2n/h dependent steps per sweep instead of n for a point ordering,
-// and each rotation streams its rows through registers and shared memory
-// instead of L2.  One cooperative launch runs all sweeps; every wait is
+// and each rotation streams its rows through shared memory instead of L2.  One cooperative launch runs all sweeps; every wait is
 // bounded (tnc_persist.cuh).
 #include "tnc_df.cuh"
 #include "tnc_persist.cuh"
+#include "tnc_rot.cuh"
 
 #include <atomic>
 #include <type_traits>
@@ -44,131 +45,11 @@ __device__ __forceinline__ void circle_pair(int64_t np, int64_t r, int64_t i, in
   else { p = (r + i) % mod; q = (r - i + mod) % mod; }
 }
 
-template <typename T>
-struct Rot {
-  typename traits<T>::real c, th;  // th = t |g|: the norms move to a - th, b + th
-  T se, sec;
-  bool apply;
-  bool big;  // |g| > stol sqrt(a b): above the stage-stop tolerance
-};
-
-// Jacobi rotation from the 2x2 Gram entries (see tnc_svd.cu for the formula)
-template <typename T>
-__device__ __forceinline__ Rot<T> make_rot_ieee(typename traits<T>::real a, typename traits<T>::real b, T g,
-                                                typename traits<T>::real rtol, typename traits<T>::real noise2,
-                                                typename traits<T>::real stol) {
-  typedef typename traits<T>::real R;
-  Rot<T> r;
-  const R h = abs_(g);
-  const R sab = sqrt(a) * sqrt(b);
-  // rows at the rounding-noise floor (or whose squared norm underflowed) count as converged
-  r.apply = (a > noise2) && (b > noise2) && (a > 0) && (b > 0) && (h > rtol * sab);
-  r.big = r.apply && h > stol * sab;
-  if (!r.apply) { r.c = 1; r.th = 0; r.se = zero_<T>(); r.sec = zero_<T>(); return r; }
-  const R tau = (b - a) / (2 * h);
-  R t;
-  if (fabs(tau) > (R)1e15) t = (R)0.5 / tau;
-  else t = (tau >= 0 ? R(1) : R(-1)) / (fabs(tau) + sqrt(R(1) + tau * tau));
-  r.c = R(1) / sqrt(R(1) + t * t);
-  r.th = t * h;
-  const R s = r.c * t;
-  const R inv_h = R(1) / h;  // one division for both parts of e = g / |g|
-  const T e = isfinite(inv_h) ? g * inv_h : div_real_(g, h);
-  r.se = s * e;
-  r.sec = s * conj_(e);
-  return r;
-}
-
-// The same rotation for single-precision rows with a shorter dependency
-// chain (the rotation parameters are on the critical path of every Jacobi
-// step): the tests compare squares (|g|^2 > tol^2 a b, no square roots),
-// |g| is one square root of |g|^2 instead of a hypot, and the divisions of
-// 1/|g|, tau, t and c become a product and correctly rounded reciprocals.  Every rounding stays round-to-nearest, so
-// the rotations carry no systematic bias (|e| = 1 and c^2 + s^2 = 1 to an
-// ulp either side; a Newton-refined hardware estimate here drifted the FP32
-// sweep's discarded weights by 1.5e-6).  Operands whose squares or products
-// leave the comfortable FP32 range take the IEEE formula.
-template <typename T>
-__device__ __forceinline__ Rot<T> make_rot(typename traits<T>::real a, typename traits<T>::real b, T g,
-                                           typename traits<T>::real rtol, typename traits<T>::real noise2,
-                                           typename traits<T>::real stol = 0) {
-  typedef typename traits<T>::real R;
-  if constexpr (sizeof(R) != 4) {
-    return make_rot_ieee<T>(a, b, g, rtol, noise2, stol);
-  } else {
-    const float h2 = abs2_(g), ab = a * b;
-    if (!(h2 > 1e-30f && h2 < 1e30f && ab > 1e-30f && ab < 1e30f))
-      return make_rot_ieee<T>(a, b, g, rtol, noise2, stol);
-    Rot<T> r;
-    r.apply = (a > noise2) && (b > noise2) && (h2 > (rtol * rtol) * ab);
-    r.big = r.apply && h2 > (stol * stol) * ab;
-    if (!r.apply) { r.c = 1; r.th = 0; r.se = zero_<T>(); r.sec = zero_<T>(); return r; }
-    // |g| and 1/|g| by correctly rounded FP32 operations (sqrt.rn, rcp.rn):
-    // a correctly rounded reciprocal square root has no FP32 instruction and
-    // would be emulated on GB300's slow FP64 pipe
-    const float hg = sqrtf(h2);
-    const float ih = __frcp_rn(hg);
-    const float tau = (b - a) * 0.5f * ih;
-    const float at = fabsf(tau);
-    float t;
-    if (at > 1e15f) {
-      t = 0.5f / tau;
-    } else {
-      t = copysignf(__frcp_rn(at + sqrtf(fmaf(tau, tau, 1.f))), tau);
-    }
-    const float c = __frcp_rn(sqrtf(fmaf(t, t, 1.f)));
-    const float s = c * t;
-    r.c = c;
-    r.th = t * hg;
-    const T e = g * ih;
-    r.se = s * e;
-    r.sec = s * conj_(e);
-    return r;
-  }
-}
-
-// rows x (registers, MAXE per lane) and y (shared memory), one warp.  The
-// squared norms a (of x) and *b (of y) are carried, not recomputed: only
-// g = <x, y> is reduced, and a rotation moves them to a - t|g|, b + t|g|
-// (exact in exact arithmetic; recomputed from the rows once per sweep).
-// Returns 0 (no rotation), 1 (a rotation) or 3 (a rotation above stol).
-template <typename T, int MAXE>
-__device__ __forceinline__ int rotate_reg_smem(T (&x)[MAXE], T* y, int64_t L, typename traits<T>::real rtol,
-                                               typename traits<T>::real noise2, typename traits<T>::real& a,
-                                               typename traits<T>::real* b, typename traits<T>::real stol) {
-  typedef typename traits<T>::real R;
-  const int lane = threadIdx.x & 31;
-  const int Li = (int)L;  // row length <= 32 * MAXE
-  T g0 = zero_<T>(), g1 = zero_<T>();
-  T yr[MAXE];  // the partner row stays in registers between the two passes
-#pragma unroll
-  for (int u = 0; u < MAXE; ++u) {
-    const int k = lane + 32 * u;
-    yr[u] = (k < Li) ? y[k] : zero_<T>();
-  }
-#pragma unroll
-  for (int u = 0; u < MAXE; ++u) {
-    if (u & 1) fma_(g1, x[u], conj_(yr[u]));
-    else fma_(g0, x[u], conj_(yr[u]));
-  }
-  const T g = warp_sum(g0 + g1);
-  const R bb = *b;
-  const Rot<T> r = make_rot<T>(a, bb, g, rtol, noise2, stol);
-  if (!r.apply) return 0;
-#pragma unroll
-  for (int u = 0; u < MAXE; ++u) {
-    const int k = lane + 32 * u;
-    const T xv = x[u];
-    x[u] = r.c * xv - r.se * yr[u];
-    if (k < Li) y[k] = r.sec * xv + r.c * yr[u];
-  }
-  a = a - r.th;
-  if (lane == 0) *b = bb + r.th;
-  return r.big ? 3 : 1;
-}
-
-// rows x and y both in shared memory, one warp; squared norms *a, *b carried;
-// returns as rotate_reg_smem
+// rows x and y in shared memory, one warp.  The squared norms *a (of x) and *b
+// (of y) are carried, not recomputed: only g = <x, y> is reduced, and a rotation
+// moves them to a - t|g|, b + t|g| (exact in exact arithmetic; recomputed from
+// the rows once per sweep).  Returns 0 (no rotation), 1 (a rotation) or 3 (a
+// rotation above stol).
 template <typename T>
 __device__ __forceinline__ int rotate_smem_smem(T* x, T* y, int64_t L, typename traits<T>::real rtol,
                                                 typename traits<T>::real noise2, typename traits<T>::real* a,
@@ -456,29 +337,23 @@ __device__ __forceinline__ bool wait_steps(const unsigned* ver, int64_t P, int64
   return ok != 0;
 }
 
-// FP32 rows of up to 512 elements in 256-thread CTAs are held to 128 registers
-// so two CTAs fit on one SM: the kernel is latency-bound (8 warps, dependent
-// rotation steps), and concurrent factorisations on other streams fill the
-// second slot.  The bound costs a few spilled registers.
-// FP64 rows (PREG = false) keep both half-blocks in shared memory and the
-// kernel at 128 registers: its rotations are bound by the FP64 pipe (1.6 FMA a
-// clock per SM on GB300, measured), not by shared-memory traffic, and the other
-// half of the register file stays free for an FP32 kernel of another instance
-// on the same SM (a register-resident FP64 row took all 255 registers a
-// thread, so nothing else could share the SM).  Double-float rows fill the
-// shared memory of an SM with one CTA (2 x 8 rows of 512 16-byte elements)
-// and keep the registers of their Dot2 chains (held to 128 registers the
-// complex kernel spills 144 bytes and took 6.8 against 4.8 ms at 512 x 512;
-// the sweep fell from 4.98 to 4.54 sweeps/s although an FP32 CTA then fits
-// beside it).
-template <typename T, int MAXE, int MAXT, bool PREG>
+// Both half-blocks lie in shared memory.  FP64 rows: at 128 registers (two CTAs
+// an SM); the rotations are bound by the FP64 pipe (1.6 FMA a clock per SM on
+// GB300, measured), not by shared-memory traffic, and the other half of the
+// register file stays free for an FP32 kernel of another instance on the same
+// SM.  Double-float rows fill the shared memory of an SM with one CTA (2 x 8
+// rows of 512 16-byte elements) and keep the registers of their Dot2 chains
+// (held to 128 registers the complex kernel spills 144 bytes and took 6.8
+// against 4.8 ms at 512 x 512; the sweep fell from 4.98 to 4.54 sweeps/s
+// although an FP32 CTA then fits beside it).
+constexpr int kBlockThreads = 256;
+template <typename T>
 constexpr int jacobi_min_blocks() {
-  if (std::is_same<T, dfc>::value || std::is_same<T, dfr>::value) return 1;
-  return (!PREG || (MAXT == 256 && MAXE <= 16 && sizeof(typename traits<T>::real) == 4)) ? 2 : 1;
+  return (std::is_same<T, dfc>::value || std::is_same<T, dfr>::value) ? 1 : 2;
 }
 
-template <typename T, int MAXE, int MAXT, bool PREG>
-__global__ void __launch_bounds__(MAXT, jacobi_min_blocks<T, MAXE, MAXT, PREG>())
+template <typename T>
+__global__ void __launch_bounds__(kBlockThreads, jacobi_min_blocks<T>())
 jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double tol, const double* frob2,
                     typename traits<T>::real* Dn, unsigned* counters, unsigned* ver, SyncWords* sw, int* info,
                     int64_t nkeep, double stop_tol) {
@@ -500,7 +375,6 @@ jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double t
   int sweep = 0;
   bool converged = false, staged = false;
   unsigned last_rot = 0;
-  T x[PREG ? MAXE : 1];
   for (; sweep < max_sweeps; ++sweep) {
     unsigned rot = 0, rotb = 0;
     // step index of this sweep's phase 0; a sweep is nbp steps (phase 0 and
@@ -556,64 +430,28 @@ jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double t
         }
         const int64_t q0 = Q * h;
         const int cntB = (int)((nr - q0) < h ? (nr - q0) : h);
-        if constexpr (PREG) {
-          const int64_t rowA = P * h + warp;
-          const bool hasA = rowA < nr;
-          R an = 0;
-          if (hasA) {
-#pragma unroll
-            for (int u = 0; u < MAXE; ++u) {
-              const int64_t k = lane + 32 * u;
-              x[u] = (k < L) ? ldcg(W + rowA * L + k) : zero_<T>();
-            }
-            an = ldcg(Dn + rowA);
+        T* sA = sB + (int64_t)h * L;
+        const int64_t p0 = P * h;
+        const int cntA = (int)((nr - p0) < h ? (nr - p0) : h);
+        rows_to_smem(W, p0, cntA, L, sA);
+        rows_to_smem(W, q0, cntB, L, sB);
+        if (threadIdx.x < cntA) snA[threadIdx.x] = ldcg(Dn + p0 + threadIdx.x);
+        if (threadIdx.x < cntB) sn[threadIdx.x] = ldcg(Dn + q0 + threadIdx.x);
+        __syncthreads();
+        for (int s = 0; s < h; ++s) {
+          const int j = (warp + s) % h;
+          if (warp < cntA && j < cntB) {
+            const int rr = rotate_smem_smem(sA + (int64_t)warp * L, sB + (int64_t)j * L, L, rtol, noise2,
+                                            &snA[warp], &sn[j], stol);
+            rot += (unsigned)(rr & 1);
+            rotb += (unsigned)(rr >> 1);
           }
-          rows_to_smem(W, q0, cntB, L, sB);
-          if (threadIdx.x < cntB) sn[threadIdx.x] = ldcg(Dn + q0 + threadIdx.x);
           __syncthreads();
-          for (int s = 0; s < h; ++s) {
-            const int j = (warp + s) % h;
-            if (hasA && j < cntB) {
-              const int rr = rotate_reg_smem<T, MAXE>(x, sB + (int64_t)j * L, L, rtol, noise2, an, &sn[j], stol);
-              rot += (unsigned)(rr & 1);
-              rotb += (unsigned)(rr >> 1);
-            }
-            __syncthreads();
-          }
-          if (hasA) {
-#pragma unroll
-            for (int u = 0; u < MAXE; ++u) {
-              const int64_t k = lane + 32 * u;
-              if (k < L) stcg(W + rowA * L + k, x[u]);
-            }
-            if (lane == 0) stcg(Dn + rowA, an);
-          }
-          rows_from_smem(W, q0, cntB, L, sB);
-          if (threadIdx.x < cntB) stcg(Dn + q0 + threadIdx.x, sn[threadIdx.x]);
-        } else {
-          T* sA = sB + (int64_t)h * L;
-          const int64_t p0 = P * h;
-          const int cntA = (int)((nr - p0) < h ? (nr - p0) : h);
-          rows_to_smem(W, p0, cntA, L, sA);
-          rows_to_smem(W, q0, cntB, L, sB);
-          if (threadIdx.x < cntA) snA[threadIdx.x] = ldcg(Dn + p0 + threadIdx.x);
-          if (threadIdx.x < cntB) sn[threadIdx.x] = ldcg(Dn + q0 + threadIdx.x);
-          __syncthreads();
-          for (int s = 0; s < h; ++s) {
-            const int j = (warp + s) % h;
-            if (warp < cntA && j < cntB) {
-              const int rr = rotate_smem_smem(sA + (int64_t)warp * L, sB + (int64_t)j * L, L, rtol, noise2,
-                                              &snA[warp], &sn[j], stol);
-              rot += (unsigned)(rr & 1);
-              rotb += (unsigned)(rr >> 1);
-            }
-            __syncthreads();
-          }
-          rows_from_smem(W, p0, cntA, L, sA);
-          if (threadIdx.x < cntA) stcg(Dn + p0 + threadIdx.x, snA[threadIdx.x]);
-          rows_from_smem(W, q0, cntB, L, sB);
-          if (threadIdx.x < cntB) stcg(Dn + q0 + threadIdx.x, sn[threadIdx.x]);
         }
+        rows_from_smem(W, p0, cntA, L, sA);
+        if (threadIdx.x < cntA) stcg(Dn + p0 + threadIdx.x, snA[threadIdx.x]);
+        rows_from_smem(W, q0, cntB, L, sB);
+        if (threadIdx.x < cntB) stcg(Dn + q0 + threadIdx.x, sn[threadIdx.x]);
         publish_steps(ver, P, Q, g + 1u);
       }
     }
@@ -995,28 +833,28 @@ template <> int dtype_code<c128>() { return TNC_C128; }
 // different row lengths share the setting).
 static const size_t kMaxHalfBlockBytes = 200 * 1024;
 
-template <typename T, int MAXE, int MAXT, bool PREG>
+template <typename T>
 static int ensure_smem_attr() {
   static std::atomic<unsigned long long> done_mask{0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return TNC_ERR_CUDA;
   const unsigned long long bit = 1ull << (dev & 63);
   if (done_mask.load() & bit) return TNC_OK;
-  if (cudaFuncSetAttribute((const void*)jacobi_block_kernel<T, MAXE, MAXT, PREG>,
+  if (cudaFuncSetAttribute((const void*)jacobi_block_kernel<T>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxHalfBlockBytes) != cudaSuccess)
     return TNC_ERR_CUDA;
   done_mask.fetch_or(bit);
   return TNC_OK;
 }
 
-template <typename T, int MAXE, int MAXT, bool PREG = true>
+template <typename T>
 static int launch_block(T* W, int64_t nr, int64_t L, int h, int ms, double tol, const double* frob2,
                         typename traits<T>::real* Dn, unsigned* counters, SyncWords* sw, int* info, int64_t nkeep,
                         cudaStream_t st, double stop_tol = 0.0) {
-  const size_t smem = (size_t)(PREG ? 1 : 2) * h * L * sizeof(T);
-  const void* fn = (const void*)jacobi_block_kernel<T, MAXE, MAXT, PREG>;
-  if (smem > kMaxHalfBlockBytes || 32 * h > MAXT) return TNC_ERR_ARG;
-  if (int rc = ensure_smem_attr<T, MAXE, MAXT, PREG>()) return rc;
+  const size_t smem = (size_t)2 * h * L * sizeof(T);
+  const void* fn = (const void*)jacobi_block_kernel<T>;
+  if (smem > kMaxHalfBlockBytes || 32 * h > kBlockThreads) return TNC_ERR_ARG;
+  if (int rc = ensure_smem_attr<T>()) return rc;
   const int threads = 32 * h;
   int cap = coop_capacity(fn, threads, smem);
   if (cap <= 0) return TNC_ERR_CUDA;
@@ -1112,46 +950,23 @@ static int svd_rows_impl(int64_t m, int64_t n, const T* A, T* W, typename traits
     if (cudaMemsetAsync(frob2, 0, sizeof(double), st) != cudaSuccess) return TNC_ERR_CUDA;
     frob2_kernel<T><<<grid1d(nr * L, 256, 152 * 4), 256, 0, st>>>(nr * L, W, frob2);
     ++launched;
-    // half-block height: 16 rows (fewest barriers) when the shared-memory half
-    // block and the register row fit, else smaller
-    // (16: 512-thread CTAs, rows up to 512 and element types up to 8 bytes)
     int h = 8;
     if (block_rows == 2 || block_rows == 4 || block_rows == 8) h = block_rows;
-    if (block_rows == 16 && L <= 512 && sizeof(T) <= 8) h = 16;
-    while (h > 2 && (size_t)h * L * sizeof(T) > kMaxHalfBlockBytes) h >>= 1;
-    while (h > 2 && h / 2 >= nr) h >>= 1;
-    const bool big = sizeof(T) >= 16;
-    // single-precision rows: the Gram-form block update on request (measured
-    // slower than the row-by-row kernel at 512 x 512 complex64: 14.5 against
-    // 9.7 ms; it executes 2.7x the FMAs and keeps the per-task L2 round trip)
-    const bool gram = sizeof(R) == 4 && block_rows == TNC_ROWS_GRAM && h == kGramH &&
-                      gram_smem_bytes<T>(L) <= kMaxHalfBlockBytes;
     int rc;
-    if (gram) {
-      if constexpr (sizeof(R) == 4)
+    if constexpr (sizeof(R) == 4) {
+      // single-precision rows: the Gram-form block update on request (measured
+      // slower than the row-by-row kernel; it executes 2.7x the FMAs and keeps
+      // the per-task L2 round trip)
+      if (block_rows == TNC_ROWS_GRAM && (nr > kGramH / 2) && gram_smem_bytes<T>(L) <= kMaxHalfBlockBytes)
         rc = launch_gram<T>(W, nr, L, max_sweeps, tol, frob2, counters, sw, info, nkeep, st, stop_tol);
-      else return TNC_ERR_ARG;
-    } else if (sizeof(typename traits<T>::real) == 8 && L <= 512) {
-      // FP64 rows: both half-blocks in shared memory (2 h L elements)
-      if (h > 8) h = 8;
-      while (h > 2 && (size_t)2 * h * L * sizeof(T) > kMaxHalfBlockBytes) h >>= 1;
-      rc = launch_block<T, 1, 256, false>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-    } else if (h == 16) {
-      if constexpr (sizeof(T) <= 8) {
-        if (L <= 256) rc = launch_block<T, 8, 512>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-        else rc = launch_block<T, 16, 512>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-      } else {
-        return TNC_ERR_ARG;
-      }
-    } else if (L <= 256) {
-      rc = launch_block<T, 8, 256>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-    } else if (L <= 512) {
-      rc = launch_block<T, 16, 256>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-    } else if (L <= 1024 && !big) {
-      if constexpr (sizeof(T) < 16) rc = launch_block<T, 32, 256>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
-      else return TNC_ERR_ARG;
+      else
+        rc = jacobi32_rows<T>(W, nullptr, nr, L, block_rows == 16 ? 16 : h, max_sweeps, tol, stop_tol, frob2, Dn,
+                              counters, sw, info, nkeep, st);
     } else {
-      return TNC_ERR_ARG;  // rows too long for the register-resident half block
+      while (h > 2 && (size_t)2 * h * L * sizeof(T) > kMaxHalfBlockBytes) h >>= 1;
+      while (h > 2 && h / 2 >= nr) h >>= 1;
+      if (L > (sizeof(T) >= 16 ? 512 : 1024)) return TNC_ERR_ARG;  // rows too long
+      rc = launch_block<T>(W, nr, L, h, max_sweeps, tol, frob2, Dn, counters, sw, info, nkeep, st, stop_tol);
     }
     if (rc) return rc;
     ++launched;
@@ -1315,7 +1130,7 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
     while (h > 2 && (size_t)2 * h * L * sizeof(Tdf) > kMaxHalfBlockBytes) h >>= 1;
     while (h > 2 && h / 2 >= nr) h >>= 1;
     if ((size_t)2 * h * L * sizeof(Tdf) > kMaxHalfBlockBytes) return TNC_ERR_ARG;  // rows too long
-    if (int rc = launch_block<Tdf, 1, 256, false>(W, nr, L, h, max_sweeps, tol, frob2 + 1, Dn, counters, sw, info,
+    if (int rc = launch_block<Tdf>(W, nr, L, h, max_sweeps, tol, frob2 + 1, Dn, counters, sw, info,
                                                  nkeep, st, kDfStopTol))
       return rc;
     ++launched;
@@ -1419,6 +1234,7 @@ extern "C" int tnc_set_spin_limit(long long polls) {
   if (int rc = spin_limit_set_qr(polls)) return rc;
   if (int rc = spin_limit_set_svd(polls)) return rc;
   if (int rc = spin_limit_set_rows(polls)) return rc;
+  if (int rc = spin_limit_set_j32(polls)) return rc;
   return spin_limit_set_tc(polls);
 }
 
