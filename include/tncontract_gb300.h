@@ -229,13 +229,18 @@ int tnc_qr_r(int dtype, int64_t m, int64_t n, const void *A, int adjoint,
  * values sorted descending (float for F32/C64, double for F64/C128), VH is
  * k x n, k = min(m, n).  QR-preconditioned one-sided (Hestenes) Jacobi:
  * the k x k triangular factor of A^H (wide A) or A (tall A) is
- * orthogonalised with a round-robin ordering by one persistent cooperative
- * launch, rotations accumulated; U and VH follow with one GEMM against Q,
- * both orthonormal however graded the spectrum.  max_sweeps <= 0 selects
- * 40; tol <= 0 selects sqrt(k) * eps (4x that for FP32 storage).  info
- * (device, 4 ints):
+ * orthogonalised by persistent cooperative launches, rotations accumulated;
+ * U and VH follow with one GEMM against Q, both orthonormal however graded
+ * the spectrum.  24 <= k <= 512: F32 / C64 run the block Jacobi of
+ * tnc_svd_rows; F64 / C128 run it on a single-precision copy and refine its
+ * rotations in FP64 products until the rows meet tol, an FP64 Jacobi taking
+ * what is left.  U and VH serve as scratch before they are written: they must
+ * not overlap A, each other or the workspace.  max_sweeps <= 0 selects
+ * 40 (below 20: the FP64 Jacobi alone for F64 / C128); tol <= 0 selects
+ * sqrt(k) * eps (4x that for FP32 storage).  info (device, 4 ints):
  * [0] status (TNC_OK / TNC_ERR_NOT_CONVERGED / TNC_ERR_NONFINITE /
- * TNC_ERR_TIMEOUT), [1] sweeps used, [2] rotations in the last sweep.
+ * TNC_ERR_TIMEOUT), [1] sweeps used (of the Jacobi that ended the work),
+ * [2] rotations in the last sweep.
  * Replaces np.linalg.svd(full_matrices=False) in tensor_svd (tensor.py:915)
  * and its scipy gesvd retry (tensor.py:916-929). */
 int tnc_svd_workspace_size(int dtype, int64_t m, int64_t n, size_t *bytes);

@@ -1,6 +1,10 @@
 // Thin SVD (np.linalg.svd(full_matrices=False) in tensor_svd,
 // tncontract/tensor.py:915, and its scipy gesvd retry, :916-929).
 //
+// 24 to 512 rows: the block Jacobi of single-precision rows (tnc_jacobi32.cuh)
+// with accumulated rotations, refined in FP64 for FP64 types (tnc_svd_refine.cuh).
+// Other sizes, and what the refinement leaves, run the kernel below.
+//
 // One-sided (Hestenes) Jacobi on the ROWS of a working matrix W (nr x nr):
 // pairs of rows are rotated until all rows are mutually orthogonal to within
 // tol.  The rotations are accumulated into J (nr x nr, rows), so
@@ -21,6 +25,7 @@
 // This is the 2x2 Hermitian Jacobi rotation of the Gram matrix [[a,g],[g*,b]]
 // (Golub & Van Loan, sec. 8.5 and 8.6.3), applied to rows.
 #include "tnc_persist.cuh"
+#include "tnc_svd_refine.cuh"
 
 namespace tnc {
 
@@ -36,8 +41,9 @@ __device__ __forceinline__ void pair_indices(int64_t np, int64_t r, int64_t i, i
 template <typename T>
 __global__ void __launch_bounds__(kSvdWarps * 32)
 jacobi_kernel(T* W, T* J, int64_t nr, int64_t L, int max_sweeps, double tol, const double* frob2,
-              unsigned* counters, SyncWords* sw, int* info) {
+              unsigned* counters, SyncWords* sw, int* info, const RefineState* refined) {
   typedef typename traits<T>::real R;
+  if (refined && refine_done(refined, kRefineSteps + 1)) return;  // nothing left to rotate
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)blockIdx.x * kSvdWarps + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * kSvdWarps;
@@ -115,14 +121,19 @@ __global__ void row_norms_kernel(const T* W, int64_t nr, int64_t L, typename tra
   }
 }
 
+// Norms compare as the integers of their bits (no sign bit): an FP64 comparison
+// would take 64 cycles of its scheduler.  NaN ranks above every number.
+__device__ __forceinline__ long long norm_bits(double v) { return __double_as_longlong(v) & 0x7fffffffffffffffLL; }
+__device__ __forceinline__ int norm_bits(float v) { return __float_as_int(v) & 0x7fffffff; }
+
 // pos[i] = #{j: D_j > D_i} + #{j < i: D_j == D_i}  (stable descending order)
 template <typename R>
 __global__ void rank_kernel(const R* D, int64_t n, int64_t* pos) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    R di = D[i];
+    const auto di = norm_bits(D[i]);
     int64_t c = 0;
     for (int64_t j = 0; j < n; ++j) {
-      R dj = D[j];
+      const auto dj = norm_bits(D[j]);
       c += (dj > di) || (dj == di && j < i);
     }
     pos[i] = c;
@@ -172,7 +183,7 @@ static SvdLayout svd_layout(int64_t m, int64_t n, int dt, size_t es, size_t rs) 
   Ly.w = off; off = align256(off + (size_t)nr * nr * es);
   Ly.j = off; off = align256(off + (size_t)nr * nr * es);
   Ly.d = off; off = align256(off + (size_t)nr * rs);
-  Ly.frob2 = off; off = align256(off + sizeof(double));
+  Ly.frob2 = off; off = align256(off + sizeof(double) + (kRefineSteps + 1) * sizeof(RefineState));
   Ly.pos = off; off = align256(off + (size_t)nr * sizeof(int64_t));
   Ly.counters = off; off = align256(off + kMaxSweepsCap * sizeof(unsigned));
   Ly.sync = off; off = align256(off + sizeof(SyncWords));
@@ -185,6 +196,88 @@ template <> int dtype_of<float>() { return TNC_F32; }
 template <> int dtype_of<double>() { return TNC_F64; }
 template <> int dtype_of<c64>() { return TNC_C64; }
 template <> int dtype_of<c128>() { return TNC_C128; }
+
+// Sizes of the single-precision Jacobi and the refinement (tnc_svd_refine.cuh):
+// below kSvdRefineMin rows their launches cost what the FP64 Jacobi takes, and the
+// scratch they keep in the QR's copy of the matrix would not fit; 512 is the
+// Jacobi's longest row with an accumulator.  A caller's sweep cap below
+// kSvdRefineSweeps is one of the FP64 Jacobi's.
+constexpr int64_t kSvdRefineMin = 24;
+constexpr int kSvdRefineSweeps = 20;
+constexpr int kSvdRefineSweeps32 = 14;
+constexpr double kSvdRefineTol32 = 3e-6, kSvdRefineStop32 = 1e-3;
+
+// The single-precision Jacobi's words: counters (2 x 100 + nr), norms, status.
+struct Jacobi32Scratch {
+  unsigned* counters;
+  float* Dn;
+  SyncWords* sw;
+  int* info;
+  double* f2;
+  unsigned* rows_large;
+  size_t bytes;
+};
+static Jacobi32Scratch jacobi32_scratch(char* p, int64_t nr) {
+  Jacobi32Scratch s;
+  s.f2 = (double*)p;  // [0] of R, [1] of the scaled copy
+  s.sw = (SyncWords*)(p + 16);
+  s.info = (int*)(p + 16 + sizeof(SyncWords));
+  s.counters = (unsigned*)(s.info + 4);
+  s.Dn = (float*)(s.counters + 200 + nr);
+  s.rows_large = (unsigned*)(s.Dn + nr);
+  s.bytes = (size_t)((char*)(s.rows_large + nr) - p + 15) & ~size_t(15);
+  return s;
+}
+
+// The single-precision Jacobi's status for one that is the whole SVD's.
+static __global__ void jacobi32_status(const SyncWords* sw, const int* from, int* info) {
+  if (sw->err) info[0] = sw->err;
+  else if (from[0]) info[0] = from[0];
+  info[1] = from[1];
+  info[2] = from[2];
+}
+// ... and for one whose result is refined (its sweeps counted; a stall is no error).
+static __global__ void jacobi32_refined_status(const SyncWords* sw, const int* from, int* info) {
+  if (sw->err) info[0] = sw->err;
+  info[1] = from[1];
+}
+
+// R (nr x nr) -> J and Wb = J R with orthogonal rows, or as near as the steps came;
+// rs (zeroed) tells the FP64 Jacobi whether anything is left.  GF: nr^2 elements;
+// scratch: nr^2 elements (the words above, then F in single precision).
+template <typename T>
+static int svd_refine(int64_t nr, const T* R, T* J, T* Wb, T* GF, char* scratch, typename traits<T>::real* a,
+                      typename traits<T>::real* d, RefineState* rs, double tol, const double* frob2, int* info,
+                      cudaStream_t st, int* launched) {
+  typedef typename narrow_of<T>::type S;
+  const Jacobi32Scratch js = jacobi32_scratch(scratch, nr);
+  S *W32 = (S*)GF, *J32 = W32 + nr * nr, *Ft = (S*)(scratch + js.bytes);
+  const unsigned g = grid1d(nr * nr, 256);
+  if (cudaMemsetAsync(scratch, 0, js.bytes, st) != cudaSuccess) return TNC_ERR_CUDA;
+  if (cudaMemcpyAsync(js.f2, frob2, sizeof(double), cudaMemcpyDeviceToDevice, st) != cudaSuccess) return TNC_ERR_CUDA;
+  refine_split_kernel<T><<<g, 256, 0, st>>>(nr, R, W32, J32, js.f2);
+  if (int rc = jacobi32_rows<S>(W32, J32, nr, nr, 8, kSvdRefineSweeps32, kSvdRefineTol32, kSvdRefineStop32, js.f2 + 1,
+                                js.Dn, js.counters, js.sw, js.info, nr, st))
+    return rc;
+  jacobi32_refined_status<<<1, 1, 0, st>>>(js.sw, js.info, info);
+  refine_widen_kernel<T><<<g, 256, 0, st>>>(nr * nr, J32, J);
+  typedef TileS<T> G;
+  const int64_t rows = (nr + G::BM - 1) / G::BM, cols = (nr + G::BN - 1) / G::BN;
+  int64_t half = 0;
+  for (int64_t c = 0; c < cols; ++c) half += 2 * (c + 1) < rows ? 2 * (c + 1) : rows;
+  refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, 0);
+  for (int s = 0; s <= kRefineSteps; ++s) {
+    refine_gram_kernel<T><<<dim3((unsigned)half, 2), G::THR, 0, st>>>(nr, Wb, J, GF, a, d, rs, s, js.rows_large);
+    refine_test_kernel<T><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, rs, s, js.rows_large);
+    if (s == kRefineSteps) break;
+    refine_f_kernel<T><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, GF, a, d, frob2, tol, rs, s, js.rows_large, Ft);
+    if (nr <= 128) refine_apply_kernel<T, 1><<<dim3((unsigned)nr, 2), 256, nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
+    else refine_apply_kernel<T, 4><<<dim3((unsigned)((nr + 3) / 4), 2), 256, 4 * nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
+    refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, s + 1);
+  }
+  *launched += 5 + 5 * kRefineSteps + 2;
+  return TNC_OK;
+}
 
 // QR-preconditioned one-sided Jacobi (Drmac & Veselic 2008).  X is the
 // matrix whose columns the Jacobi would orthogonalise (X = A^H for a wide A,
@@ -225,16 +318,44 @@ static int svd_impl(int64_t m, int64_t n, const T* A, int64_t lda, T* U, typenam
   int s = qr_qt<T>(L, nr, A, tall ? 0 : 1, true, W, w + Ly.qr, qr_qt_workspace(L, nr, dtype_of<T>()), J, info,
                    st, &Qt);
   if (s) return s;
-  T* small = (T*)(w + Ly.qr);  // the QR's transposed copy (nr * L >= nr * nr elements) is free now
-  eye_kernel<T><<<grid1d(nr * nr, 256), 256, 0, st>>>(J, nr);
+  char* bt = w + Ly.qr;  // the QR's transposed copy (nr * L elements) is free now: scratch, then the small factor
+  T* small = (T*)bt;
   if (cudaMemsetAsync(counters, 0, kMaxSweepsCap * sizeof(unsigned), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(sw, 0, sizeof(SyncWords), st) != cudaSuccess) return TNC_ERR_CUDA;
   // info[0] holds the QR's status (a wait timeout) until the Jacobi writes its own
   if (cudaMemsetAsync(info + 1, 0, 3 * sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
-  if (cudaMemsetAsync(frob2, 0, sizeof(double), st) != cudaSuccess) return TNC_ERR_CUDA;
+  if (cudaMemsetAsync(frob2, 0, sizeof(double) + (kRefineSteps + 1) * sizeof(RefineState), st) != cudaSuccess)
+    return TNC_ERR_CUDA;
   frob2_kernel<T><<<grid1d(nr * nr, 256, 152 * 4), 256, 0, st>>>(nr * nr, W, frob2);
-  if (launch_status(2)) return TNC_ERR_CUDA;  // eye, frob2
-  if (nr > 1) {
+  int launched = 4;  // frob2, then row norms, rank, output
+  const RefineState* refined = nullptr;
+  constexpr bool single = sizeof(R) == 4;
+  const bool fits = nr >= kSvdRefineMin && nr <= 512;
+  const bool fast = fits && (single || max_sweeps >= kSvdRefineSweeps);
+  if (!fast || single) {
+    eye_kernel<T><<<grid1d(nr * nr, 256), 256, 0, st>>>(J, nr);
+    ++launched;
+  }
+  if (fast) {
+    if constexpr (single) {
+      const Jacobi32Scratch js = jacobi32_scratch(bt, nr);
+      if (cudaMemsetAsync(bt, 0, js.bytes, st) != cudaSuccess) return TNC_ERR_CUDA;
+      if (int rc = jacobi32_rows<T>(W, J, nr, nr, 8, max_sweeps, tol, 0.0, frob2, js.Dn, js.counters, js.sw, js.info,
+                                    nr, st))
+        return rc;
+      jacobi32_status<<<1, 1, 0, st>>>(js.sw, js.info, info);
+      launched += 2;
+    } else {
+      // W in the output that is written last, G and delta in the other
+      T* Wb = tall ? U : VH;
+      if (int rc = svd_refine<T>(nr, W, J, Wb, tall ? VH : U, bt, (R*)(w + Ly.d), (R*)pos, (RefineState*)(frob2 + 1),
+                                 tol, frob2, info, st, &launched))
+        return rc;
+      refined = (RefineState*)(frob2 + 1);
+      W = Wb;
+    }
+  }
+  if (nr > 1 && !(fast && single)) {
     const int threads = kSvdWarps * 32;
     int cap = coop_capacity((const void*)jacobi_kernel<T>, threads, 0);
     if (cap <= 0) return TNC_ERR_CUDA;
@@ -245,10 +366,11 @@ static int svd_impl(int64_t m, int64_t n, const T* A, int64_t lda, T* U, typenam
     int ms = max_sweeps;
     double tl = tol;
     void* args[] = {(void*)&W, (void*)&J, (void*)&nr_, (void*)&L_, (void*)&ms, (void*)&tl,
-                    (void*)&frob2, (void*)&counters, (void*)&sw, (void*)&info};
+                    (void*)&frob2, (void*)&counters, (void*)&sw, (void*)&info, (void*)&refined};
     if (cudaLaunchCooperativeKernel((const void*)jacobi_kernel<T>, dim3(grid), dim3(threads), args, 0, st) !=
         cudaSuccess)
       return TNC_ERR_CUDA;
+    ++launched;
   }
   copy_sync_error<<<1, 1, 0, st>>>(sw, info);
   row_norms_kernel<T><<<grid1d(nr * 32, 256), 256, 0, st>>>(W, nr, nr, D, info);
@@ -256,7 +378,7 @@ static int svd_impl(int64_t m, int64_t n, const T* A, int64_t lda, T* U, typenam
   // the square problem's factors: wide -> U = Y^H (out), J -> small; tall -> VH = Y (out), J^H -> small
   if (tall) svd_output_kernel<T><<<grid1d(nr * nr, 256), 256, 0, st>>>(W, J, D, pos, nr, nr, 0, small, S, VH);
   else svd_output_kernel<T><<<grid1d(nr * nr, 256), 256, 0, st>>>(W, J, D, pos, nr, nr, 1, U, S, small);
-  if (launch_status(nr > 1 ? 4 : 3)) return TNC_ERR_CUDA;  // [jacobi], error copy, row norms, rank, output
+  if (launch_status(launched + 1)) return TNC_ERR_CUDA;  // and the error copy
   const T one = one_<T>(), zero = zero_<T>();
   if (tall)  // U (m x n) = Q (small) = (Q^T)^T small
     return gemm_launch<T>(TNC_OP_T, TNC_OP_N, L, nr, nr, one, Qt, L, 0, small, nr, 0, zero, U, nr, 0, 1, st);
