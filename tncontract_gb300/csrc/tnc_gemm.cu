@@ -33,6 +33,105 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, con
     }
 }
 
+// FP32 tile with K split over the S CTAs of a cluster: every CTA multiplies its
+// run of K slices, leaves its 32 x 32 sums in shared memory, and adds up (in the
+// order of K) and writes 32 / S of the tile's rows from all of them.
+template <typename T, bool AK, bool BKM>
+__device__ __forceinline__ void split_tile(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, const T* A,
+                                           int64_t lda, const T* B, int64_t ldb, T beta, T* C, int64_t ldc, int64_t m0,
+                                           int64_t n0, int S, int rank, T (*As)[Tile32<T>::BK * Tile32<T>::LDA],
+                                           T (*Bs)[Tile32<T>::BK * Tile32<T>::LDB], T* part) {
+  typedef Tile32<T> G;
+  const int64_t slices = (K + G::BK - 1) / G::BK;
+  const int64_t k0 = slices * rank / S * G::BK, k1 = slices * (rank + 1) / S * G::BK, kn = (k1 < K ? k1 : K) - k0;
+  T acc[G::TM][G::TN];
+#pragma unroll
+  for (int i = 0; i < G::TM; ++i)
+#pragma unroll
+    for (int j = 0; j < G::TN; ++j) acc[i][j] = zero_<T>();
+  if (kn > 0)
+    gemm_acc<T, G, AK, BKM>(M, N, kn, aC, bC, AK ? A + k0 : A + k0 * lda, lda, BKM ? B + k0 : B + k0 * ldb, ldb, m0, n0,
+                            As, Bs, acc);
+#pragma unroll
+  for (int i = 0; i < G::TM; ++i)
+#pragma unroll
+    for (int j = 0; j < G::TN; ++j) part[tile_row<G>(i) * G::BN + tile_col<G>(j)] = acc[i][j];
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const bool beta_zero = (abs2_(beta) == 0);
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(part);
+  const int rows = G::BM / S;
+  for (int e = threadIdx.x; e < rows * G::BN; e += G::THR) {
+    const int r = rank * rows + e / G::BN, c = e % G::BN;
+    const int64_t gm = m0 + r, gn = n0 + c;
+    if (gm >= M || gn >= N) continue;
+    T sum = zero_<T>();
+    for (int q = 0; q < S; ++q) {
+      uint32_t at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(base + (uint32_t)((r * G::BN + c) * sizeof(T))), "r"(q));
+      T v;
+      if constexpr (traits<T>::is_complex)
+        asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.re), "=f"(v.im) : "r"(at) : "memory");
+      else
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+      sum += v;
+    }
+    T v = alpha * sum;
+    if (!beta_zero) v += beta * C[gm * ldc + gn];
+    C[gm * ldc + gn] = v;
+  }
+  // no CTA leaves, or starts its next tile, while another reads its sums
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ int split_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+
+template <typename T, bool AK, bool BKM>
+__global__ void __launch_bounds__(Tile32<T>::THR)
+gemm_split_kernel(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, const T* __restrict__ A, int64_t lda,
+                  int64_t sA, const T* __restrict__ B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC,
+                  int64_t batch, int S) {
+  typedef Tile32<T> G;
+  __shared__ __align__(16) T As[2][G::BK * G::LDA];
+  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
+  __shared__ T part[G::BM * G::BN];
+  const int64_t n0 = (int64_t)(blockIdx.x / (unsigned)S) * G::BN;
+  const int rank = split_rank();
+  for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z)
+    for (int64_t m0 = (int64_t)blockIdx.y * G::BM; m0 < M; m0 += (int64_t)gridDim.y * G::BM)
+      split_tile<T, AK, BKM>(M, N, K, aC, bC, alpha, A + bz * sA, lda, B + bz * sB, ldb, beta, C + bz * sC, ldc, m0, n0, S,
+                             rank, As, Bs, part);
+}
+
+// CTAs of the cluster that splits K when the 64 x 64 tiles would not fill the chip
+// (0: they do): as many as keep two slices or more each and about four small CTAs
+// an SM.
+template <typename Count>
+static int split_of(Count tiles, int64_t k) {
+  if (tiles(64, 64) >= 152) return 0;
+  const int64_t t = tiles(32, 32);
+  int s = 1;
+  while (s < 8 && t * s * 2 <= 152 * 4 && k >= 64 * s) s *= 2;
+  return s;
+}
+
+static cudaLaunchConfig_t split_config(dim3 grid, int threads, int S, cudaStream_t st, cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)S;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 // FP64 tile of a set of products by the time of the busiest SM: tiles are dealt
 // to 152 SMs and a tile takes BM BN K / 2 cycles of its SM (four times that in
 // complex), so the cost is ceil(tiles / 152) BM BN; the larger tile among equals
@@ -86,8 +185,34 @@ __global__ void __launch_bounds__(G::THR) gemm_grouped_kernel(const __grid_const
   else gemm_tile<T, G, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
 }
 
-template <typename T, typename G>
-static int grouped_launch(GemmGroup& g, cudaStream_t st) {
+template <typename T>
+__global__ void __launch_bounds__(Tile32<T>::THR) gemm_grouped_split_kernel(const __grid_constant__ GemmGroup g, int S) {
+  typedef Tile32<T> G;
+  __shared__ __align__(16) T As[2][G::BK * G::LDA];
+  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
+  __shared__ T part[G::BM * G::BN];
+  const int64_t tile = blockIdx.x / (unsigned)S;
+  int q = 0;
+  while (q + 1 < g.count && tile >= g.p[q + 1].tile0) ++q;
+  const GroupProblem& P = g.p[q];
+  const int64_t t = tile - P.tile0;
+  const int64_t m0 = (t / P.tiles_n) * G::BM, n0 = (t % P.tiles_n) * G::BN;
+  const T alpha = from_pair<T>(P.alpha), beta = from_pair<T>(P.beta);
+  const bool aK = (P.opA == TNC_OP_N || P.opA == TNC_OP_R), bK = (P.opB == TNC_OP_T || P.opB == TNC_OP_C);
+  const bool aC = (P.opA == TNC_OP_C || P.opA == TNC_OP_R), bC = (P.opB == TNC_OP_C || P.opB == TNC_OP_R);
+  const T* A = (const T*)P.A;
+  const T* B = (const T*)P.B;
+  T* C = (T*)P.C;
+  const int rank = split_rank();
+  if (aK && bK) split_tile<T, true, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
+  else if (aK) split_tile<T, true, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
+  else if (bK) split_tile<T, false, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
+  else split_tile<T, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
+}
+
+// Tiles of a shape over the problems of a group, laid out for the kernel.
+template <typename G>
+static int64_t group_tiles(GemmGroup& g) {
   int64_t tiles = 0;
   for (int i = 0; i < g.count; ++i) {
     GroupProblem& q = g.p[i];
@@ -95,6 +220,12 @@ static int grouped_launch(GemmGroup& g, cudaStream_t st) {
     q.tile0 = tiles;
     tiles += q.tiles_n * ((q.m + G::BM - 1) / G::BM);
   }
+  return tiles;
+}
+
+template <typename T, typename G>
+static int grouped_launch(GemmGroup& g, cudaStream_t st) {
+  const int64_t tiles = group_tiles<G>(g);
   if (tiles > 0x7fffffff) return TNC_ERR_ARG;
   gemm_grouped_kernel<T, G><<<(unsigned)tiles, G::THR, 0, st>>>(g);
   return launch_status();
@@ -117,19 +248,27 @@ int gemm_grouped_launch(int count, const tnc_gemm_problem* probs, cudaStream_t s
     q.alpha[0] = p.alpha[0]; q.alpha[1] = p.alpha[1]; q.beta[0] = p.beta[0]; q.beta[1] = p.beta[1];
   }
   if (g.count == 0) return TNC_OK;
+  auto count_tiles = [&](int bm, int bn) {
+    int64_t t = 0;
+    for (int i = 0; i < g.count; ++i) t += ((g.p[i].m + bm - 1) / bm) * ((g.p[i].n + bn - 1) / bn);
+    return t;
+  };
   if constexpr (Tile64<T>::WIDE) {
-    auto count_tiles = [&](int bm, int bn) {
-      int64_t t = 0;
-      for (int i = 0; i < g.count; ++i) t += ((g.p[i].m + bm - 1) / bm) * ((g.p[i].n + bn - 1) / bn);
-      return t;
-    };
     switch (wide_tile(count_tiles)) {
       case kTileS: return grouped_launch<T, TileS<T>>(g, st);
       case kTileM: return grouped_launch<T, TileM<T>>(g, st);
       default: return grouped_launch<T, TileL<T>>(g, st);
     }
   } else {
-    return grouped_launch<T, Tile64<T>>(g, st);
+    int64_t k = 0;
+    for (int i = 0; i < g.count; ++i) k = g.p[i].k > k ? g.p[i].k : k;
+    const int S = split_of(count_tiles, k);
+    if (S == 0) return grouped_launch<T, Tile64<T>>(g, st);
+    cudaLaunchAttribute attr;
+    const int64_t tiles = group_tiles<Tile32<T>>(g);  // at most 4 x 151 with S
+    const cudaLaunchConfig_t cfg = split_config(dim3((unsigned)(tiles * S)), Tile32<T>::THR, S, st, &attr);
+    if (cudaLaunchKernelEx(&cfg, gemm_grouped_split_kernel<T>, g, S) != cudaSuccess) return TNC_ERR_CUDA;
+    return launch_status();
   }
 }
 
@@ -179,15 +318,28 @@ int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, cons
     return launch_status();
   }
   if ((m + 63) / 64 > 65535) return TNC_ERR_ARG;
+  auto tiles = [&](int bm, int bn) { return ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch; };
   if constexpr (Tile64<T>::WIDE) {
-    auto tiles = [&](int bm, int bn) { return ((m + bm - 1) / bm) * ((n + bn - 1) / bn) * batch; };
     switch (wide_tile(tiles)) {
       case kTileS: return simt_launch<T, TileS<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
       case kTileM: return simt_launch<T, TileM<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
       default: return simt_launch<T, TileL<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
     }
   } else {
-    return simt_launch<T, Tile64<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+    const int S = split_of(tiles, k);
+    if (S == 0) return simt_launch<T, Tile64<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
+    typedef Tile32<T> G;  // fewer than 152 tiles of 64 x 64: every count is small
+    const dim3 grid((unsigned)((n + G::BN - 1) / G::BN * S), (unsigned)((m + G::BM - 1) / G::BM), (unsigned)batch);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = split_config(grid, G::THR, S, st, &attr);
+    const bool aK = (opA == TNC_OP_N || opA == TNC_OP_R), bK = (opB == TNC_OP_T || opB == TNC_OP_C);
+    const bool aC = (opA == TNC_OP_C || opA == TNC_OP_R), bC = (opB == TNC_OP_C || opB == TNC_OP_R);
+    const auto fn = aK ? (bK ? gemm_split_kernel<T, true, true> : gemm_split_kernel<T, true, false>)
+                       : (bK ? gemm_split_kernel<T, false, true> : gemm_split_kernel<T, false, false>);
+    if (cudaLaunchKernelEx(&cfg, fn, m, n, k, aC, bC, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, S) !=
+        cudaSuccess)
+      return TNC_ERR_CUDA;
+    return launch_status();
   }
 }
 
