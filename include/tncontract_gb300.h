@@ -418,6 +418,35 @@ int tnc_sweep_apply_compress(int dtype, int n_sites, int64_t d,
                              double *log_norm, int *folded, double *profile,
                              void *stream);
 
+/* MatrixProductState.svd_compress (onedim_core.py:463-484) of the state itself, as
+ * the sweep above without its MPO and in the storage precision (workspace:
+ * tnc_sweep_workspace_size with MPO bonds of 1 and TNC_CORE_STORAGE; work 256-byte
+ * aligned).  Each bond's largest singular value is divided out of the returned
+ * sites; *log_norm: in, the log of the input's norm factor, out, that of the
+ * output.  out_discarded[i]: the discarded squared values over the squared largest
+ * one, bond between sites i and i+1. */
+int tnc_sweep_compress(int dtype, int n_sites, int64_t d,
+                       const void *const *sites, const int64_t *mps_bonds,
+                       int64_t chi, double threshold, void *work,
+                       size_t work_bytes, int64_t *out_bonds,
+                       int64_t *out_offsets, double *out_discarded,
+                       double *log_norm, void *stream);
+
+/* <bra|ket> of two states (ladder_contract, onedim_core.py:1587-1607): site i
+ * (d[i], bonds[i], bonds[i+1]), bonds[0] = 1; conj_bra conjugates the bra.
+ * scaled: the norms of the sites and of the environment are taken out as powers
+ * of two.  out (HOST): the first element of the last environment (its real and
+ * imaginary part), and the natural log of what was taken out.  d, the bonds and
+ * the pointer lists are HOST arrays. */
+int tnc_mps_overlap_workspace_size(int dtype, int n_sites, const int64_t *d,
+                                   const int64_t *bra_bonds,
+                                   const int64_t *ket_bonds, size_t *bytes);
+int tnc_mps_overlap(int dtype, int n_sites, const int64_t *d,
+                    const void *const *bra, const int64_t *bra_bonds,
+                    const void *const *ket, const int64_t *ket_bonds,
+                    int conj_bra, int scaled, void *work, size_t work_bytes,
+                    double *out, void *stream);
+
 /* ------------------------------------------------------------ learned rank
  * Kernels of the rank predictor (a small MLP trained on singular spectra the
  * plain method produces) and of the randomized-SVD sketch it sizes.  No

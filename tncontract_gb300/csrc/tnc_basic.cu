@@ -395,13 +395,22 @@ __global__ void cast_kernel(int64_t n, const S* __restrict__ x, D* __restrict__ 
     y[i] = cvt<S, D>(x[i]);
 }
 
+// acc += |x|^2, squared in double: single-precision squares leave their range at
+// 1e19 and 1e-23
+__device__ __forceinline__ void add_sq(double& acc, float x) { acc = fma((double)x, (double)x, acc); }
+__device__ __forceinline__ void add_sq(double& acc, double x) { acc = fma(x, x, acc); }
+template <typename R> __device__ __forceinline__ void add_sq(double& acc, cplx<R> x) {
+  add_sq(acc, x.re);
+  add_sq(acc, x.im);
+}
+
 // sum |x|^2 in double, one atomic per block
 template <typename T>
 __global__ void sumsq_kernel(int64_t n, const T* __restrict__ x, double* out) {
   __shared__ double red[32];
   double acc = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    acc += (double)abs2_(x[i]);
+    add_sq(acc, x[i]);
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) atomicAdd(out, acc);
 }

@@ -40,7 +40,9 @@
 // bond dimensions (tnc_sweep_workspace_size); nothing is allocated.
 #include "tnc_common.cuh"
 
+#include <algorithm>
 #include <cmath>
+#include <new>
 #include <vector>
 
 namespace tnc {
@@ -288,6 +290,11 @@ struct Prof {
   }
 };
 
+// The power of two at or below |x|: factors taken out of a state are powers of two,
+// so that scaling by them rounds nothing (a factor 1 / |R| rounded to FP32 is off
+// by up to 6e-8, and the state's norm by the product over its sites).
+double pow2_of(double x) { return x > 0 && std::isfinite(x) ? std::ldexp(1.0, std::ilogb(x)) : x; }
+
 double qr_flops(int64_t m, int64_t n, bool cplx) {
   const double mm = (double)(m > n ? m : n), nn = (double)(m < n ? m : n);
   return (2.0 * mm * nn * nn - 2.0 / 3.0 * nn * nn * nn) * (cplx ? 4.0 : 1.0);
@@ -318,8 +325,8 @@ int64_t rank_rule(const std::vector<R>& s, int64_t chi, double threshold, double
 }
 
 template <typename T>
-int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const int64_t* b, const void* const* mpo,
-               const int64_t* D, int64_t chi, double threshold, int block_rows, int core, double core_tol, void* work,
+int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const int64_t* b,
+               const void* const* mpo /* null: compress the state itself */, const int64_t* D, int64_t chi, double threshold, int block_rows, int core, double core_tol, void* work,
                size_t wb, int64_t* out_bonds, int64_t* out_offsets, double* out_discarded, double* log_norm,
                int* folded, double* profile, cudaStream_t st) {
   typedef typename traits<T>::real R;
@@ -336,8 +343,13 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
   std::vector<int64_t> sl(n_sites), sr(n_sites);  // current bonds of every site
   // 1. apply: site i -> (d, b_i D_i, b_{i+1} D_{i+1}), fused bond a * D + w
   for (int i = 0; i < n_sites; ++i) {
-    if (int rc = tnc_mps_mpo_site(dt, d, d, b[i], b[i + 1], D[i], D[i + 1], sites[i], mpo[i], B.slot[i], 1, st))
+    if (!mpo) {
+      if (cudaMemcpyAsync(B.slot[i], sites[i], (size_t)d * b[i] * b[i + 1] * sizeof(T), cudaMemcpyDeviceToDevice, st) !=
+          cudaSuccess)
+        return TNC_ERR_CUDA;
+    } else if (int rc = tnc_mps_mpo_site(dt, d, d, b[i], b[i + 1], D[i], D[i + 1], sites[i], mpo[i], B.slot[i], 1, st)) {
       return rc;
+    }
     sl[i] = P.bp[i];
     sr[i] = P.bp[i + 1];
   }
@@ -355,6 +367,7 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     if (int rc = host_norm(dt, k * r, B.rbuf, B.dnorm, &rn, st)) return rc;
     if (int stq = device_status(B.info, st)) return stq;
     prof.add(0, qr_flops(rows, r, cplx));
+    rn = pow2_of(rn);
     if (rn > 0) lnorm += std::log(rn);
     const int64_t r2 = sr[i + 1];  // sl[i + 1] == r
     if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_N, k, r2, r, rn > 0 ? 1.0 / rn : 1.0, B.rbuf, r, 0, B.slot[i + 1], r2,
@@ -375,7 +388,10 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     lnorm += std::log(last);
   }
   // 3. truncating SVD right sweep
-  double norm_acc = 1.0;
+  // the powers of two taken out of the sites, and what the largest value of the
+  // last bond has beside its own: the product of all bonds' largest values, each
+  // in units of the one before, is norm_acc rest
+  double norm_acc = 1.0, rest = 1.0;
   std::vector<R> s_host((size_t)P.max_kmin);
   std::vector<double> sd;  // the spectrum the truncation decision reads
   std::vector<int64_t> ord;  // the FP64 stage's row order
@@ -500,7 +516,7 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
         tot += sd[j] * sd[j];
         if (j >= k) dis += sd[j] * sd[j];
       }
-      out_discarded[i - 1] = tot > 0 ? dis / tot : 0.0;
+      out_discarded[i - 1] = !(tot > 0) ? 0.0 : mpo ? dis / tot : dis / (smax * smax);
     }
     // U (m x k)
     if (core_path) {
@@ -535,30 +551,144 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     sl[i] = k;
     // P_{i-1} <- P_{i-1} (S V^H)^T / s_max  ((d lp) x k)
     const int64_t lp = sl[i - 1], rp = sr[i - 1];  // rp == l
-    if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_T, d * lp, k, rp, 1.0 / smax, B.slot[i - 1], rp, 0, B.svbuf, n, 0,
+    if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_T, d * lp, k, rp, 1.0 / pow2_of(smax), B.slot[i - 1], rp, 0, B.svbuf, n, 0,
                           B.scratch, k, 0, 1, B.fact, factb, st))
       return rc;
     if (cudaMemcpyAsync(B.slot[i - 1], B.scratch, (size_t)d * lp * k * sizeof(T), cudaMemcpyDeviceToDevice, st) !=
         cudaSuccess)
       return TNC_ERR_CUDA;
     sr[i - 1] = k;
-    norm_acc *= smax;
+    norm_acc *= pow2_of(smax);
+    rest = smax / pow2_of(smax);
   }
-  // 4. the norm: s_max products into the first site; the QR sweep's factor too
-  //    when it is representable in the storage type
-  if (int rc = scale(dt, d * sl[0] * sr[0], norm_acc, B.slot[0], st)) return rc;
+  // 4. the norm: what the sweep took out back into the first site; the QR sweep's
+  //    factor too when it is representable in the storage type.  A compressed
+  //    state keeps its sites over their s_max, and the norm beside them.
+  if (int rc = scale(dt, d * sl[0] * sr[0], mpo ? norm_acc : 1.0 / rest, B.slot[0], st)) return rc;
   const double lim = fp32_class(dt) ? 60.0 : 600.0;
-  *folded = std::fabs(lnorm) <= lim ? 1 : 0;
+  *folded = mpo && std::fabs(lnorm) <= lim ? 1 : 0;
   if (*folded) {
     if (int rc = scale(dt, d * sl[0] * sr[0], std::exp(lnorm), B.slot[0], st)) return rc;
   }
-  *log_norm = lnorm + (norm_acc > 0 ? std::log(norm_acc) : 0.0);
+  *log_norm = lnorm + (norm_acc > 0 ? std::log(norm_acc) + std::log(rest) : 0.0);
   out_bonds[0] = sl[0];
   for (int i = 0; i < n_sites; ++i) {
     out_bonds[i + 1] = sr[i];
     out_offsets[i] = (int64_t)((char*)B.slot[i] - (char*)work);
   }
   return launch_status(0);
+}
+
+// ---------------------------------------------------------------- overlaps
+// <bra|ket> by the environment sweep from the left: X_p = a_p^H E (written with
+// rows (ra, p, lb), so that the next product contracts p and lb at once),
+// E' = X b.  With scaling, the sites' norms are read once at the start and the
+// environment's after every site, and powers of two are taken out in the
+// products' factors.
+struct OverlapPlan {
+  size_t norms, x, e[2], tc, total, tcb;
+};
+int overlap_plan(int dt, int n, const int64_t* d, const int64_t* ba, const int64_t* bb, OverlapPlan& P) {
+  const size_t es = (size_t)elem_size(dt);
+  size_t x = 0, e = 0, t = 0, w = 0;
+  if (ba[0] != 1 || bb[0] != 1) return TNC_ERR_ARG;
+  for (int i = 0; i < n; ++i) {
+    const int64_t la = ba[i], ra = ba[i + 1], lb = bb[i], rb = bb[i + 1];
+    if (d[i] <= 0 || ra <= 0 || rb <= 0) return TNC_ERR_ARG;
+    x = std::max(x, (size_t)d[i] * ra * lb * es);
+    e = std::max(e, (size_t)ra * rb * es);
+    w = tc_ws(dt, ra, lb, la, d[i]);
+    t = std::max(t, w);
+    w = tc_ws(dt, ra, rb, d[i] * lb, 1);
+    t = std::max(t, w);
+  }
+  Carve c{nullptr, 0};
+  auto take = [&](size_t bytes) {
+    c.take(bytes);
+    return c.off - bytes;
+  };
+  P.norms = take((size_t)(2 * n + 1) * sizeof(double));
+  P.x = take(x);
+  P.e[0] = take(e);
+  P.e[1] = take(e);
+  P.tc = take(t);
+  P.tcb = t;
+  P.total = c.off;
+  return TNC_OK;
+}
+
+template <typename T>
+int overlap_impl(int dt, int n, const int64_t* d, const void* const* bra, const int64_t* ba, const void* const* ket,
+                 const int64_t* bb, int conj_bra, int scaled, void* work, size_t wb, double* out, cudaStream_t st) {
+  OverlapPlan P;
+  if (int rc = overlap_plan(dt, n, d, ba, bb, P)) return rc;
+  if (wb < P.total) return TNC_ERR_WORKSPACE;
+  char* w = (char*)work;
+  double* norms = (double*)(w + P.norms);
+  const int lim = fp32_class(dt) ? 100 : 1000;  // exponents that a factor may have in the type
+  const double ln2 = 0.69314718055994530942;
+  double logs = 0.0;
+  std::vector<double> h((size_t)(2 * n));
+  if (scaled) {
+    for (int i = 0; i < n; ++i) {
+      if (int rc = tnc_nrm2(dt, d[i] * ba[i] * ba[i + 1], bra[i], norms + i, st)) return rc;
+      if (int rc = tnc_nrm2(dt, d[i] * bb[i] * bb[i + 1], ket[i], norms + n + i, st)) return rc;
+    }
+    if (cudaMemcpyAsync(h.data(), norms, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+      return TNC_ERR_CUDA;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return TNC_ERR_CUDA;
+  }
+  // the factor 2^-e for a norm, its logarithm kept
+  auto take_out = [&](double x, int extra) {
+    if (!scaled) return 1.0;
+    int e = extra + (x > 0 && std::isfinite(x) ? std::ilogb(x) : 0);
+    e = e > lim ? lim : e < -lim ? -lim : e;
+    logs += e * ln2;
+    return std::ldexp(1.0, -e);
+  };
+  const int opa = conj_bra ? TNC_OP_C : TNC_OP_T;
+  T* X = (T*)(w + P.x);
+  int cur = 0, left = 0;  // left: the environment's own exponent, taken out with the next site's
+  for (int i = 0; i < n; ++i) {
+    const int64_t la = ba[i], ra = ba[i + 1], lb = bb[i], rb = bb[i + 1];
+    T* E = (T*)(w + P.e[cur]);
+    T* E2 = (T*)(w + P.e[cur ^ 1]);
+    const double fa = take_out(h[(size_t)i], 0), fb = take_out(h[(size_t)(n + i)], left);
+    if (i == 0) {  // (d x ra)^H (d x rb); the bra's factor before the product, in which the two norms could leave the
+                   // type's range
+      const void* a = bra[i];
+      if (fa != 1.0) {
+        const double f[2] = {fa, 0.0};
+        if (int rc = tnc_scale(dt, d[i] * ra, f, bra[i], X, 0, st)) return rc;
+        a = X;
+      }
+      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, rb, d[i], fb, a, ra, 0, ket[i], rb, 0, E2, rb, 0, 1, w + P.tc, P.tcb,
+                            st))
+        return rc;
+    } else {
+      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, lb, la, fa, bra[i], ra, la * ra, E, lb, 0, X, d[i] * lb, lb, d[i],
+                            w + P.tc, P.tcb, st))
+        return rc;
+      if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_N, ra, rb, d[i] * lb, fb, X, d[i] * lb, 0, ket[i], rb, 0, E2, rb, 0, 1,
+                            w + P.tc, P.tcb, st))
+        return rc;
+    }
+    cur ^= 1;
+    left = 0;
+    if (scaled && i + 1 < n) {
+      double en = 0.0;
+      if (int rc = host_norm(dt, ra * rb, E2, norms + 2 * n, &en, st)) return rc;
+      if (en > 0 && std::isfinite(en)) left = std::ilogb(en);
+    }
+  }
+  T v;
+  if (cudaMemcpyAsync(&v, w + P.e[cur], sizeof(T), cudaMemcpyDeviceToHost, st) != cudaSuccess) return TNC_ERR_CUDA;
+  if (cudaStreamSynchronize(st) != cudaSuccess) return TNC_ERR_CUDA;
+  out[0] = (double)real_(v);
+  out[1] = 0.0;
+  if constexpr (traits<T>::is_complex) out[1] = (double)v.im;
+  out[2] = logs;
+  return TNC_OK;
 }
 
 }  // namespace
@@ -592,5 +722,46 @@ extern "C" int tnc_sweep_apply_compress(int dtype, int n_sites, int64_t d, const
                return sweep_impl<T>(dtype, n_sites, d, sites, mps_bonds, mpo, mpo_bonds, chi, threshold, block_rows,
                                     core, core_tol, work, work_bytes, out_bonds, out_offsets, out_discarded, log_norm,
                                     folded, profile, st));
+  return TNC_ERR_ARG;
+}
+
+extern "C" int tnc_sweep_compress(int dtype, int n_sites, int64_t d, const void* const* sites, const int64_t* mps_bonds,
+                                  int64_t chi, double threshold, void* work, size_t work_bytes, int64_t* out_bonds,
+                                  int64_t* out_offsets, double* out_discarded, double* log_norm, void* stream) {
+  if (n_sites < 2 || d <= 0 || !sites || !mps_bonds || !work || !out_bonds || !out_offsets || !log_norm || chi < 0)
+    return TNC_ERR_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  try {
+    const std::vector<int64_t> ones((size_t)n_sites + 1, 1);
+    int folded = 0;
+    TNC_DISPATCH(dtype, T,
+                 return sweep_impl<T>(dtype, n_sites, d, sites, mps_bonds, nullptr, ones.data(), chi, threshold, 0, 0, 0.0,
+                                      work, work_bytes, out_bonds, out_offsets, out_discarded, log_norm, &folded,
+                                      nullptr, st));
+  } catch (const std::bad_alloc&) {  // host memory: nothing may unwind into a C caller
+  }
+  return TNC_ERR_ARG;
+}
+
+extern "C" int tnc_mps_overlap_workspace_size(int dtype, int n_sites, const int64_t* d, const int64_t* bra_bonds,
+                                              const int64_t* ket_bonds, size_t* bytes) {
+  if (!elem_size(dtype) || n_sites < 1 || !d || !bra_bonds || !ket_bonds || !bytes) return TNC_ERR_ARG;
+  OverlapPlan P;
+  if (int rc = overlap_plan(dtype, n_sites, d, bra_bonds, ket_bonds, P)) return rc;
+  *bytes = P.total;
+  return TNC_OK;
+}
+
+extern "C" int tnc_mps_overlap(int dtype, int n_sites, const int64_t* d, const void* const* bra,
+                               const int64_t* bra_bonds, const void* const* ket, const int64_t* ket_bonds, int conj_bra,
+                               int scaled, void* work, size_t work_bytes, double* out, void* stream) {
+  if (n_sites < 1 || !d || !bra || !bra_bonds || !ket || !ket_bonds || !work || !out) return TNC_ERR_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  try {
+    TNC_DISPATCH(dtype, T,
+                 return overlap_impl<T>(dtype, n_sites, d, bra, bra_bonds, ket, ket_bonds, conj_bra, scaled, work,
+                                        work_bytes, out, st));
+  } catch (const std::bad_alloc&) {
+  }
   return TNC_ERR_ARG;
 }

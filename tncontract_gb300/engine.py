@@ -516,17 +516,66 @@ def _log_norm_of(sites):
     return 0.5 * float(np.log(v)) if v > 0 else 0.0
 
 
+def _native_chain(P):
+    """Sites that the native sweep takes: a chain of two or more device sites
+    of one dtype and physical dimension, its ends closed."""
+    d, dt = P[0].shape[0], P[0].dtype
+    return (len(P) > 1 and _ops.PROFILE is None and all(s.is_cuda and s.dtype == dt and s.dim() == 3 and s.shape[0] == d
+                                                        and min(s.shape) > 0 for s in P)
+            and P[0].shape[1] == 1 and P[-1].shape[2] == 1
+            and all(a.shape[2] == b.shape[1] for a, b in zip(P, P[1:])))
+
+
+def _compress_native(P, chi, threshold, stats, log_norm_in):
+    import ctypes as C
+    N, dt, d = len(P), P[0].dtype, int(P[0].shape[0])
+    P = [s.contiguous() for s in P]
+    bonds = (C.c_int64 * (N + 1))(1, *[int(s.shape[2]) for s in P])
+    ones = (C.c_int64 * (N + 1))(*[1] * (N + 1))
+    code = _ops.code(dt)
+    sz = C.c_size_t()
+    _ops._call("tnc_sweep_workspace_size", code, N, d, bonds, ones, L.CORE_STORAGE, C.byref(sz))
+    ws = torch.empty(int(sz.value), dtype=torch.uint8, device=P[0].device)
+    ptrs = (C.c_void_p * N)(*[s.data_ptr() for s in P])
+    out_b, out_o, out_d = (C.c_int64 * (N + 1))(), (C.c_int64 * N)(), (C.c_double * (N - 1))()
+    log_norm = C.c_double(float(log_norm_in))
+    st = L.lib().tnc_sweep_compress(code, N, d, ptrs, bonds, int(chi or 0), float(threshold), _ops._p(ws), sz.value, out_b,
+                                    out_o, out_d, C.byref(log_norm), _ops._stream())
+    if st == L.ERR_ARG:
+        raise ValueError("zero state in the sweep")
+    if st == L.ERR_NONFINITE:
+        raise ValueError("array must not contain infs or NaNs")
+    if st == L.ERR_NOT_CONVERGED:
+        raise _ops.LinAlgError("SVD did not converge")
+    L.check("tnc_sweep_compress", st)
+    es = P[0].element_size()
+    out = []
+    for i in range(N):
+        n = d * out_b[i] * out_b[i + 1]
+        out.append(ws[out_o[i]: out_o[i] + n * es].view(dt).view(d, out_b[i], out_b[i + 1]).clone())
+    if stats is not None:
+        stats.bonds.extend(list(out_b)[N - 1:0:-1])     # as the sweep meets them, from the right
+        stats.discarded.extend(list(out_d)[::-1])
+    return out, log_norm.value
+
+
 def compress(sites, chi, threshold=1e-15, stats=None, log_norm_in=0.0, fold_norm=True):
     """``MatrixProductState.svd_compress(chi, threshold)`` on (phys, left,
     right) device sites (no MPO).  Returns (sites, log_norm): the state is
     exp(log_norm) times the returned sites; with ``fold_norm`` the factor is
-    folded into the first site when it is representable (log_norm is then 0)."""
+    folded into the first site when it is representable (log_norm is then 0).
+    Device sites of one dtype and physical dimension run as one native call
+    (``tnc_sweep_compress``), so that instances on concurrent threads do not
+    contend for the interpreter at every operation."""
     P = [s for s in sites]
-    log_norm = qr_left_sweep(P) + log_norm_in
-    norm_acc = svd_right_sweep(P, chi, threshold, stats)
-    if norm_acc > 0:
-        log_norm += float(np.log(norm_acc))
-        P[0] = _ops.scale(P[0], 1.0 / norm_acc)   # keep the returned sites normalised
+    if _native_chain(P):
+        P, log_norm = _compress_native(P, chi, threshold, stats, log_norm_in)
+    else:
+        log_norm = qr_left_sweep(P) + log_norm_in
+        norm_acc = svd_right_sweep(P, chi, threshold, stats)
+        if norm_acc > 0:
+            log_norm += float(np.log(norm_acc))
+            P[0] = _ops.scale(P[0], 1.0 / norm_acc)   # keep the returned sites normalised
     if fold_norm and abs(log_norm) <= _FOLD_LIMIT.get(P[0].dtype, 600.0):
         P[0] = _ops.scale(P[0], float(np.exp(log_norm)))
         log_norm = 0.0
@@ -735,6 +784,32 @@ def _unit_site(x):
     return _ops.scale(x, 1.0 / n), shift + math.log(n)
 
 
+def _native_overlap(bra, ket):
+    for P in (bra, ket):
+        if not all(s.is_cuda and s.dim() == 3 and min(s.shape) > 0 for s in P) or P[0].shape[1] != 1 or \
+                not all(a.shape[2] == b.shape[1] for a, b in zip(P, P[1:])):
+            return False
+    return _ops.PROFILE is None and all(a.shape[0] == b.shape[0] for a, b in zip(bra, ket))
+
+
+def _overlap_native(bra, ket, dt, conj_bra, log_scale):
+    """``inner_product`` as one native call (``tnc_mps_overlap``)."""
+    import ctypes as C
+    N, code = len(bra), _ops.code(dt)
+    sides = [[_ops.cast(s, dt).contiguous() for s in P] for P in (bra, ket)]
+    d = (C.c_int64 * N)(*[int(s.shape[0]) for s in bra])
+    ba, bb = ((C.c_int64 * (N + 1))(1, *[int(s.shape[2]) for s in P]) for P in sides)
+    pa, pb = ((C.c_void_p * N)(*[s.data_ptr() for s in P]) for P in sides)
+    sz = C.c_size_t()
+    _ops._call("tnc_mps_overlap_workspace_size", code, N, d, ba, bb, C.byref(sz))
+    ws = torch.empty(int(sz.value), dtype=torch.uint8, device=sides[0][0].device)
+    out = (C.c_double * 3)()
+    _ops._call("tnc_mps_overlap", code, N, d, pa, ba, pb, bb, int(bool(conj_bra)), int(bool(log_scale)), _ops._p(ws),
+               sz.value, out, _ops._stream())
+    v = complex(out[0], out[1])
+    return (v, out[2]) if log_scale else v
+
+
 def inner_product(bra, ket, conj_bra=True, log_scale=False):
     """<bra|ket> of two (phys, left, right) site lists on the device, by the
     left-to-right environment sweep of ladder_contract (onedim_core.py:1587-1607).
@@ -743,6 +818,9 @@ def inner_product(bra, ket, conj_bra=True, log_scale=False):
     natural log of the scale) is returned, for states whose overlaps leave
     the FP64 range."""
     dt = torch.promote_types(bra[0].dtype, ket[0].dtype)
+    n = min(len(bra), len(ket))
+    if _native_overlap(bra[:n], ket[:n]):
+        return _overlap_native(bra[:n], ket[:n], dt, conj_bra, log_scale)
     C = None
     logs = 0.0
     for a, b in zip(bra, ket):
