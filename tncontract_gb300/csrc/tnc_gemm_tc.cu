@@ -12,10 +12,10 @@
 // of op(B) is scaled by a power of two to |x| < 1 and cut into three signed
 // 8-bit digits, x = 2^e 2^-8 (d0 + d1 2^-8 + d2 2^-16) (d0 in [-256, 256],
 // d1, d2 in [-128, 128], the last rounded to nearest), each digit an exact
-// BF16 value.  Digit products are integers below 2^16, so a 64-deep K chunk of
-// the products of one level (i + j = 0, 1, 2) sums to an integer below 2^24:
-// the FP32 accumulation in tensor memory is exact and its truncation never
-// acts.  After each chunk the three level accumulators are read with
+// BF16 value.  The digit products of one k are at most 65536 at levels i + j = 0
+// and 1 and 81920 at level 2, so 192 of them sum to an integer below 2^24: over
+// three 64-deep K slices the FP32 accumulation in tensor memory is exact and its
+// truncation never acts.  After each such group the three level accumulators are read with
 // tcgen05.ld and added into registers as L0 + 2^-8 L1 + 2^-16 L2 with
 // round-to-nearest FP32 adds.  Levels 3 and 4 are dropped (relative weight
 // 2^-24), so the result is FP32-accurate normwise and unbiased.
@@ -32,8 +32,11 @@
 // the six planes into shared memory with TMA (cp.async.bulk.tensor, 128-byte
 // swizzle, completion on an mbarrier), two stages, and issue the six
 // tcgen05.mma (kind::f16, BF16 inputs, FP32 accumulators, M = 128, N = 128,
-// K = 16) of every K step into three TMEM accumulators; after each slice all
-// four warps read their lanes (warp w: tile rows 32w..32w+31) and accumulate.
+// K = 16) of every K step into three TMEM accumulators; a slice is loaded while
+// the one before it is multiplied, and after each group of three all four warps
+// read their lanes (warp w: tile rows 32w..32w+31) and accumulate, the next two
+// slices on their way.  (Reading after every slice, and loading only then, left
+// the tensor pipe 28 % active: 69 us for 1536 x 768 x 512 complex64.)
 //
 // Every mbarrier wait is bounded; a wait that gives up records an error
 // (tnc_gemm_tc_error), waits (bounded) for the copies and MMAs it issued and
@@ -53,6 +56,7 @@ constexpr int kTcBM = 128;  // tile rows of A' (UMMA M)
 constexpr int kTcBN = 128;  // tile rows of B' (UMMA N)
 constexpr int kTcBK = 64;   // K elements per stage = one 128-byte swizzle atom of BF16
 constexpr int kTcNP = 3;    // digit planes
+constexpr int kTcGroup = 3;  // slices summed exactly in tensor memory
 // mbarrier polls before giving up: twice the library's wait limit
 // (tnc_set_spin_limit), a try_wait poll being shorter than a sleeping one
 static __device__ long long g_tc_spin = 2 * kSpinLimitDefault;
@@ -169,89 +173,255 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint
 }
 
 // ------------------------------------------------------------------ split kernel
-// One warp per source row r of X (X = op(A), rows x K, or X = op(B)^T): the
-// row's largest component fixes the power-of-two scale (|x| 2^-e < 1, scale
-// 2^e stored), then its digits go to the three planes
-// dst[batch][plane][rowsOutPad][Kpad].  Real: output row r, K' = K.  Complex
-// A: output rows 2r = [Re, -Im], 2r + 1 = [Im, Re]; complex B: output row r =
-// [Re, Im] (K' = 2K).  Rows and columns beyond the data are written as zeros.
-template <bool CPLX>
-__global__ void tc_split_kernel(const float* __restrict__ src, int op, int isB, int64_t rows, int64_t K, int64_t ld,
-                                int64_t sbatch, int64_t batch, int64_t rowsSrcPad, int64_t rowsOutPad, int64_t Kpad,
-                                __nv_bfloat16* __restrict__ dst, float* __restrict__ scale) {
+// Row r of X (X = op(A), rows x K, or X = op(B)^T): its largest component fixes
+// the power-of-two scale (|x| 2^-e < 1, scale 2^e stored), then its digits go to
+// the three planes dst[batch][plane][rowsOutPad][Kpad].  Real: output row r,
+// K' = K.  Complex A: output rows 2r = [Re, -Im], 2r + 1 = [Im, Re]; complex B:
+// output row r = [Re, Im] (K' = 2K).  Rows and columns beyond the data are
+// written as zeros.  One launch splits both operands.
+//
+// Bound by memory: the planes are three (B) or six (complex A) times the
+// operand's elements in BF16.  Rows that are contiguous in k take a warp each,
+// two elements a lane (one when an odd K or stride breaks the alignment); rows
+// that are strided (the operand is stored along them) take a CTA for 16, read
+// along the rows and turned in shared memory.  One warp a row for both layouts,
+// element by element, took 44 us for the operands of a 1536 x 768 x 512 complex64
+// product, these 12.
+struct SplitOperand {
+  const float* src;
+  int op, isB;
+  int64_t rows, ld, sbatch, rowsSrcPad, rowsOutPad, blocks;
+  __nv_bfloat16* dst;
+  float* scale;
+};
+constexpr int kSplitRows = 8;    // rows of a CTA, contiguous in k: a warp each
+constexpr int kSplitCols = 16;   // ... strided
+constexpr int kSplitK = 32;      // k of a turned tile
+
+// x 2^(8 - e) as two exact factors (one could leave FP32's range)
+struct SplitScale {
+  float a, b;
+};
+__device__ __forceinline__ int split_exp(float mx) {
+  int e = 0;
+  if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);  // mx = f 2^e, f in [0.5, 1)
+  return e > 127 ? 127 : e;
+}
+__device__ __forceinline__ SplitScale split_scale(int e) {
+  const int t = 8 - e, h = t / 2;
+  return {ldexpf(1.f, h), ldexpf(1.f, t - h)};
+}
+// x 2^-e in (-1, 1): three digits, the last rounded to nearest
+__device__ __forceinline__ void split_digits(float x, SplitScale sc, float (&d)[kTcNP]) {
+  const float y = x * sc.a * sc.b;
+  d[0] = rintf(y);
+  const float r1 = (y - d[0]) * 256.f;
+  d[1] = rintf(r1);
+  d[2] = rintf((r1 - d[1]) * 256.f);
+}
+
+template <bool CPLX, int V>
+__device__ __forceinline__ void split_row(const SplitOperand& o, int64_t b, int64_t r, int64_t K, int64_t Kpad) {
   const int lane = threadIdx.x & 31;
-  const bool trans = (op == TNC_OP_T || op == TNC_OP_C);
-  const bool cj = (op == TNC_OP_C || op == TNC_OP_R);
-  const bool rowmajor_rk = isB ? trans : !trans;
-  const bool pairA = CPLX && !isB;  // two output rows per source row
-  const int64_t plane = rowsOutPad * Kpad;
-  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < batch * rowsSrcPad; w += nw) {
-    const int64_t b = w / rowsSrcPad, r = w - b * rowsSrcPad;
-    const bool real_row = r < rows;
-    const float* sb = src + b * sbatch * (CPLX ? 2 : 1);
-    auto load = [&](int64_t k, float& re, float& im) {
-      const int64_t off = rowmajor_rk ? (r * ld + k) : (k * ld + r);
-      if (CPLX) {
-        const float2 v = reinterpret_cast<const float2*>(sb)[off];
-        re = v.x;
-        im = cj ? -v.y : v.y;
-      } else {
-        re = sb[off];
-        im = 0.f;
-      }
-    };
-    float mx = 0.f;
-    if (real_row)
-      for (int64_t k = lane; k < K; k += 32) {
-        float re, im;
-        load(k, re, im);
-        mx = fmaxf(mx, fmaxf(fabsf(re), fabsf(im)));
-      }
+  const bool cj = (o.op == TNC_OP_C || o.op == TNC_OP_R), pairA = CPLX && !o.isB;
+  const bool real_row = r < o.rows;
+  constexpr int W = CPLX ? 2 : 1;
+  const float* src = o.src + (b * o.sbatch + r * o.ld) * W;
+  auto load = [&](int64_t k, float (&v)[V * W]) {  // V elements from k
+    if constexpr (V * W == 4) {
+      const float4 q = *reinterpret_cast<const float4*>(src + k * W);
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else if constexpr (V * W == 2) {
+      const float2 q = *reinterpret_cast<const float2*>(src + k * W);
+      v[0] = q.x; v[1] = q.y;
+    } else {
+      v[0] = src[k];
+    }
+  };
+  float mx = 0.f;
+  if (real_row) {
+#pragma unroll 4
+    for (int64_t k = lane * V; k < K; k += 32 * V) {
+      float v[V * W];
+      load(k, v);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int e = 0;
-    if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);  // mx = f 2^e, f in [0.5, 1)
-    if (e > 127) e = 127;
-    const int64_t outRows = pairA ? 2 : 1;
-    const int64_t o0 = pairA ? 2 * r : r;
-    if (lane == 0) {
-      scale[b * rowsOutPad + o0] = ldexpf(1.f, e);
-      if (pairA) scale[b * rowsOutPad + o0 + 1] = ldexpf(1.f, e);
+      for (int i = 0; i < V * W; ++i) mx = fmaxf(mx, fabsf(v[i]));
     }
-    __nv_bfloat16* base = dst + b * kTcNP * plane;
-    auto put = [&](int64_t orow, int64_t kk, float x) {
-      // x 2^-e in (-1, 1): three digits, the last rounded to nearest
-      const float y = ldexpf(x, 8 - e);
-      const float d0 = rintf(y);
-      const float r1 = (y - d0) * 256.f;
-      const float d1 = rintf(r1);
-      const float d2 = rintf((r1 - d1) * 256.f);
-      __nv_bfloat16* q = base + orow * Kpad + kk;
-      q[0] = __float2bfloat16_rn(d0);
-      q[plane] = __float2bfloat16_rn(d1);
-      q[2 * plane] = __float2bfloat16_rn(d2);
-    };
-    const int64_t Kp = CPLX ? 2 * K : K;
-    for (int64_t k = lane; k < Kpad; k += 32) {
-      if (CPLX) {
-        // k indexes the K' axis: [0, K) real parts, [K, 2K) imaginary parts
-        float re = 0.f, im = 0.f;
-        const int64_t ks = k < K ? k : k - K;
-        if (real_row && k < Kp) load(ks, re, im);
-        if (pairA) {
-          put(o0, k, k < K ? re : -im);      // row 2r:   [Re, -Im] . [Re', Im']
-          put(o0 + 1, k, k < K ? im : re);   // row 2r+1: [Im,  Re]
-        } else {
-          put(o0, k, k < K ? re : im);       // B: [Re, Im]
-        }
-      } else {
-        float re = 0.f, im;
-        if (real_row && k < K) load(k, re, im);
-        put(o0, k, re);
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+  const int e = split_exp(mx);
+  const SplitScale sc = split_scale(e);
+  const int64_t o0 = pairA ? 2 * r : r;
+  if (lane == 0) {
+    o.scale[b * o.rowsOutPad + o0] = ldexpf(1.f, e);
+    if (pairA) o.scale[b * o.rowsOutPad + o0 + 1] = ldexpf(1.f, e);
+  }
+  const int64_t plane = o.rowsOutPad * Kpad, Kp = W * K;
+  __nv_bfloat16* base = o.dst + b * kTcNP * plane + o0 * Kpad;
+  auto put = [&](__nv_bfloat16* q, const float (&d)[V]) {
+    if constexpr (V == 2) *reinterpret_cast<__nv_bfloat162*>(q) = __floats2bfloat162_rn(d[0], d[1]);
+    else q[0] = __float2bfloat16_rn(d[0]);
+  };
+#pragma unroll 2
+  for (int64_t k = lane * V; k < K; k += 32 * V) {
+    float v[V * W];
+#pragma unroll
+    for (int i = 0; i < V * W; ++i) v[i] = 0.f;
+    if (real_row) load(k, v);
+    float re[kTcNP][V], im[kTcNP][V], ni[kTcNP][V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      float d[kTcNP];
+      split_digits(v[i * W], sc, d);
+#pragma unroll
+      for (int p = 0; p < kTcNP; ++p) re[p][i] = d[p];
+      if constexpr (CPLX) {
+        split_digits(cj ? -v[i * W + 1] : v[i * W + 1], sc, d);
+#pragma unroll
+        for (int p = 0; p < kTcNP; ++p) { im[p][i] = d[p]; ni[p][i] = -d[p]; }
       }
     }
-    (void)outRows;
+#pragma unroll
+    for (int p = 0; p < kTcNP; ++p) {
+      __nv_bfloat16* q = base + p * plane + k;
+      put(q, re[p]);
+      if constexpr (CPLX) {
+        if (pairA) {
+          put(q + K, ni[p]);
+          put(q + Kpad, im[p]);
+          put(q + Kpad + K, re[p]);
+        } else {
+          put(q + K, im[p]);
+        }
+      }
+    }
+  }
+  for (int64_t k = Kp + lane; k < Kpad; k += 32)
+#pragma unroll
+    for (int p = 0; p < kTcNP; ++p) {
+      base[p * plane + k] = __float2bfloat16_rn(0.f);
+      if (pairA) base[p * plane + Kpad + k] = __float2bfloat16_rn(0.f);
+    }
+}
+
+// 16 rows stored along the operand's other axis: element (r, k) at k ld + r.
+template <bool CPLX>
+__device__ __forceinline__ void split_cols(const SplitOperand& o, int64_t b, int64_t r0, int64_t K, int64_t Kpad) {
+  constexpr int W = CPLX ? 2 : 1, R = kSplitCols;
+  __shared__ float tile[W][R][kSplitK + 1];
+  __shared__ float red[R][16 + 1];
+  __shared__ int es[R];
+  const bool cj = (o.op == TNC_OP_C || o.op == TNC_OP_R), pairA = CPLX && !o.isB;
+  const float* src = o.src + b * o.sbatch * W;
+  const int tr = threadIdx.x % R, tk = threadIdx.x / R;  // 16 rows x 16 k
+  const int64_t r = r0 + tr;
+  const bool real_row = r < o.rows;
+  auto load = [&](int64_t k, float (&v)[W]) {
+    const int64_t at = k * o.ld + r;
+    if constexpr (CPLX) {
+      const float2 q = reinterpret_cast<const float2*>(src)[at];
+      v[0] = q.x;
+      v[1] = cj ? -q.y : q.y;
+    } else {
+      v[0] = src[at];
+    }
+  };
+  float mx = 0.f;
+  if (real_row) {
+#pragma unroll 8
+    for (int64_t k = tk; k < K; k += 16) {
+      float v[W];
+      load(k, v);
+#pragma unroll
+      for (int i = 0; i < W; ++i) mx = fmaxf(mx, fabsf(v[i]));
+    }
+  }
+  red[tr][tk] = mx;
+  __syncthreads();
+  if (threadIdx.x < R) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, red[threadIdx.x][i]);
+    const int e = split_exp(m);
+    es[threadIdx.x] = e;
+    const int64_t o0 = pairA ? 2 * (r0 + threadIdx.x) : r0 + threadIdx.x;
+    o.scale[b * o.rowsOutPad + o0] = ldexpf(1.f, e);
+    if (pairA) o.scale[b * o.rowsOutPad + o0 + 1] = ldexpf(1.f, e);
+  }
+  __syncthreads();
+  const int64_t plane = o.rowsOutPad * Kpad, Kp = W * K;
+  __nv_bfloat16* base = o.dst + b * kTcNP * plane;
+  // tiles of 32 k: read along the rows, written along k (lane = k, a warp 2 rows)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const SplitScale s0 = split_scale(es[2 * warp]), s1 = split_scale(es[2 * warp + 1]);
+  for (int64_t k0 = 0; k0 < K; k0 += kSplitK) {
+#pragma unroll
+    for (int h = 0; h < kSplitK / 16; ++h) {
+      const int64_t k = k0 + tk + 16 * h;
+      float v[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) v[i] = 0.f;
+      if (real_row && k < K) load(k, v);
+#pragma unroll
+      for (int i = 0; i < W; ++i) tile[i][tr][tk + 16 * h] = v[i];
+    }
+    __syncthreads();
+    const int64_t k = k0 + lane;
+    if (k < K) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int rr = 2 * warp + h;
+        const int64_t o0 = pairA ? 2 * (r0 + rr) : r0 + rr;
+        float d[kTcNP], di[kTcNP];
+        split_digits(tile[0][rr][lane], h ? s1 : s0, d);
+        if constexpr (CPLX) split_digits(tile[W - 1][rr][lane], h ? s1 : s0, di);
+#pragma unroll
+        for (int p = 0; p < kTcNP; ++p) {
+          __nv_bfloat16* q = base + p * plane + o0 * Kpad + k;
+          q[0] = __float2bfloat16_rn(d[p]);
+          if constexpr (CPLX) {
+            if (pairA) {
+              q[K] = __float2bfloat16_rn(-di[p]);
+              q[Kpad] = __float2bfloat16_rn(di[p]);
+              q[Kpad + K] = __float2bfloat16_rn(d[p]);
+            } else {
+              q[K] = __float2bfloat16_rn(di[p]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int64_t k = Kp + lane; k < Kpad; k += 32)
+    for (int h = 0; h < 2; ++h) {
+      const int64_t o0 = pairA ? 2 * (r0 + 2 * warp + h) : r0 + 2 * warp + h;
+      for (int p = 0; p < kTcNP; ++p) {
+        base[p * plane + o0 * Kpad + k] = __float2bfloat16_rn(0.f);
+        if (pairA) base[p * plane + (o0 + 1) * Kpad + k] = __float2bfloat16_rn(0.f);
+      }
+    }
+}
+
+__host__ __device__ inline bool split_contiguous(const SplitOperand& o) {
+  const bool trans = (o.op == TNC_OP_T || o.op == TNC_OP_C);
+  return o.isB ? trans : !trans;
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(256)
+tc_split_kernel(const SplitOperand oa, const SplitOperand ob, int64_t K, int64_t Kpad, int vecA, int vecB) {
+  const bool second = (int64_t)blockIdx.x >= oa.blocks;
+  const SplitOperand& o = second ? ob : oa;
+  const int64_t t = (int64_t)blockIdx.x - (second ? oa.blocks : 0);
+  if (split_contiguous(o)) {
+    const int64_t per = o.rowsSrcPad / kSplitRows, b = t / per, r = (t - b * per) * kSplitRows + (threadIdx.x >> 5);
+    if (second ? vecB : vecA) split_row<CPLX, 2>(o, b, r, K, Kpad);
+    else split_row<CPLX, 1>(o, b, r, K, Kpad);
+  } else {
+    const int64_t per = o.rowsSrcPad / kSplitCols, b = t / per;
+    split_cols<CPLX>(o, b, (t - b * per) * kSplitCols, K, Kpad);
   }
 }
 
@@ -275,7 +445,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   constexpr int STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full_bar[STAGES];
-  __shared__ uint64_t done_bar;
+  __shared__ uint64_t free_bar[STAGES];  // a stage's MMAs are complete (thread 0 alone waits, never two phases behind)
+  __shared__ uint64_t group_bar;         // a group's are (every thread waits once a group)
   __shared__ uint32_t tmem_base;
   __shared__ float sbc[kTcBN];
   __shared__ int ok_s;
@@ -286,8 +457,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const int nk = (int)(Kpad / kTcBK);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) mbar_init(&full_bar[s], 1);
-    mbar_init(&done_bar, 1);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&free_bar[s], 1);
+    }
+    mbar_init(&group_bar, 1);
     mbar_fence_init();
     ok_s = 1;
   }
@@ -312,8 +486,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                   (int)((b * kTcNP + p) * rowsB + n0));
     issued[s]++;
   };
+  int next = 0;  // next slice to load (thread 0)
   if (threadIdx.x == 0)
-    for (int s = 0; s < STAGES && s < nk; ++s) load_stage(s, s);
+    for (; next < STAGES && next < nk; ++next) load_stage(next, next);
 
   float acc[kTcBN];
 #pragma unroll
@@ -322,37 +497,53 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
   const uint32_t L0 = tmem, L1 = tmem + kTcBN, L2 = tmem + 2 * kTcBN;
   const uint32_t lanes = (uint32_t)(warp * 32) << 16;
   bool ok = true;
-  for (int kt = 0; kt < nk; ++kt) {
-    const int s = kt % STAGES;
+  for (int g0 = 0; g0 < nk; g0 += kTcGroup) {
+    const int g1 = g0 + kTcGroup < nk ? g0 + kTcGroup : nk;
     if (threadIdx.x == 0) {
-      if (ok && mbar_wait(&full_bar[s], (uint32_t)((kt / STAGES) & 1))) {
-        consumed[s]++;
-        tc_fence_after();
-        const uint32_t st = smem_u32(smem + (size_t)s * Cfg::STAGE);
+      for (int kt = g0; kt < g1; ++kt) {
+        const int s = kt % STAGES;
+        if (ok && mbar_wait(&full_bar[s], (uint32_t)((kt / STAGES) & 1))) {
+          consumed[s]++;
+          tc_fence_after();
+          const uint32_t st = smem_u32(smem + (size_t)s * Cfg::STAGE);
 #pragma unroll
-        for (int kk = 0; kk < kTcBK / 16; ++kk) {
-          const uint32_t koff = (uint32_t)kk * 32u;  // 16 BF16 = 32 bytes along K
-          uint64_t ad[kTcNP], bd[kTcNP];
+          for (int kk = 0; kk < kTcBK / 16; ++kk) {
+            const uint32_t koff = (uint32_t)kk * 32u;  // 16 BF16 = 32 bytes along K
+            uint64_t ad[kTcNP], bd[kTcNP];
 #pragma unroll
-          for (int p = 0; p < kTcNP; ++p) {
-            ad[p] = sw128_kmajor_desc(st + p * Cfg::A_TILE + koff);
-            bd[p] = sw128_kmajor_desc(st + kTcNP * Cfg::A_TILE + p * Cfg::B_TILE + koff);
+            for (int p = 0; p < kTcNP; ++p) {
+              ad[p] = sw128_kmajor_desc(st + p * Cfg::A_TILE + koff);
+              bd[p] = sw128_kmajor_desc(st + kTcNP * Cfg::A_TILE + p * Cfg::B_TILE + koff);
+            }
+            const uint32_t more = (kt == g0 && kk == 0) ? 0u : 1u;  // a group starts the level sums afresh
+            umma_bf16(L0, ad[0], bd[0], ID, more);
+            umma_bf16(L1, ad[0], bd[1], ID, more);
+            umma_bf16(L1, ad[1], bd[0], ID, 1u);
+            umma_bf16(L2, ad[0], bd[2], ID, more);
+            umma_bf16(L2, ad[1], bd[1], ID, 1u);
+            umma_bf16(L2, ad[2], bd[0], ID, 1u);
           }
-          const uint32_t acc0 = kk == 0 ? 0u : 1u;  // every slice starts the level sums afresh
-          umma_bf16(L0, ad[0], bd[0], ID, acc0);
-          umma_bf16(L1, ad[0], bd[1], ID, acc0);
-          umma_bf16(L1, ad[1], bd[0], ID, 1u);
-          umma_bf16(L2, ad[0], bd[2], ID, acc0);
-          umma_bf16(L2, ad[1], bd[1], ID, 1u);
-          umma_bf16(L2, ad[2], bd[0], ID, 1u);
+        } else {
+          ok = false;
+          ok_s = 0;
         }
-      } else {
-        ok = false;
-        ok_s = 0;
+        umma_commit(&free_bar[s]);  // arrives when this slice's MMAs (if any) are complete
+        if (kt == g1 - 1) umma_commit(&group_bar);
+        // the stage of the slice before is free when its MMAs are: load the next slice into it
+        if (ok && kt > g0 && next < nk) {
+          if (mbar_wait(&free_bar[(kt - 1) % STAGES], (uint32_t)(((kt - 1) / STAGES) & 1))) {
+            load_stage(next, next % STAGES);
+            ++next;
+          } else {
+            ok = false;
+            ok_s = 0;
+          }
+        }
       }
-      umma_commit(&done_bar);  // arrives when this slice's MMAs (if any) are complete
     }
-    const bool done = mbar_wait(&done_bar, (uint32_t)(kt & 1));
+    const bool done = mbar_wait(&group_bar, (uint32_t)((g0 / kTcGroup) & 1));
+    if (threadIdx.x == 0 && ok && done)  // every slice up to g1 is multiplied: both stages are free
+      for (; next < nk && next < g1 + STAGES; ++next) load_stage(next, next % STAGES);
     tc_fence_after();
 #pragma unroll
     for (int c0 = 0; c0 < kTcBN; c0 += 32) {
@@ -368,7 +559,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     if (!done || !ok_s) { ok = false; break; }
-    if (threadIdx.x == 0 && kt + STAGES < nk) load_stage(kt + STAGES, s);
   }
   if (threadIdx.x == 0 && !ok) {
     // drain: copies issued but not consumed must land before the CTA exits
@@ -495,10 +685,16 @@ static int gemm_tc_impl(int opA, int opB, int64_t m, int64_t n, int64_t k, const
   __nv_bfloat16* wB = reinterpret_cast<__nv_bfloat16*>(w + L.b_off);
   float* sa = reinterpret_cast<float*>(w + L.sa_off);
   float* sbv = reinterpret_cast<float*>(w + L.sb_off);
-  tc_split_kernel<CPLX><<<grid1d(batch * L.MsPad * 32, 256), 256, 0, st>>>(A, opA, 0, m, k, lda, sA, batch, L.MsPad,
-                                                                         L.MoPad, L.Kpad, wA, sa);
-  tc_split_kernel<CPLX><<<grid1d(batch * L.NPad * 32, 256), 256, 0, st>>>(B, opB, 1, n, k, ldb, sB, batch, L.NPad,
-                                                                        L.NPad, L.Kpad, wB, sbv);
+  // padded row counts are multiples of 64 (of 128 for B and real A)
+  SplitOperand oa = {A, opA, 0, m, lda, sA, L.MsPad, L.MoPad, 0, wA, sa}, ob = {B, opB, 1, n, ldb, sB, L.NPad, L.NPad, 0, wB, sbv};
+  oa.blocks = batch * (oa.rowsSrcPad / (split_contiguous(oa) ? kSplitRows : kSplitCols));
+  ob.blocks = batch * (ob.rowsSrcPad / (split_contiguous(ob) ? kSplitRows : kSplitCols));
+  if (oa.blocks + ob.blocks > 0x7fffffff) return TNC_ERR_ARG;
+  constexpr size_t kPair = CPLX ? 16 : 8;  // bytes of two elements
+  auto vec = [&](const SplitOperand& o) {
+    return (int)(k % 2 == 0 && o.ld % 2 == 0 && (batch == 1 || o.sbatch % 2 == 0) && (uintptr_t)o.src % kPair == 0);
+  };
+  tc_split_kernel<CPLX><<<(unsigned)(oa.blocks + ob.blocks), 256, 0, st>>>(oa, ob, k, L.Kpad, vec(oa), vec(ob));
   CUtensorMap mapA, mapB;
   if (make_map(&mapA, wA, (uint64_t)L.Kpad, (uint64_t)(batch * kTcNP * L.MoPad), kTcBM)) return TNC_ERR_CUDA;
   if (make_map(&mapB, wB, (uint64_t)L.Kpad, (uint64_t)(batch * kTcNP * L.NPad), kTcBN)) return TNC_ERR_CUDA;
@@ -507,7 +703,7 @@ static int gemm_tc_impl(int opA, int opB, int64_t m, int64_t n, int64_t k, const
   gemm_tc_kernel<CPLX><<<grid, 128, TcCfg::SMEM, st>>>(mapA, mapB, m, n, L.Kpad, L.MoPad, L.NPad, sa, sbv,
                                                        (float)alpha[0], (float)alpha[1], (float)beta[0],
                                                        (float)beta[1], C, ldc, sC);
-  return launch_status(3);
+  return launch_status(2);
 }
 
 }  // namespace tnc
