@@ -1,5 +1,5 @@
 """The GEMM's tile shapes: sizes at the edges of the FP64 tiles (8 x 16, 16 x 16,
-32 x 32) and of the FP32 ones (64 x 64; 32 x 32 with K split over a cluster) and on
+32 x 32) and of the FP32 ones (64 x 64 and 32 x 32, with K split over a cluster) and on
 both sides of the lines between them, ragged K, every operand layout, batches, and
 groups.  Bound: (k + 2) roundings of |A| |B| per term of a real sum, twice that
 in complex."""

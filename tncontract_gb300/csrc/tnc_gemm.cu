@@ -34,14 +34,21 @@ gemm_simt_kernel(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, con
 }
 
 // FP32 tile with K split over the S CTAs of a cluster: every CTA multiplies its
-// run of K slices, leaves its 32 x 32 sums in shared memory, and adds up (in the
-// order of K) and writes 32 / S of the tile's rows from all of them.
-template <typename T, bool AK, bool BKM>
+// run of K slices, leaves its sums in shared memory (where its slices were), and
+// adds up (in the order of K) and writes 1 / S of the tile's rows from all of them.
+template <typename T, typename G>
+struct SplitSmem {
+  static constexpr int A = 2 * G::BK * G::LDA, B = 2 * G::BK * G::LDB;
+  static_assert(A + B >= G::BM * G::BN, "the sums lie over the slices");
+  T v[A + B];
+};
+template <typename T, typename G, bool AK, bool BKM>
 __device__ __forceinline__ void split_tile(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, const T* A,
                                            int64_t lda, const T* B, int64_t ldb, T beta, T* C, int64_t ldc, int64_t m0,
-                                           int64_t n0, int S, int rank, T (*As)[Tile32<T>::BK * Tile32<T>::LDA],
-                                           T (*Bs)[Tile32<T>::BK * Tile32<T>::LDB], T* part) {
-  typedef Tile32<T> G;
+                                           int64_t n0, int S, int rank, SplitSmem<T, G>& sm) {
+  T(*As)[G::BK * G::LDA] = reinterpret_cast<T(*)[G::BK * G::LDA]>(sm.v);
+  T(*Bs)[G::BK * G::LDB] = reinterpret_cast<T(*)[G::BK * G::LDB]>(sm.v + SplitSmem<T, G>::A);
+  T* part = sm.v;
   const int64_t slices = (K + G::BK - 1) / G::BK;
   const int64_t k0 = slices * rank / S * G::BK, k1 = slices * (rank + 1) / S * G::BK, kn = (k1 < K ? k1 : K) - k0;
   T acc[G::TM][G::TN];
@@ -89,34 +96,35 @@ __device__ __forceinline__ int split_rank() {
   return (int)r;
 }
 
-template <typename T, bool AK, bool BKM>
-__global__ void __launch_bounds__(Tile32<T>::THR)
+template <typename T, typename G, bool AK, bool BKM>
+__global__ void __launch_bounds__(G::THR)
 gemm_split_kernel(int64_t M, int64_t N, int64_t K, bool aC, bool bC, T alpha, const T* __restrict__ A, int64_t lda,
                   int64_t sA, const T* __restrict__ B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC,
                   int64_t batch, int S) {
-  typedef Tile32<T> G;
-  __shared__ __align__(16) T As[2][G::BK * G::LDA];
-  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
-  __shared__ T part[G::BM * G::BN];
+  __shared__ __align__(16) SplitSmem<T, G> sm;
   const int64_t n0 = (int64_t)(blockIdx.x / (unsigned)S) * G::BN;
   const int rank = split_rank();
   for (int64_t bz = blockIdx.z; bz < batch; bz += gridDim.z)
     for (int64_t m0 = (int64_t)blockIdx.y * G::BM; m0 < M; m0 += (int64_t)gridDim.y * G::BM)
-      split_tile<T, AK, BKM>(M, N, K, aC, bC, alpha, A + bz * sA, lda, B + bz * sB, ldb, beta, C + bz * sC, ldc, m0, n0, S,
-                             rank, As, Bs, part);
+      split_tile<T, G, AK, BKM>(M, N, K, aC, bC, alpha, A + bz * sA, lda, B + bz * sB, ldb, beta, C + bz * sC, ldc, m0, n0,
+                                S, rank, sm);
 }
 
 // CTAs of the cluster that splits K when the 64 x 64 tiles would not fill the chip
-// (0: they do): as many as keep two slices or more each and about four small CTAs
-// an SM.
+// (0: they do, or K is too short to split): two slices or more each, and two CTAs
+// of 64 x 64 an SM or four of 32 x 32 (the two larger products of a chi = 256,
+// D = 3 environment update: 128 us in 32 x 32 tiles, two warps each, 107 in parts of
+// 64 x 64 ones, from a cold cache).
 template <typename Count>
-static int split_of(Count tiles, int64_t k) {
+static int split_of(Count tiles, int64_t k, bool small) {
   if (tiles(64, 64) >= 152) return 0;
-  const int64_t t = tiles(32, 32);
+  const int64_t t = small ? tiles(32, 32) : tiles(64, 64), most = small ? 152 * 4 : 152 * 2;
   int s = 1;
-  while (s < 8 && t * s * 2 <= 152 * 4 && k >= 64 * s) s *= 2;
+  while (s < 8 && t * s * 2 <= most && k >= 64 * s) s *= 2;
   return s;
 }
+// Products with a side of at most 32 take the 32 x 32 tile.
+static bool split_small(int64_t m, int64_t n) { return m <= 32 || n <= 32; }
 
 static cudaLaunchConfig_t split_config(dim3 grid, int threads, int S, cudaStream_t st, cudaLaunchAttribute* attr) {
   attr->id = cudaLaunchAttributeClusterDimension;
@@ -185,12 +193,9 @@ __global__ void __launch_bounds__(G::THR) gemm_grouped_kernel(const __grid_const
   else gemm_tile<T, G, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, As, Bs);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(Tile32<T>::THR) gemm_grouped_split_kernel(const __grid_constant__ GemmGroup g, int S) {
-  typedef Tile32<T> G;
-  __shared__ __align__(16) T As[2][G::BK * G::LDA];
-  __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
-  __shared__ T part[G::BM * G::BN];
+template <typename T, typename G>
+__global__ void __launch_bounds__(G::THR) gemm_grouped_split_kernel(const __grid_constant__ GemmGroup g, int S) {
+  __shared__ __align__(16) SplitSmem<T, G> sm;
   const int64_t tile = blockIdx.x / (unsigned)S;
   int q = 0;
   while (q + 1 < g.count && tile >= g.p[q + 1].tile0) ++q;
@@ -204,10 +209,10 @@ __global__ void __launch_bounds__(Tile32<T>::THR) gemm_grouped_split_kernel(cons
   const T* B = (const T*)P.B;
   T* C = (T*)P.C;
   const int rank = split_rank();
-  if (aK && bK) split_tile<T, true, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
-  else if (aK) split_tile<T, true, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
-  else if (bK) split_tile<T, false, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
-  else split_tile<T, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, As, Bs, part);
+  if (aK && bK) split_tile<T, G, true, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, sm);
+  else if (aK) split_tile<T, G, true, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, sm);
+  else if (bK) split_tile<T, G, false, true>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, sm);
+  else split_tile<T, G, false, false>(P.m, P.n, P.k, aC, bC, alpha, A, P.lda, B, P.ldb, beta, C, P.ldc, m0, n0, S, rank, sm);
 }
 
 // Tiles of a shape over the problems of a group, laid out for the kernel.
@@ -261,13 +266,19 @@ int gemm_grouped_launch(int count, const tnc_gemm_problem* probs, cudaStream_t s
     }
   } else {
     int64_t k = 0;
-    for (int i = 0; i < g.count; ++i) k = g.p[i].k > k ? g.p[i].k : k;
-    const int S = split_of(count_tiles, k);
+    bool small = true;  // of all problems
+    for (int i = 0; i < g.count; ++i) {
+      k = g.p[i].k > k ? g.p[i].k : k;
+      small = small && split_small(g.p[i].m, g.p[i].n);
+    }
+    const int S = split_of(count_tiles, k, small);
     if (S == 0) return grouped_launch<T, Tile64<T>>(g, st);
     cudaLaunchAttribute attr;
-    const int64_t tiles = group_tiles<Tile32<T>>(g);  // at most 4 x 151 with S
-    const cudaLaunchConfig_t cfg = split_config(dim3((unsigned)(tiles * S)), Tile32<T>::THR, S, st, &attr);
-    if (cudaLaunchKernelEx(&cfg, gemm_grouped_split_kernel<T>, g, S) != cudaSuccess) return TNC_ERR_CUDA;
+    const int64_t tiles = small ? group_tiles<Tile32<T>>(g) : group_tiles<Tile64<T>>(g);  // a few hundred at most
+    const cudaLaunchConfig_t cfg =
+        split_config(dim3((unsigned)(tiles * S)), small ? Tile32<T>::THR : Tile64<T>::THR, S, st, &attr);
+    const auto fn = small ? gemm_grouped_split_kernel<T, Tile32<T>> : gemm_grouped_split_kernel<T, Tile64<T>>;
+    if (cudaLaunchKernelEx(&cfg, fn, g, S) != cudaSuccess) return TNC_ERR_CUDA;
     return launch_status();
   }
 }
@@ -306,6 +317,24 @@ static int simt_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alph
   return launch_status();
 }
 
+// Fewer than 152 tiles of 64 x 64: every count of the grid is small.
+template <typename T, typename G>
+static int split_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, const T* A, int64_t lda, int64_t sA,
+                        const T* B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC, int64_t batch, int S,
+                        cudaStream_t st) {
+  const dim3 grid((unsigned)((n + G::BN - 1) / G::BN * S), (unsigned)((m + G::BM - 1) / G::BM), (unsigned)batch);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = split_config(grid, G::THR, S, st, &attr);
+  const bool aK = (opA == TNC_OP_N || opA == TNC_OP_R), bK = (opB == TNC_OP_T || opB == TNC_OP_C);
+  const bool aC = (opA == TNC_OP_C || opA == TNC_OP_R), bC = (opB == TNC_OP_C || opB == TNC_OP_R);
+  const auto fn = aK ? (bK ? gemm_split_kernel<T, G, true, true> : gemm_split_kernel<T, G, true, false>)
+                     : (bK ? gemm_split_kernel<T, G, false, true> : gemm_split_kernel<T, G, false, false>);
+  if (cudaLaunchKernelEx(&cfg, fn, m, n, k, aC, bC, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, S) !=
+      cudaSuccess)
+    return TNC_ERR_CUDA;
+  return launch_status();
+}
+
 template <typename T>
 int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, const T* A, int64_t lda,
                 int64_t sA, const T* B, int64_t ldb, int64_t sB, T beta, T* C, int64_t ldc, int64_t sC,
@@ -326,20 +355,11 @@ int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha, cons
       default: return simt_launch<T, TileL<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
     }
   } else {
-    const int S = split_of(tiles, k);
+    const bool small = split_small(m, n);
+    const int S = split_of(tiles, k, small);
     if (S == 0) return simt_launch<T, Tile64<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, st);
-    typedef Tile32<T> G;  // fewer than 152 tiles of 64 x 64: every count is small
-    const dim3 grid((unsigned)((n + G::BN - 1) / G::BN * S), (unsigned)((m + G::BM - 1) / G::BM), (unsigned)batch);
-    cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = split_config(grid, G::THR, S, st, &attr);
-    const bool aK = (opA == TNC_OP_N || opA == TNC_OP_R), bK = (opB == TNC_OP_T || opB == TNC_OP_C);
-    const bool aC = (opA == TNC_OP_C || opA == TNC_OP_R), bC = (opB == TNC_OP_C || opB == TNC_OP_R);
-    const auto fn = aK ? (bK ? gemm_split_kernel<T, true, true> : gemm_split_kernel<T, true, false>)
-                       : (bK ? gemm_split_kernel<T, false, true> : gemm_split_kernel<T, false, false>);
-    if (cudaLaunchKernelEx(&cfg, fn, m, n, k, aC, bC, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, S) !=
-        cudaSuccess)
-      return TNC_ERR_CUDA;
-    return launch_status();
+    if (small) return split_launch<T, Tile32<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, S, st);
+    return split_launch<T, Tile64<T>>(opA, opB, m, n, k, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, S, st);
   }
 }
 

@@ -34,7 +34,7 @@ struct GemmTile {
   static constexpr int PA = BM * BK / THR, PB = BN * BK / THR;  // tile elements each thread moves
 };
 template <typename T> using Tile64 = GemmTile<T, 64, 64, 4, 4>;  // FP32
-template <typename T> using Tile32 = GemmTile<T, 32, 32, 4, 4>;  // FP32, K split over a cluster
+template <typename T> using Tile32 = GemmTile<T, 32, 32, 4, 4>;  // FP32, narrow products, K split over a cluster
 template <typename T> using TileL = GemmTile<T, 32, 32, 4, 2>;   // FP64, 128 threads each
 template <typename T> using TileM = GemmTile<T, 16, 16, 2, 1>;
 template <typename T> using TileS = GemmTile<T, 8, 16, 1, 1>;
