@@ -28,12 +28,26 @@ class LinAlgError(np.linalg.LinAlgError):
     pass
 
 
+# On the launch path of every call: torch.device objects are kept per index, and
+# the current stream's handle is read without building a Stream object (0.1 us
+# instead of 3).
+_DEVICES = {}
+
+
 def device():
-    return torch.device("cuda", torch.cuda.current_device())
+    i = torch.cuda.current_device()
+    d = _DEVICES.get(i)
+    if d is None:
+        d = _DEVICES[i] = torch.device("cuda", i)
+    return d
+
+
+def _raw_stream():
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_raw_stream())
 
 
 def _p(t):
@@ -97,7 +111,7 @@ def profile_summary(prof):
 
 
 def empty(shape, dtype):
-    return torch.empty(tuple(int(s) for s in shape), dtype=dtype, device=device())
+    return torch.empty(tuple(map(int, shape)), dtype=dtype, device=device())
 
 
 def zeros(shape, dtype):
@@ -110,7 +124,7 @@ _WS = {}
 
 def workspace(nbytes):
     """Per-stream reusable workspace (stream ordering makes reuse safe)."""
-    key = (torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream)
+    key = (torch.cuda.current_device(), _raw_stream())
     buf = _WS.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=device())
@@ -166,7 +180,7 @@ def fuse_permutation(shape, perm):
         else:
             groups.append([a])
     by_input = sorted(range(len(groups)), key=lambda g: groups[g][0])
-    fused_shape = [int(np.prod([dims[a] for a in groups[g]], dtype=np.int64)) for g in by_input]
+    fused_shape = [math.prod([dims[a] for a in groups[g]]) for g in by_input]
     position = {g: i for i, g in enumerate(by_input)}
     return fused_shape, [position[g] for g in range(len(groups))]
 
@@ -312,8 +326,8 @@ def slice_axis(data, axis, k):
     n = data.shape[axis]
     if k == n:
         return data
-    after = int(np.prod(data.shape[axis + 1:], dtype=np.int64))
-    rows = int(np.prod(data.shape[:axis], dtype=np.int64))
+    after = math.prod(data.shape[axis + 1:])
+    rows = math.prod(data.shape[:axis])
     out = empty(tuple(data.shape[:axis]) + (k,) + tuple(data.shape[axis + 1:]), data.dtype)
     if out.numel():
         copy2d(data, rows, k * after, n * after, out, k * after)
@@ -363,7 +377,7 @@ def fuse_trace(shape, a1, a2):
     """(shape, a1, a2) of the same trace on five axes: the axes before,
     between and after the traced pair fused."""
     lo, hi = min(a1, a2), max(a1, a2)
-    prod = lambda d: int(np.prod(d, dtype=np.int64))
+    prod = math.prod
     fused = [prod(shape[:lo]), int(shape[lo]), prod(shape[lo + 1:hi]), int(shape[hi]), prod(shape[hi + 1:])]
     return (fused, 1, 3) if a1 < a2 else (fused, 3, 1)
 
@@ -401,7 +415,7 @@ _TC_WS = {}
 
 
 def _tc_workspace(nbytes):
-    key = (torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream)
+    key = (torch.cuda.current_device(), _raw_stream())
     buf = _TC_WS.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=device())
@@ -450,9 +464,9 @@ def tensordot(a, b, axes_a, axes_b):
     b = cast(b.contiguous(), dt)
     free_a = [i for i in range(a.dim()) if i not in axes_a]
     free_b = [i for i in range(b.dim()) if i not in axes_b]
-    ma = int(np.prod([a.shape[i] for i in free_a], dtype=np.int64))
-    nb = int(np.prod([b.shape[i] for i in free_b], dtype=np.int64))
-    kk = int(np.prod([a.shape[i] for i in axes_a], dtype=np.int64))
+    ma = math.prod([a.shape[i] for i in free_a])
+    nb = math.prod([b.shape[i] for i in free_b])
+    kk = math.prod([a.shape[i] for i in axes_a])
     out = empty([a.shape[i] for i in free_a] + [b.shape[i] for i in free_b], dt)
     if ma == 0 or nb == 0:
         return out
@@ -482,9 +496,9 @@ def _tensordot_prepare(a, b, axes_a, axes_b):
     b = cast(b.contiguous(), dt)
     free_a = [i for i in range(a.dim()) if i not in axes_a]
     free_b = [i for i in range(b.dim()) if i not in axes_b]
-    ma = int(np.prod([a.shape[i] for i in free_a], dtype=np.int64))
-    nb = int(np.prod([b.shape[i] for i in free_b], dtype=np.int64))
-    kk = int(np.prod([a.shape[i] for i in axes_a], dtype=np.int64))
+    ma = math.prod([a.shape[i] for i in free_a])
+    nb = math.prod([b.shape[i] for i in free_b])
+    kk = math.prod([a.shape[i] for i in axes_a])
     out = empty([a.shape[i] for i in free_a] + [b.shape[i] for i in free_b], dt)
     if ma == 0 or nb == 0:
         return out, None

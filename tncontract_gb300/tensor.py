@@ -16,6 +16,7 @@ returns the discarded singular values as a device tensor.
 from __future__ import annotations
 
 import copy as _copy
+import math
 import warnings
 
 import numpy as np
@@ -270,7 +271,7 @@ class Tensor():
             fused = (label, [a for g in groups[p:p + n] for a in g[1]])
             groups[p:p + n] = [fused]
         perm = [a for g in groups for a in g[1]]
-        shape = [int(np.prod([self.data.shape[a] for a in g[1]], dtype=np.int64)) for g in groups]
+        shape = [math.prod([self.data.shape[a] for a in g[1]]) for g in groups]
         self.data = _ops.permute(self.data, perm).reshape(tuple(shape))
         self._labels = [g[0] for g in groups]
 
@@ -351,8 +352,8 @@ class Tensor():
         shp = list(old)
         shp[index] += inc
         out = _ops.zeros(shp, self.data.dtype)
-        outer = int(np.prod(old[:index], dtype=np.int64))
-        inner = int(np.prod(old[index + 1:], dtype=np.int64))
+        outer = math.prod(old[:index])
+        inner = math.prod(old[index + 1:])
         # rows = outer blocks; each block is (dim * inner) contiguous elements
         _ops.copy2d(self.data.contiguous(), outer, old[index] * inner, old[index] * inner,
                     out, shp[index] * inner, dst_off=(inc * inner if before else 0))
@@ -534,7 +535,7 @@ def tensor_to_matrix(tensor, row_labels):
     for i, label in enumerate(row_labels):
         ax.move_index(label, i)
     data = _ops.permute(tensor.data, ax.perm)
-    nrow = int(np.prod(data.shape[:len(row_labels)], dtype=np.int64))
+    nrow = math.prod(data.shape[:len(row_labels)])
     ncol = data.numel() // nrow if nrow else 0
     return data.reshape(nrow, ncol)
 
@@ -560,8 +561,8 @@ def _matricise(tensor, row_labels):
         ax.move_index(label, i)
     data = _ops.permute(tensor.data, ax.perm)
     shape = tuple(data.shape)
-    nrow = int(np.prod(shape[:len(row_labels)], dtype=np.int64))
-    ncol = int(np.prod(shape[len(row_labels):], dtype=np.int64))
+    nrow = math.prod(shape[:len(row_labels)])
+    ncol = math.prod(shape[len(row_labels):])
     return data.reshape(nrow, ncol), shape, ax.labels
 
 

@@ -23,6 +23,8 @@ returns what the reference returns.  Every step is a device ``contract`` /
 """
 from __future__ import annotations
 
+import math
+
 import numpy as np
 
 from . import _ops
@@ -187,9 +189,9 @@ def _greedy_plan(shapes, labels, partner):
                 if j <= i:
                     continue
                 la = [l for l in nodes[i] if l in partner and owner[partner[l]] == j]
-                shared = int(np.prod([dims[l] for l in la], dtype=np.float64))
-                size_i = int(np.prod([dims[l] for l in nodes[i]], dtype=np.float64))
-                size_j = int(np.prod([dims[l] for l in nodes[j]], dtype=np.float64))
+                shared = math.prod([dims[l] for l in la])
+                size_i = math.prod([dims[l] for l in nodes[i]])
+                size_j = math.prod([dims[l] for l in nodes[j]])
                 cost = size_i * size_j // max(shared, 1)
                 out = cost // max(shared, 1)
                 key = (cost, out, i, j)
@@ -241,8 +243,8 @@ def _argument_cost(shapes, labels, internal_contract, pairwise_contract, index_l
         @staticmethod
         def contract(t1, t2, l1, l2):
             l1 = l1 if isinstance(l1, list) else [l1]
-            total[0] += int(np.prod([dims[l] for l in t1 + t2], dtype=np.float64)) // max(
-                int(np.prod([dims[l] for l in l1], dtype=np.float64)), 1)
+            total[0] += math.prod([dims[l] for l in t1 + t2]) // max(
+                math.prod([dims[l] for l in l1]), 1)
             return _Labels.contract(t1, t2, l1, l2)
 
     _argument_order(_Count, labels, internal_contract, pairwise_contract, index_lookup)
@@ -291,7 +293,17 @@ def con(*args, order="cost"):
     if order not in ("cost", "argument"):
         raise ValueError("order must be 'cost' or 'argument'")
     tensor_list, contract_list = _split_args(args)
-    tensor_list = [t.copy() for t in tensor_list]
+    out = _contract_network(tensor_list, contract_list, order)
+    # nothing writes to a tensor's data, so the network is contracted from the
+    # arguments' own; a result that is still (a view of) one of them is copied
+    held = out.data.untyped_storage().data_ptr()
+    if any(t.data.untyped_storage().data_ptr() == held for t in tensor_list):
+        out = out.copy()
+    return out
+
+
+def _contract_network(tensor_list, contract_list, order):
+    tensor_list = [tn._new(t.data, list(t.labels)) for t in tensor_list]
     all_labels = [t.labels for t in tensor_list]
     index_lookup = _index_lookup(all_labels, contract_list)
     internal, pairwise = _group_pairs(contract_list, index_lookup)
