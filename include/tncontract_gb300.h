@@ -341,10 +341,13 @@ int tnc_permute_rows(int dtype, int64_t n, int64_t L, const void *src,
  * scaled by a power of two to unit Frobenius norm inside; W (m x n) receives
  * the orthogonalised rows as FP64 / complex128 elements, S (FP64) and order
  * as tnc_svd_rows for the FP64 type, and the rows are orthogonal to tol
- * relative (<= 0: 1e-7).  The finish ends without a checking sweep (info[3]
- * = 1) after a rotating sweep whose rotations were all small angles below
- * 1e-5 relative: their residual is second order (about 1e-8).  Rows beyond nkeep as in tnc_svd_rows_keep.  Rows
- * up to 800 complex / 1600 real elements.  Workspace:
+ * relative (<= 0: 1e-7).  24 rows or more first take a few steps that rotate
+ * every pair at once, as FP64 and compensated FP32 products of the whole matrix;
+ * what they leave (clusters of nearly equal values) the double-float Jacobi
+ * takes.  Either ends without a checking pass (info[3] = 1) after one whose
+ * rotations were all small angles below 1e-5: their residual is second order.
+ * info[1]: passes of the one that ended the work.  Rows beyond nkeep as in
+ * tnc_svd_rows_keep.  Rows up to 800 complex / 1600 real elements.  Workspace:
  * tnc_svd_rows_workspace_size of the FP64 type.  Replaces, in the sweep,
  * the FP64 finish (tnc_cast to the FP64 type + tnc_svd_rows_keep). */
 int tnc_svd_rows_df(int dtype, int64_t m, int64_t n, const void *A, void *W,

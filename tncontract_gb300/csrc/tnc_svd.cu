@@ -263,16 +263,20 @@ static int svd_refine(int64_t nr, const T* R, T* J, T* Wb, T* GF, char* scratch,
   refine_widen_kernel<T><<<g, 256, 0, st>>>(nr * nr, J32, J);
   typedef TileS<T> G;
   const int64_t rows = (nr + G::BM - 1) / G::BM, cols = (nr + G::BN - 1) / G::BN;
-  int64_t half = 0;
-  for (int64_t c = 0; c < cols; ++c) half += 2 * (c + 1) < rows ? 2 * (c + 1) : rows;
+  const unsigned half = refine_half_tiles(nr);
+  const double eps = traits<T>::eps;
   refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, 0);
   for (int s = 0; s <= kRefineSteps; ++s) {
-    refine_gram_kernel<T><<<dim3((unsigned)half, 2), G::THR, 0, st>>>(nr, Wb, J, GF, a, d, rs, s, js.rows_large);
-    refine_test_kernel<T><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, rs, s, js.rows_large);
+    refine_gram_kernel<T><<<dim3(half, 2), G::THR, 0, st>>>(nr, nr, Wb, J, GF, a, d, rs, s, -1.f, js.rows_large);
+    refine_test_kernel<T, true><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, eps, nr, rs, s, -1.f, js.rows_large,
+                                                     nullptr);
     if (s == kRefineSteps) break;
-    refine_f_kernel<T><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, GF, a, d, frob2, tol, rs, s, js.rows_large, Ft);
-    if (nr <= 128) refine_apply_kernel<T, 1><<<dim3((unsigned)nr, 2), 256, nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
-    else refine_apply_kernel<T, 4><<<dim3((unsigned)((nr + 3) / 4), 2), 256, 4 * nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
+    refine_f_kernel<T, true><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, GF, a, d, frob2, tol, eps, nr, rs, s, -1.f,
+                                                                 js.rows_large, Ft);
+    if (nr <= 128)
+      refine_apply_kernel<T, 1><<<dim3((unsigned)nr, 2), 256, nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
+    else
+      refine_apply_kernel<T, 4><<<dim3((unsigned)((nr + 3) / 4), 2), 256, 4 * nr * sizeof(S), st>>>(nr, Ft, J, Wb, frob2, rs, s);
     refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, s + 1);
   }
   *launched += 5 + 5 * kRefineSteps + 2;

@@ -39,8 +39,24 @@ struct RefineState {
   unsigned hard;       // pairs whose rotation this step could not take
   float fmax;          // largest |F|
 };
+// Whether a step before `upto` found nothing to do.  Without J (accept >= 0), also
+// whether one took an F below `accept`; a hard one is the last then, and the steps
+// after it have not run.
+__device__ __forceinline__ bool refine_done(const RefineState* st, int upto, float accept = -1.f) {
+  for (int s = 0; s < upto; ++s) {
+    if (st[s].rot == 0 && st[s].unit == 0) return true;
+    if (accept >= 0.f && st[s].hard) return false;
+    if (st[s].fmax < accept) return true;
+  }
+  return false;
+}
+// The same from inside step `step`, after its test.
+__device__ __forceinline__ bool refine_idle(const RefineState* st, int step, float accept = -1.f) {
+  return refine_done(st, step, accept) || (st[step].rot == 0 && st[step].unit == 0);
+}
 // A step with pairs that it cannot rotate leaves them to the FP64 Jacobi: the
-// steps after it make J unitary and rotate nothing.
+// steps after it make J unitary and rotate nothing; without J such a step does
+// nothing and is the last.
 __device__ __forceinline__ bool refine_hard(const RefineState* st, int upto) {
   for (int s = 0; s < upto; ++s)
     if (st[s].hard) return true;
@@ -50,11 +66,6 @@ __device__ __forceinline__ bool refine_hard(const RefineState* st, int upto) {
 template <typename T> struct narrow_of { typedef float type; };
 template <> struct narrow_of<c128> { typedef c64 type; };
 
-__device__ __forceinline__ bool refine_done(const RefineState* st, int upto) {
-  for (int s = 0; s < upto; ++s)
-    if (st[s].rot == 0 && st[s].unit == 0) return true;
-  return false;
-}
 
 // Exponent k with |R|_F about 2^k: the single-precision copy is R 2^-k.
 __device__ __forceinline__ int refine_exp(const double* f2) {
@@ -109,17 +120,18 @@ refine_product_kernel(int64_t n, const T* __restrict__ J, const T* __restrict__ 
   if (gm < n && gn < n) W[gm * n + gn] = acc[0][0];
 }
 
-// X = W (blockIdx.y = 0) or J (1): <x_i, x_k> for i < k, G's above the diagonal of
-// GF, delta's below it (at (k, i)); the diagonals to a and d.
+// X = W (blockIdx.y = 0; n rows of K elements) or J (1; n x n): <x_i, x_k> for
+// i < k, G's above the diagonal of GF, delta's below it (at (k, i)); the diagonals
+// to a and d.
 template <typename T>
 __global__ void __launch_bounds__(TileS<T>::THR)
-refine_gram_kernel(int64_t n, const T* __restrict__ W, const T* __restrict__ J, T* __restrict__ GF,
+refine_gram_kernel(int64_t n, int64_t K, const T* __restrict__ W, const T* __restrict__ J, T* __restrict__ GF,
                    typename traits<T>::real* __restrict__ a, typename traits<T>::real* __restrict__ d,
-                   const RefineState* st, int upto, unsigned* rows_large) {
+                   const RefineState* st, int upto, float accept, unsigned* rows_large) {
   typedef TileS<T> G;
   __shared__ __align__(16) T As[2][G::BK * G::LDA];
   __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
-  if (refine_done(st, upto)) return;
+  if (refine_done(st, upto, accept) || (J == nullptr && refine_hard(st, upto))) return;
   if (blockIdx.y == 0)
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
       rows_large[i] = 0;
@@ -135,8 +147,9 @@ refine_gram_kernel(int64_t n, const T* __restrict__ W, const T* __restrict__ J, 
   if (cb >= cols) return;
   const int64_t m0 = t * G::BM, n0 = cb * G::BN;
   const T* X = blockIdx.y ? J : W;
+  const int64_t kx = blockIdx.y ? n : K;
   T acc[G::TM][G::TN];
-  gemm_acc<T, G, true, true>(n, n, n, false, true, X, n, X, n, m0, n0, As, Bs, acc);
+  gemm_acc<T, G, true, true>(n, n, kx, false, true, X, kx, X, kx, m0, n0, As, Bs, acc);
   const int64_t i = m0 + tile_row<G>(0), k = n0 + tile_col<G>(0);
   if (i > k || k >= n) return;
   const T v = acc[0][0];
@@ -191,35 +204,46 @@ __device__ __forceinline__ RefinePair<typename narrow_of<T>::type> refine_pair(T
   r.large = r.t > 1e-3f;
   return r;
 }
-// Relative inner products that a step leaves alone: the second order of the
-// Jacobi's 1e-6 at first, then half the tolerance.
-__device__ __forceinline__ float refine_skip(int step, double tol) { return step == 0 ? 1e-9f : 0.5f * (float)tol; }
+// Relative inner products that a step leaves alone: half the tolerance, and with J
+// the second order of the Jacobi's 1e-6 at first.
+template <bool HASJ>
+__device__ __forceinline__ float refine_skip(int step, double tol) {
+  return HASJ && step == 0 ? 1e-9f : 0.5f * (float)tol;
+}
 
 // Counts of the pairs above the tolerances, and for every row its pairs with a
-// large angle.  A thread takes a pair i < k.
-template <typename T>
+// large angle (and its partner in the last).  A thread takes a pair i < k.  Without J, delta is nothing and d is
+// not read.  Pairs of two rows from nkeep on are left alone.
+template <typename T, bool HASJ>
 __global__ void refine_test_kernel(int64_t n, const T* __restrict__ GF, const typename traits<T>::real* __restrict__ a,
                                    const typename traits<T>::real* __restrict__ d, const double* frob2, double tol,
-                                   RefineState* st, int step, unsigned* rows_large) {
-  if (refine_done(st, step)) return;
-  const double sc = refine_scale2(frob2), noise2 = noise_floor2<T>(frob2) * sc, tol2 = tol * tol, utol2 = 16.0 * tol2;
-  const float skip = refine_skip(step, tol);
+                                   double eps, int64_t nkeep, RefineState* st, int step, float accept,
+                                   unsigned* rows_large, unsigned* partner) {
+  if (refine_done(st, step, accept) || (!HASJ && refine_hard(st, step))) return;
+  const double sc = refine_scale2(frob2), noise2 = eps * eps * frob2[0] * sc, tol2 = tol * tol, utol2 = 16.0 * tol2;
+  const float skip = refine_skip<HASJ>(step, tol);
   unsigned rot = 0, unit = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e / n, k = e - i * n;
     if (i > k) continue;
     if (i == k) {
-      unit += d[i] * d[i] > utol2;
+      if (HASJ) unit += d[i] * d[i] > utol2;
       continue;
     }
-    const T g = GF[i * n + k] * sc, dl = GF[k * n + i];
-    const double ai = a[i] * sc, ak = a[k] * sc;
-    unit += abs2_(dl) > utol2;
+    if (i >= nkeep) continue;
+    const T g = GF[i * n + k] * sc, dl = HASJ ? GF[k * n + i] : zero_<T>();
+    const double ai = a[i] * sc, ak = a[k] * sc, di = HASJ ? d[i] : 0.0, dk = HASJ ? d[k] : 0.0;
+    if (HASJ) unit += abs2_(dl) > utol2;
     if (ai > noise2 && ak > noise2 && abs2_(g) > tol2 * (ai * ak)) {
       ++rot;
-      if (refine_pair<T>(g, dl, ai - ai * d[i], ak - ak * d[k], noise2, skip).large) {
-        atomicAdd(&rows_large[i], 1u);
-        atomicAdd(&rows_large[k], 1u);
+      if (refine_pair<T>(g, dl, ai - ai * di, ak - ak * dk, noise2, skip).large) {
+        // two in a row: the simultaneous rotations do not hold for them
+        const unsigned before = atomicAdd(&rows_large[i], 1u) + atomicAdd(&rows_large[k], 1u);
+        if (before) atomicOr(&st[step].hard, 1u);
+        if (partner) {  // read only where a row has one
+          partner[i] = (unsigned)k;
+          partner[k] = (unsigned)i;
+        }
       }
     }
   }
@@ -229,46 +253,52 @@ __global__ void refine_test_kernel(int64_t n, const T* __restrict__ GF, const ty
 
 // F^T in single precision, Ft[k][i] = F(i, k).  A pair takes its first-order
 // rotation, or, when its angle is large and neither row has another such pair,
-// the full one (with its part of the diagonal).  Late steps take small angles
-// only, so that what they leave of J's defect is below rounding.
-template <typename T>
+// the full one (with its part of the diagonal; without J, refine_pairs_kernel does
+// it in FP64).  Late steps take small angles only, so that what they leave of J's
+// defect is below rounding.
+template <typename T, bool HASJ>
 __global__ void refine_f_kernel(int64_t n, const T* __restrict__ GF, const typename traits<T>::real* __restrict__ a,
                                 const typename traits<T>::real* __restrict__ d, const double* frob2, double tol,
-                                RefineState* st, int step, const unsigned* __restrict__ rows_large,
+                                double eps, int64_t nkeep, RefineState* st, int step, float accept,
+                                const unsigned* __restrict__ rows_large,
                                 typename narrow_of<T>::type* __restrict__ Ft) {
   typedef typename narrow_of<T>::type S;
-  if (refine_done(st, step + 1)) return;
-  const double sc = refine_scale2(frob2), noise2 = noise_floor2<T>(frob2) * sc;
+  if (refine_idle(st, step, accept) || (!HASJ && refine_hard(st, step + 1))) return;
+  const double sc = refine_scale2(frob2), noise2 = eps * eps * frob2[0] * sc;
   const bool rotate = !refine_hard(st, step);
-  const float skip = refine_skip(step, tol), top = step < 2 ? 2.f : step == 2 ? 1e-5f : 1e-7f;
+  const float skip = refine_skip<HASJ>(step, tol), top = step < 2 ? 2.f : step == 2 ? 1e-5f : 1e-7f;
   // a warp takes row i: its own F(i, k) for every k, and F(i, i)
   const int lane = threadIdx.x & 31;
   float fmax2 = 0.f;
   for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n;
        i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-    const double di = d[i], raw = a[i] * sc, ai = raw - raw * di;
+    const double di = HASJ ? d[i] : 0.0, raw = a[i] * sc, ai = raw - raw * di;
     const unsigned li = rows_large[i];
     float diag = 0.f;
     for (int64_t k = lane; k < n; k += 32) {
       if (k == i) continue;
       const bool up = i < k;  // G above the diagonal, delta below it
-      const T g = (up ? GF[i * n + k] : GF[k * n + i]) * sc, dl = up ? GF[k * n + i] : GF[i * n + k];
-      const double rk = a[k] * sc, ak = rk - rk * d[k];
+      const T g = (up ? GF[i * n + k] : GF[k * n + i]) * sc;
+      const T dl = !HASJ ? zero_<T>() : up ? GF[k * n + i] : GF[i * n + k];
+      const double rk = a[k] * sc, ak = HASJ ? rk - rk * d[k] : rk;
       S f = zero_<S>();
-      if (rotate) {
+      if (rotate && (i < nkeep || k < nkeep)) {
         RefinePair<S> r = refine_pair<T>(g, dl, up ? ai : ak, up ? ak : ai, noise2, skip);
-        if (r.large && li == 1 && rows_large[k] == 1 && r.t < top) {
+        if (!HASJ && r.large && li == 1 && rows_large[k] == 1) {
+          r.f = zero_<S>();
+          fmax2 = 1.f;  // another look
+        } else if (HASJ && r.large && li == 1 && rows_large[k] == 1 && r.t < top) {
           const float c = 1.f / sqrtf(fmaf(r.t, r.t, 1.f));
           diag -= r.t * r.t * c / (1.f + 1.f / c);  // c - 1
           r.f = r.f * c;
-        } else if (r.large || r.t >= top) {
+        } else if (r.large || (HASJ && r.t >= top)) {
           r.f = zero_<S>();
           atomicOr(&st[step].hard, 1u);
         }
         f = up ? -r.f : conj_(r.f);
       }
       const bool larger = up ? raw >= rk : raw > rk;
-      if (larger) f = f - refine_narrow(up ? dl : conj_(dl));
+      if (HASJ && larger) f = f - refine_narrow(up ? dl : conj_(dl));
       Ft[k * n + i] = f;
       fmax2 = fmaxf(fmax2, abs2_(f));
     }
@@ -281,9 +311,9 @@ __global__ void refine_f_kernel(int64_t n, const T* __restrict__ GF, const typen
   if (lane == 0) atomicMax(reinterpret_cast<unsigned*>(&st[step].fmax), __float_as_uint(sqrtf(fmax2)));  // not negative
 }
 
-// X += F X for X = J and, with a small F, W (blockIdx.y = 1), in place by columns: a
-// CTA keeps C columns of X (rounded to FP32; W in units of 2^k) in shared memory
-// and a thread takes rows of the result, reading F^T along them.
+// X += F X for X = J (n x n) and, with a small F, W (blockIdx.y = 1), in place by
+// columns: a CTA keeps C columns of X (rounded to FP32; W in units of 2^k) in
+// shared memory and a thread takes rows of the result, reading F^T along them.
 template <typename T, int C>
 __global__ void __launch_bounds__(256)
 refine_apply_kernel(int64_t n, const typename narrow_of<T>::type* __restrict__ Ft, T* __restrict__ J, T* __restrict__ W,
@@ -291,7 +321,7 @@ refine_apply_kernel(int64_t n, const typename narrow_of<T>::type* __restrict__ F
   typedef typename narrow_of<T>::type S;
   extern __shared__ __align__(16) unsigned char refine_smem[];
   S* s = reinterpret_cast<S*>(refine_smem);  // [n][C]
-  if (refine_done(st, step + 1) || (blockIdx.y && !(st[step].fmax < kRefineDirect))) return;
+  if (refine_idle(st, step) || (blockIdx.y && !(st[step].fmax < kRefineDirect))) return;
   T* X = blockIdx.y ? W : J;
   const int e2 = blockIdx.y ? refine_exp(frob2) : 0;
   const int64_t c0 = (int64_t)blockIdx.x * C;
@@ -314,6 +344,124 @@ refine_apply_kernel(int64_t n, const typename narrow_of<T>::type* __restrict__ F
     for (int c = 0; c < C; ++c)
       if (c0 + c < n) X[i * n + c0 + c] = X[i * n + c0 + c] + refine_ldexp(refine_widen(acc[c]), e2);
   }
+}
+
+// (s, c) += f (h + l) with the rounding errors of products and sums kept in c
+// (TwoProd by FMA, TwoSum; Ogita, Rump and Oishi 2005): relative 2^-46 of the terms.
+__device__ __forceinline__ void comp_add(float& s, float& c, float f, float h, float l) {
+  const float p = __fmul_rn(f, h), e = __fmaf_rn(f, h, -p), t = __fadd_rn(s, p), z = __fsub_rn(t, s);
+  c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z)), e));
+  c = __fmaf_rn(f, l, c);
+  s = t;
+}
+__device__ __forceinline__ void comp_add(c64& s, c64& c, c64 f, c64 h, c64 l) {
+  comp_add(s.re, c.re, f.re, h.re, l.re);
+  comp_add(s.re, c.re, -f.im, h.im, l.im);
+  comp_add(s.im, c.im, f.re, h.im, l.im);
+  comp_add(s.im, c.im, f.im, h.re, l.re);
+}
+
+// W += F W + F F W / 2 without an accumulator: I + F + F^2 / 2 is unitary to |F|^4,
+// and F W is summed as exactly as W is held (F may reach 1e-3, and FP32 sums
+// would leave 6e-8 of that in the singular values).  By columns as above, W as a
+// pair of floats; up to four rows a thread (n <= 1024).
+template <typename T, int C>
+__global__ void __launch_bounds__(256)
+refine_rotate_kernel(int64_t n, int64_t cols, const typename narrow_of<T>::type* __restrict__ Ft, T* __restrict__ W,
+                     const double* frob2, const RefineState* st, int step, float accept) {
+  typedef typename narrow_of<T>::type S;
+  extern __shared__ __align__(16) unsigned char refine_smem[];
+  S* h = reinterpret_cast<S*>(refine_smem);  // [n][C] high parts
+  S* l = h + n * C;                          // low parts
+  if (refine_idle(st, step, accept) || refine_hard(st, step + 1)) return;
+  const int e2 = refine_exp(frob2);
+  const int64_t c0 = (int64_t)blockIdx.x * C;
+  for (int64_t e = threadIdx.x; e < n * C; e += blockDim.x) {
+    const int64_t i = e / C, c = c0 + e % C;
+    const T v = c < cols ? refine_ldexp(W[i * cols + c], -e2) : zero_<T>();
+    h[e] = refine_narrow(v);
+    l[e] = refine_narrow(v - refine_widen(h[e]));
+  }
+  __syncthreads();
+  S z[4][C];  // F W / 2
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t i = threadIdx.x + 256 * r;
+#pragma unroll
+    for (int c = 0; c < C; ++c) z[r][c] = zero_<S>();
+    if (i >= n) continue;
+#pragma unroll 8
+    for (int64_t k = 0; k < n; ++k) {
+      const S f = 0.5f * Ft[k * n + i];
+#pragma unroll
+      for (int c = 0; c < C; ++c) fma_(z[r][c], f, h[k * C + c]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t i = threadIdx.x + 256 * r;
+    if (i >= n) continue;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {  // the small part joins the low one
+      l[i * C + c] = l[i * C + c] + z[r][c];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int64_t i = threadIdx.x; i < n; i += 256) {
+    S acc[C], err[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = err[c] = zero_<S>();
+#pragma unroll 4
+    for (int64_t k = 0; k < n; ++k) {
+      const S f = Ft[k * n + i];
+#pragma unroll
+      for (int c = 0; c < C; ++c) comp_add(acc[c], err[c], f, h[k * C + c], l[k * C + c]);
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (c0 + c < cols) {
+        T* x = W + i * cols + c0 + c;
+        *x = *x + refine_ldexp(refine_widen(acc[c]) + refine_widen(err[c]), e2);
+      }
+  }
+}
+
+// The rotations of large angle whose rows have no other, in FP64: a warp takes the
+// pair of its row.
+template <typename T>
+__global__ void refine_pairs_kernel(int64_t n, int64_t cols, const T* __restrict__ GF,
+                                    const typename traits<T>::real* __restrict__ a, T* __restrict__ W,
+                                    const RefineState* st, int step, float accept, const unsigned* __restrict__ rows_large,
+                                    const unsigned* __restrict__ partner) {
+  if (refine_idle(st, step, accept) || refine_hard(st, step + 1)) return;
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n;
+       i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
+    if (rows_large[i] != 1) continue;
+    const int64_t k = partner[i];
+    if (k <= i || rows_large[k] != 1) continue;
+    const T g = GF[i * n + k];
+    const double h = abs_(g), tau = (a[k] - a[i]) / (2 * h);
+    const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+    const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
+    const T se = s * div_real_(g, h);
+    T *x = W + i * cols, *y = W + k * cols;
+    for (int64_t e = lane; e < cols; e += 32) {
+      const T xv = x[e], yv = y[e];
+      x[e] = c * xv - se * yv;
+      y[e] = conj_(se) * xv + c * yv;
+    }
+  }
+}
+
+// Row tiles of the half that refine_gram_kernel takes.
+inline unsigned refine_half_tiles(int64_t n) {
+  const int64_t rows = (n + 7) / 8, cols = (n + 15) / 16;
+  int64_t half = 0;
+  for (int64_t c = 0; c < cols; ++c) half += 2 * (c + 1) < rows ? 2 * (c + 1) : rows;
+  return (unsigned)half;
 }
 
 }  // namespace tnc

@@ -28,6 +28,7 @@
 #include "tnc_df.cuh"
 #include "tnc_persist.cuh"
 #include "tnc_rot.cuh"
+#include "tnc_svd_refine.cuh"
 
 #include <atomic>
 #include <type_traits>
@@ -38,6 +39,7 @@ namespace tnc {
 // of the rotations above the stage-stop tolerance per sweep, then one step
 // counter per half-block
 constexpr int kRowsMaxSweeps = 100;
+constexpr int kDfSteps = 3;  // steps of the finish's refinement
 
 __device__ __forceinline__ void circle_pair(int64_t np, int64_t r, int64_t i, int64_t& p, int64_t& q) {
   const int64_t mod = np - 1;
@@ -356,8 +358,9 @@ template <typename T>
 __global__ void __launch_bounds__(kBlockThreads, jacobi_min_blocks<T>())
 jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double tol, const double* frob2,
                     typename traits<T>::real* Dn, unsigned* counters, unsigned* ver, SyncWords* sw, int* info,
-                    int64_t nkeep, double stop_tol) {
+                    int64_t nkeep, double stop_tol, const RefineState* refined, float accept) {
   typedef typename traits<T>::real R;
+  if (refined && refine_done(refined, kDfSteps + 1, accept)) return;  // nothing left to rotate
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sB = reinterpret_cast<T*>(smem_raw);
   __shared__ R sn[32];   // squared norms of the shared-memory rows
@@ -850,7 +853,7 @@ static int ensure_smem_attr() {
 template <typename T>
 static int launch_block(T* W, int64_t nr, int64_t L, int h, int ms, double tol, const double* frob2,
                         typename traits<T>::real* Dn, unsigned* counters, SyncWords* sw, int* info, int64_t nkeep,
-                        cudaStream_t st, double stop_tol = 0.0) {
+                        cudaStream_t st, double stop_tol = 0.0, const RefineState* refined = nullptr, float accept = 0.f) {
   const size_t smem = (size_t)2 * h * L * sizeof(T);
   const void* fn = (const void*)jacobi_block_kernel<T>;
   if (smem > kMaxHalfBlockBytes || 32 * h > kBlockThreads) return TNC_ERR_ARG;
@@ -872,7 +875,8 @@ static int launch_block(T* W, int64_t nr, int64_t L, int h, int ms, double tol, 
   int64_t nkeep_ = nkeep;
   double stop_ = stop_tol;
   void* args[] = {(void*)&W,  (void*)&nr_,      (void*)&L_,  (void*)&h_,  (void*)&ms_,   (void*)&tol_,    (void*)&frob2,
-                  (void*)&Dn, (void*)&counters, (void*)&ver, (void*)&sw,  (void*)&info,  (void*)&nkeep_,  (void*)&stop_};
+                  (void*)&Dn, (void*)&counters, (void*)&ver, (void*)&sw,  (void*)&info,  (void*)&nkeep_,  (void*)&stop_,
+                    (void*)&refined, (void*)&accept};
   if (cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st) != cudaSuccess) return TNC_ERR_CUDA;
   return TNC_OK;
 }
@@ -1075,6 +1079,37 @@ __device__ __forceinline__ dfc df_widen(c64 v, int k) {
 __device__ __forceinline__ double df_narrow(dfr v, int k) { return ldexp(to_double(v), k); }
 __device__ __forceinline__ c128 df_narrow(dfc v, int k) { return c128(ldexp(to_double(v.re), k), ldexp(to_double(v.im), k)); }
 
+// FP64 rows in place to DF rows 2^-k, when the refinement left something to rotate
+template <typename Tdf> struct wide_of { typedef double type; };
+template <> struct wide_of<dfc> { typedef c128 type; };
+__device__ __forceinline__ dfr df_of_wide(double v, int k) { return dfr(ldexp(v, -k)); }
+__device__ __forceinline__ dfc df_of_wide(c128 v, int k) {
+  dfc r;
+  r.re = df_of_wide(v.re, k);
+  r.im = df_of_wide(v.im, k);
+  return r;
+}
+template <typename Tdf>
+__global__ void df_from_wide_kernel(int64_t n, Tdf* W, double* frob2, const RefineState* refined, float accept) {
+  if (refine_done(refined, kDfSteps + 1, accept)) return;
+  const int k = df_scale_exp(frob2);
+  if (blockIdx.x == 0 && threadIdx.x == 0) frob2[1] = ldexp(frob2[0], -2 * k);
+  const auto* in = reinterpret_cast<const typename wide_of<Tdf>::type*>(W);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const auto v = in[i];
+    W[i] = df_of_wide(v, k);
+  }
+}
+// ... and the status of a finish that left nothing
+__global__ void df_refined_status(const RefineState* refined, float accept, int* info) {
+  if (!refine_done(refined, kDfSteps + 1, accept)) return;
+  int steps = 0;
+  while (steps < kDfSteps && !refine_done(refined, steps + 1, accept)) ++steps;
+  const bool checked = refined[steps].rot == 0;
+  info[1] = steps + 1;
+  info[3] = checked ? 0 : 1;
+}
+
 // W = A 2^-k as DF; frob2[1] = frob2[0] 2^-2k (the scaled rows' squared norm)
 template <typename Tin, typename Tdf>
 __global__ void df_widen_kernel(int64_t n, const Tin* A, Tdf* W, double* frob2) {
@@ -1085,7 +1120,8 @@ __global__ void df_widen_kernel(int64_t n, const Tin* A, Tdf* W, double* frob2) 
 }
 // in place: the DF element i becomes the FP64 element i (same size) times 2^k
 template <typename Tdf, typename Tout>
-__global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2) {
+__global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2, const RefineState* refined, float accept) {
+  if (refined && refine_done(refined, kDfSteps + 1, accept)) return;  // FP64 rows already
   static_assert(sizeof(Tdf) == sizeof(Tout), "in-place narrowing keeps the element size");
   const int k = df_scale_exp(frob2);
   Tout* out = reinterpret_cast<Tout*>(W);
@@ -1093,6 +1129,34 @@ __global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2) {
     const Tdf v = W[i];
     out[i] = df_narrow(v, k);
   }
+}
+
+// The finish first takes a few steps of whole-matrix products in FP64
+// (tnc_svd_refine.cuh, here without an accumulator): G = W W^H of the widened rows
+// and W += F W, F in FP32.  From the single-precision stage's 1e-6 one step leaves
+// about 1e-10 and is accepted without another look when |F| is below kDfStopTol,
+// as a sweep of small rotations is; pairs of clustered values take a second step,
+// and what is left then goes to the double-float Jacobi.  Rows of 512 complex64
+// elements, 512 of them: 1.5 ms, of which a Gram matrix is 0.5 and F's product 0.2,
+// where the Jacobi took 2.2 to 3.5; the values are 2e-14 off instead of 2e-13.
+constexpr int64_t kDfRefineMin = 24;
+constexpr int kDfRefineSweeps = 8;  // a smaller cap of the caller's is the Jacobi's
+struct DfRefine {
+  size_t g, ft, large, state, total;
+};
+static DfRefine df_refine_layout(int64_t nr, size_t es) {
+  DfRefine X;
+  size_t off = 0;
+  X.g = off; off = align256(off + (size_t)nr * nr * es);
+  X.ft = off; off = align256(off + (size_t)nr * nr * (es / 2));
+  X.large = off; off = align256(off + 2 * (size_t)nr * sizeof(unsigned));  // and the partners
+  X.state = off; off = align256(off + (kDfSteps + 1) * sizeof(RefineState));
+  X.total = off;
+  return X;
+}
+// refine_rotate_kernel holds four columns of pairs in 48 KB and four rows a thread.
+static bool df_refine_fits(int64_t nr, size_t es) {
+  return nr >= kDfRefineMin && nr <= 1024 && 8 * (size_t)nr * (es / 2) <= 48 * 1024;
 }
 
 // The finish of single-precision rows in double-float: A (m x n, m <= n,
@@ -1122,21 +1186,55 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
   if (cudaMemsetAsync(info, 0, 4 * sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(frob2, 0, 2 * sizeof(double), st) != cudaSuccess) return TNC_ERR_CUDA;
   frob2_kernel<Tin><<<grid1d(nr * L, 256, 152 * 4), 256, 0, st>>>(nr * L, A, frob2);
-  df_widen_kernel<Tin, Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, A, W, frob2);
   int launched = 2;
+  const RefineState* refined = nullptr;
+  float accept = 0.f;
+  const DfRefine X = df_refine_layout(nr, sizeof(Tout));
+  if (df_refine_fits(nr, sizeof(Tout)) && max_sweeps >= kDfRefineSweeps && wb >= Ly.total + X.total) {
+    typedef typename narrow_of<Tout>::type S;
+    char* x = w + Ly.total;
+    Tout *Wd = (Tout*)Wv, *G = (Tout*)(x + X.g);
+    S* Ft = (S*)(x + X.ft);
+    unsigned* large = (unsigned*)(x + X.large);
+    RefineState* rs = (RefineState*)(x + X.state);
+    accept = tol >= 1e-8 ? (float)kDfStopTol : 0.f;
+    const double eps = traits<Tdf>::eps;
+    const int64_t keep = nkeep < nr ? (nkeep + 7) / 8 * 8 : nr;  // whole half-blocks, as below
+    const unsigned half = refine_half_tiles(nr), g = grid1d(nr * nr, 256);
+    if (cudaMemsetAsync(rs, 0, (kDfSteps + 1) * sizeof(RefineState), st) != cudaSuccess) return TNC_ERR_CUDA;
+    if (int rc = tnc_cast(dtype_code<Tin>(), dtype_code<Tout>(), nr * L, A, Wd, st)) return rc;
+    for (int s = 0; s <= kDfSteps; ++s) {
+      refine_gram_kernel<Tout><<<dim3(half, 1), TileS<Tout>::THR, 0, st>>>(nr, L, Wd, (const Tout*)nullptr, G, D,
+                                                                         (double*)nullptr, rs, s, accept, large);
+      refine_test_kernel<Tout, false><<<g, 256, 0, st>>>(nr, G, D, nullptr, frob2, tol, eps, keep, rs, s, accept, large,
+                                                               large + nr);
+      if (s == kDfSteps) break;
+      refine_f_kernel<Tout, false><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, G, D, nullptr, frob2, tol, eps, keep, rs, s,
+                                                                       accept, large, Ft);
+      refine_rotate_kernel<Tout, 4><<<(unsigned)((L + 3) / 4), 256, 8 * nr * sizeof(S), st>>>(nr, L, Ft, Wd, frob2, rs, s,
+                                                                                            accept);
+      refine_pairs_kernel<Tout><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, L, G, D, Wd, rs, s, accept, large, large + nr);
+    }
+    df_from_wide_kernel<Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2, rs, accept);
+    df_refined_status<<<1, 1, 0, st>>>(rs, accept, info);
+    refined = rs;
+    launched += 5 * kDfSteps + 3;
+  } else {
+    df_widen_kernel<Tin, Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, A, W, frob2);
+  }
   if (nr > 1) {
     int h = 8;
     if (block_rows == 2 || block_rows == 4) h = block_rows;
     while (h > 2 && (size_t)2 * h * L * sizeof(Tdf) > kMaxHalfBlockBytes) h >>= 1;
     while (h > 2 && h / 2 >= nr) h >>= 1;
     if ((size_t)2 * h * L * sizeof(Tdf) > kMaxHalfBlockBytes) return TNC_ERR_ARG;  // rows too long
-    if (int rc = launch_block<Tdf>(W, nr, L, h, max_sweeps, tol, frob2 + 1, Dn, counters, sw, info,
-                                                 nkeep, st, kDfStopTol))
+    if (int rc = launch_block<Tdf>(W, nr, L, h, max_sweeps, tol, frob2 + 1, Dn, counters, sw, info, nkeep, st, kDfStopTol,
+                                   refined, accept))
       return rc;
     ++launched;
   }
   copy_sync_error<<<1, 1, 0, st>>>(sw, info);
-  df_narrow_kernel<Tdf, Tout><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2);
+  df_narrow_kernel<Tdf, Tout><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2, refined, accept);
   rows_norm_kernel<Tout><<<grid1d(nr * 32, 256), 256, 0, st>>>((const Tout*)Wv, nr, L, D, info);
   sort_desc_kernel<double><<<grid1d(nr, 128), 128, 0, st>>>(D, nr, order, S);
   return launch_status(4 + launched);
@@ -1151,7 +1249,9 @@ using namespace tnc;
 extern "C" int tnc_svd_rows_workspace_size(int dtype, int64_t m, int64_t n, size_t* bytes) {
   if (!elem_size(dtype) || m <= 0 || n <= 0 || !bytes) return TNC_ERR_ARG;
   size_t rs = (dtype == TNC_F32 || dtype == TNC_C64) ? 4 : 8;
-  *bytes = rows_layout(m < n ? m : n, rs).total;
+  const int64_t nr = m < n ? m : n;
+  const size_t es = (size_t)elem_size(dtype);
+  *bytes = rows_layout(nr, rs).total + (rs == 8 && df_refine_fits(nr, es) ? df_refine_layout(nr, es).total : 0);
   return TNC_OK;
 }
 
