@@ -162,6 +162,17 @@ __device__ __forceinline__ void j32_stg(T* row, int L, bool vec, const float2 (&
   }
 }
 
+// Step counters: the store publishes what the warp stored before it, the load takes
+// what was published (rows are read through L2, so no fence follows it).
+__device__ __forceinline__ void j32_publish(unsigned* p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned j32_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 struct J32Args {
   void *W, *J;  // rows of L elements each (J: ACC only)
   int nr, L, h, N, kb, max_sweeps, vec;  // N: half-blocks, padded to even; kb: half-blocks with kept rows
@@ -208,21 +219,17 @@ jacobi32_kernel(const J32Args p) {
     if constexpr (ACC) j32_stg<T, P, D, D>(J + (int64_t)row * p.L, p.L, vec, v);
     if (lane == 0) __stcg(p.Dn + row, n2);
     __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      *(volatile unsigned*)(p.ver + row) = step;
-    }
+    if (lane == 0) j32_publish(p.ver + row, step);
   };
   auto take_row = [&](int row, unsigned step) {
     if (ok) {
       int good = 1;
       if (lane == 0) {
         const long long limit = spin_limit();
-        for (long long spins = 0; ld_volatile(p.ver + row) < step; ++spins) {
+        for (long long spins = 0; j32_acquire(p.ver + row) < step; ++spins) {
           if (ld_volatile(&p.sw->err)) { good = 0; break; }
           if (spins > limit) { atomicCAS(&p.sw->err, 0, TNC_ERR_TIMEOUT); good = 0; break; }
         }
-        __threadfence();
       }
       ok = __shfl_sync(0xffffffffu, good, 0) != 0;
       __syncwarp();
