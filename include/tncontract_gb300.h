@@ -342,7 +342,7 @@ int tnc_permute_rows(int dtype, int64_t n, int64_t L, const void *src,
  * the orthogonalised rows as FP64 / complex128 elements, S (FP64) and order
  * as tnc_svd_rows for the FP64 type, and the rows are orthogonal to tol
  * relative (<= 0: 1e-7).  24 rows or more first take a few steps that rotate
- * every pair at once, as FP64 and compensated FP32 products of the whole matrix;
+ * every pair at once, as compensated FP32 products of the whole matrix;
  * what they leave (clusters of nearly equal values) the double-float Jacobi
  * takes.  Either ends without a checking pass (info[3] = 1) after one whose
  * rotations were all small angles below 1e-5: their residual is second order.

@@ -267,7 +267,7 @@ static int svd_refine(int64_t nr, const T* R, T* J, T* Wb, T* GF, char* scratch,
   const double eps = traits<T>::eps;
   refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, 0);
   for (int s = 0; s <= kRefineSteps; ++s) {
-    refine_gram_kernel<T><<<dim3(half, 2), G::THR, 0, st>>>(nr, nr, Wb, J, GF, a, d, rs, s, -1.f, js.rows_large);
+    refine_gram_kernel<T><<<dim3(half, 2), G::THR, 0, st>>>(nr, Wb, J, GF, a, d, rs, s, js.rows_large);
     refine_test_kernel<T, true><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, eps, nr, rs, s, -1.f, js.rows_large,
                                                      nullptr);
     if (s == kRefineSteps) break;

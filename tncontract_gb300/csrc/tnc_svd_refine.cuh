@@ -120,18 +120,17 @@ refine_product_kernel(int64_t n, const T* __restrict__ J, const T* __restrict__ 
   if (gm < n && gn < n) W[gm * n + gn] = acc[0][0];
 }
 
-// X = W (blockIdx.y = 0; n rows of K elements) or J (1; n x n): <x_i, x_k> for
-// i < k, G's above the diagonal of GF, delta's below it (at (k, i)); the diagonals
+// X = W (blockIdx.y = 0) or J (1), n x n: <x_i, x_k> for i < k, G's above the diagonal of GF, delta's below it (at (k, i)); the diagonals
 // to a and d.
 template <typename T>
 __global__ void __launch_bounds__(TileS<T>::THR)
-refine_gram_kernel(int64_t n, int64_t K, const T* __restrict__ W, const T* __restrict__ J, T* __restrict__ GF,
+refine_gram_kernel(int64_t n, const T* __restrict__ W, const T* __restrict__ J, T* __restrict__ GF,
                    typename traits<T>::real* __restrict__ a, typename traits<T>::real* __restrict__ d,
-                   const RefineState* st, int upto, float accept, unsigned* rows_large) {
+                   const RefineState* st, int upto, unsigned* rows_large) {
   typedef TileS<T> G;
   __shared__ __align__(16) T As[2][G::BK * G::LDA];
   __shared__ __align__(16) T Bs[2][G::BK * G::LDB];
-  if (refine_done(st, upto, accept) || (J == nullptr && refine_hard(st, upto))) return;
+  if (refine_done(st, upto)) return;
   if (blockIdx.y == 0)
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
       rows_large[i] = 0;
@@ -147,9 +146,8 @@ refine_gram_kernel(int64_t n, int64_t K, const T* __restrict__ W, const T* __res
   if (cb >= cols) return;
   const int64_t m0 = t * G::BM, n0 = cb * G::BN;
   const T* X = blockIdx.y ? J : W;
-  const int64_t kx = blockIdx.y ? n : K;
   T acc[G::TM][G::TN];
-  gemm_acc<T, G, true, true>(n, n, kx, false, true, X, kx, X, kx, m0, n0, As, Bs, acc);
+  gemm_acc<T, G, true, true>(n, n, n, false, true, X, n, X, n, m0, n0, As, Bs, acc);
   const int64_t i = m0 + tile_row<G>(0), k = n0 + tile_col<G>(0);
   if (i > k || k >= n) return;
   const T v = acc[0][0];
@@ -343,116 +341,6 @@ refine_apply_kernel(int64_t n, const typename narrow_of<T>::type* __restrict__ F
 #pragma unroll
     for (int c = 0; c < C; ++c)
       if (c0 + c < n) X[i * n + c0 + c] = X[i * n + c0 + c] + refine_ldexp(refine_widen(acc[c]), e2);
-  }
-}
-
-// (s, c) += f (h + l) with the rounding errors of products and sums kept in c
-// (TwoProd by FMA, TwoSum; Ogita, Rump and Oishi 2005): relative 2^-46 of the terms.
-__device__ __forceinline__ void comp_add(float& s, float& c, float f, float h, float l) {
-  const float p = __fmul_rn(f, h), e = __fmaf_rn(f, h, -p), t = __fadd_rn(s, p), z = __fsub_rn(t, s);
-  c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z)), e));
-  c = __fmaf_rn(f, l, c);
-  s = t;
-}
-__device__ __forceinline__ void comp_add(c64& s, c64& c, c64 f, c64 h, c64 l) {
-  comp_add(s.re, c.re, f.re, h.re, l.re);
-  comp_add(s.re, c.re, -f.im, h.im, l.im);
-  comp_add(s.im, c.im, f.re, h.im, l.im);
-  comp_add(s.im, c.im, f.im, h.re, l.re);
-}
-
-// W += F W + F F W / 2 without an accumulator: I + F + F^2 / 2 is unitary to |F|^4,
-// and F W is summed as exactly as W is held (F may reach 1e-3, and FP32 sums
-// would leave 6e-8 of that in the singular values).  By columns as above, W as a
-// pair of floats; up to four rows a thread (n <= 1024).
-template <typename T, int C>
-__global__ void __launch_bounds__(256)
-refine_rotate_kernel(int64_t n, int64_t cols, const typename narrow_of<T>::type* __restrict__ Ft, T* __restrict__ W,
-                     const double* frob2, const RefineState* st, int step, float accept) {
-  typedef typename narrow_of<T>::type S;
-  extern __shared__ __align__(16) unsigned char refine_smem[];
-  S* h = reinterpret_cast<S*>(refine_smem);  // [n][C] high parts
-  S* l = h + n * C;                          // low parts
-  if (refine_idle(st, step, accept) || refine_hard(st, step + 1)) return;
-  const int e2 = refine_exp(frob2);
-  const int64_t c0 = (int64_t)blockIdx.x * C;
-  for (int64_t e = threadIdx.x; e < n * C; e += blockDim.x) {
-    const int64_t i = e / C, c = c0 + e % C;
-    const T v = c < cols ? refine_ldexp(W[i * cols + c], -e2) : zero_<T>();
-    h[e] = refine_narrow(v);
-    l[e] = refine_narrow(v - refine_widen(h[e]));
-  }
-  __syncthreads();
-  S z[4][C];  // F W / 2
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int64_t i = threadIdx.x + 256 * r;
-#pragma unroll
-    for (int c = 0; c < C; ++c) z[r][c] = zero_<S>();
-    if (i >= n) continue;
-#pragma unroll 8
-    for (int64_t k = 0; k < n; ++k) {
-      const S f = 0.5f * Ft[k * n + i];
-#pragma unroll
-      for (int c = 0; c < C; ++c) fma_(z[r][c], f, h[k * C + c]);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int64_t i = threadIdx.x + 256 * r;
-    if (i >= n) continue;
-#pragma unroll
-    for (int c = 0; c < C; ++c) {  // the small part joins the low one
-      l[i * C + c] = l[i * C + c] + z[r][c];
-    }
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int64_t i = threadIdx.x; i < n; i += 256) {
-    S acc[C], err[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = err[c] = zero_<S>();
-#pragma unroll 4
-    for (int64_t k = 0; k < n; ++k) {
-      const S f = Ft[k * n + i];
-#pragma unroll
-      for (int c = 0; c < C; ++c) comp_add(acc[c], err[c], f, h[k * C + c], l[k * C + c]);
-    }
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-      if (c0 + c < cols) {
-        T* x = W + i * cols + c0 + c;
-        *x = *x + refine_ldexp(refine_widen(acc[c]) + refine_widen(err[c]), e2);
-      }
-  }
-}
-
-// The rotations of large angle whose rows have no other, in FP64: a warp takes the
-// pair of its row.
-template <typename T>
-__global__ void refine_pairs_kernel(int64_t n, int64_t cols, const T* __restrict__ GF,
-                                    const typename traits<T>::real* __restrict__ a, T* __restrict__ W,
-                                    const RefineState* st, int step, float accept, const unsigned* __restrict__ rows_large,
-                                    const unsigned* __restrict__ partner) {
-  if (refine_idle(st, step, accept) || refine_hard(st, step + 1)) return;
-  const int lane = threadIdx.x & 31;
-  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n;
-       i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-    if (rows_large[i] != 1) continue;
-    const int64_t k = partner[i];
-    if (k <= i || rows_large[k] != 1) continue;
-    const T g = GF[i * n + k];
-    const double h = abs_(g), tau = (a[k] - a[i]) / (2 * h);
-    const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-    const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-    const T se = s * div_real_(g, h);
-    T *x = W + i * cols, *y = W + k * cols;
-    for (int64_t e = lane; e < cols; e += 32) {
-      const T xv = x[e], yv = y[e];
-      x[e] = c * xv - se * yv;
-      y[e] = conj_(se) * xv + c * yv;
-    }
   }
 }
 

@@ -25,10 +25,9 @@
 // That is 2n/h dependent steps per sweep instead of n for a point ordering,
 // and each rotation streams its rows through shared memory instead of L2.  One cooperative launch runs all sweeps; every wait is
 // bounded (tnc_persist.cuh).
-#include "tnc_df.cuh"
+#include "tnc_df_refine.cuh"
 #include "tnc_persist.cuh"
 #include "tnc_rot.cuh"
-#include "tnc_svd_refine.cuh"
 
 #include <atomic>
 #include <type_traits>
@@ -1079,28 +1078,7 @@ __device__ __forceinline__ dfc df_widen(c64 v, int k) {
 __device__ __forceinline__ double df_narrow(dfr v, int k) { return ldexp(to_double(v), k); }
 __device__ __forceinline__ c128 df_narrow(dfc v, int k) { return c128(ldexp(to_double(v.re), k), ldexp(to_double(v.im), k)); }
 
-// FP64 rows in place to DF rows 2^-k, when the refinement left something to rotate
-template <typename Tdf> struct wide_of { typedef double type; };
-template <> struct wide_of<dfc> { typedef c128 type; };
-__device__ __forceinline__ dfr df_of_wide(double v, int k) { return dfr(ldexp(v, -k)); }
-__device__ __forceinline__ dfc df_of_wide(c128 v, int k) {
-  dfc r;
-  r.re = df_of_wide(v.re, k);
-  r.im = df_of_wide(v.im, k);
-  return r;
-}
-template <typename Tdf>
-__global__ void df_from_wide_kernel(int64_t n, Tdf* W, double* frob2, const RefineState* refined, float accept) {
-  if (refine_done(refined, kDfSteps + 1, accept)) return;
-  const int k = df_scale_exp(frob2);
-  if (blockIdx.x == 0 && threadIdx.x == 0) frob2[1] = ldexp(frob2[0], -2 * k);
-  const auto* in = reinterpret_cast<const typename wide_of<Tdf>::type*>(W);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const auto v = in[i];
-    W[i] = df_of_wide(v, k);
-  }
-}
-// ... and the status of a finish that left nothing
+// The status of a finish whose refinement left nothing.
 __global__ void df_refined_status(const RefineState* refined, float accept, int* info) {
   if (!refine_done(refined, kDfSteps + 1, accept)) return;
   int steps = 0;
@@ -1120,8 +1098,7 @@ __global__ void df_widen_kernel(int64_t n, const Tin* A, Tdf* W, double* frob2) 
 }
 // in place: the DF element i becomes the FP64 element i (same size) times 2^k
 template <typename Tdf, typename Tout>
-__global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2, const RefineState* refined, float accept) {
-  if (refined && refine_done(refined, kDfSteps + 1, accept)) return;  // FP64 rows already
+__global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2) {
   static_assert(sizeof(Tdf) == sizeof(Tout), "in-place narrowing keeps the element size");
   const int k = df_scale_exp(frob2);
   Tout* out = reinterpret_cast<Tout*>(W);
@@ -1131,14 +1108,14 @@ __global__ void df_narrow_kernel(int64_t n, Tdf* W, const double* frob2, const R
   }
 }
 
-// The finish first takes a few steps of whole-matrix products in FP64
-// (tnc_svd_refine.cuh, here without an accumulator): G = W W^H of the widened rows
-// and W += F W, F in FP32.  From the single-precision stage's 1e-6 one step leaves
+// The finish first takes a few steps of whole-matrix products (tnc_svd_refine.cuh,
+// here without an accumulator and on double-float rows, tnc_df_refine.cuh):
+// G = W W^H and W += F W.  From the single-precision stage's 1e-6 one step leaves
 // about 1e-10 and is accepted without another look when |F| is below kDfStopTol,
 // as a sweep of small rotations is; pairs of clustered values take a second step,
 // and what is left then goes to the double-float Jacobi.  Rows of 512 complex64
-// elements, 512 of them: 1.5 ms, of which a Gram matrix is 0.5 and F's product 0.2,
-// where the Jacobi took 2.2 to 3.5; the values are 2e-14 off instead of 2e-13.
+// elements, 512 of them: 1.0 ms, where the Jacobi took 2.2 to 3.5; the values are
+// 2e-14 off instead of 2e-13.
 constexpr int64_t kDfRefineMin = 24;
 constexpr int kDfRefineSweeps = 8;  // a smaller cap of the caller's is the Jacobi's
 struct DfRefine {
@@ -1154,7 +1131,7 @@ static DfRefine df_refine_layout(int64_t nr, size_t es) {
   X.total = off;
   return X;
 }
-// refine_rotate_kernel holds four columns of pairs in 48 KB and four rows a thread.
+// df_rotate_kernel holds four columns of pairs in 48 KB and four rows a thread.
 static bool df_refine_fits(int64_t nr, size_t es) {
   return nr >= kDfRefineMin && nr <= 1024 && 8 * (size_t)nr * (es / 2) <= 48 * 1024;
 }
@@ -1186,41 +1163,38 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
   if (cudaMemsetAsync(info, 0, 4 * sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(frob2, 0, 2 * sizeof(double), st) != cudaSuccess) return TNC_ERR_CUDA;
   frob2_kernel<Tin><<<grid1d(nr * L, 256, 152 * 4), 256, 0, st>>>(nr * L, A, frob2);
+  df_widen_kernel<Tin, Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, A, W, frob2);
   int launched = 2;
   const RefineState* refined = nullptr;
   float accept = 0.f;
   const DfRefine X = df_refine_layout(nr, sizeof(Tout));
   if (df_refine_fits(nr, sizeof(Tout)) && max_sweeps >= kDfRefineSweeps && wb >= Ly.total + X.total) {
-    typedef typename narrow_of<Tout>::type S;
+    typedef typename df_parts<Tdf>::S S;
     char* x = w + Ly.total;
-    Tout *Wd = (Tout*)Wv, *G = (Tout*)(x + X.g);
+    Tout* G = (Tout*)(x + X.g);
     S* Ft = (S*)(x + X.ft);
     unsigned* large = (unsigned*)(x + X.large);
     RefineState* rs = (RefineState*)(x + X.state);
+    const double* f2 = frob2 + 1;  // of the scaled rows
     accept = tol >= 1e-8 ? (float)kDfStopTol : 0.f;
     const double eps = traits<Tdf>::eps;
     const int64_t keep = nkeep < nr ? (nkeep + 7) / 8 * 8 : nr;  // whole half-blocks, as below
-    const unsigned half = refine_half_tiles(nr), g = grid1d(nr * nr, 256);
+    const int64_t tiles = (nr + kDfTile - 1) / kDfTile;
+    const unsigned g = grid1d(nr * nr, 256);
     if (cudaMemsetAsync(rs, 0, (kDfSteps + 1) * sizeof(RefineState), st) != cudaSuccess) return TNC_ERR_CUDA;
-    if (int rc = tnc_cast(dtype_code<Tin>(), dtype_code<Tout>(), nr * L, A, Wd, st)) return rc;
     for (int s = 0; s <= kDfSteps; ++s) {
-      refine_gram_kernel<Tout><<<dim3(half, 1), TileS<Tout>::THR, 0, st>>>(nr, L, Wd, (const Tout*)nullptr, G, D,
-                                                                         (double*)nullptr, rs, s, accept, large);
-      refine_test_kernel<Tout, false><<<g, 256, 0, st>>>(nr, G, D, nullptr, frob2, tol, eps, keep, rs, s, accept, large,
-                                                               large + nr);
+      df_gram_kernel<Tdf><<<(unsigned)(tiles * (tiles + 1) / 2), 256, 0, st>>>(nr, L, W, G, D, rs, s, accept, large);
+      refine_test_kernel<Tout, false><<<g, 256, 0, st>>>(nr, G, D, nullptr, f2, tol, eps, keep, rs, s, accept, large,
+                                                         large + nr);
       if (s == kDfSteps) break;
-      refine_f_kernel<Tout, false><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, G, D, nullptr, frob2, tol, eps, keep, rs, s,
+      refine_f_kernel<Tout, false><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, G, D, nullptr, f2, tol, eps, keep, rs, s,
                                                                        accept, large, Ft);
-      refine_rotate_kernel<Tout, 4><<<(unsigned)((L + 3) / 4), 256, 8 * nr * sizeof(S), st>>>(nr, L, Ft, Wd, frob2, rs, s,
-                                                                                            accept);
-      refine_pairs_kernel<Tout><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, L, G, D, Wd, rs, s, accept, large, large + nr);
+      df_rotate_kernel<Tdf, 4><<<(unsigned)((L + 3) / 4), 256, 8 * nr * sizeof(S), st>>>(nr, L, Ft, W, rs, s, accept);
+      df_pairs_kernel<Tdf><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, L, G, D, W, rs, s, accept, large, large + nr);
     }
-    df_from_wide_kernel<Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2, rs, accept);
     df_refined_status<<<1, 1, 0, st>>>(rs, accept, info);
     refined = rs;
     launched += 5 * kDfSteps + 3;
-  } else {
-    df_widen_kernel<Tin, Tdf><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, A, W, frob2);
   }
   if (nr > 1) {
     int h = 8;
@@ -1234,7 +1208,7 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
     ++launched;
   }
   copy_sync_error<<<1, 1, 0, st>>>(sw, info);
-  df_narrow_kernel<Tdf, Tout><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2, refined, accept);
+  df_narrow_kernel<Tdf, Tout><<<grid1d(nr * L, 256), 256, 0, st>>>(nr * L, W, frob2);
   rows_norm_kernel<Tout><<<grid1d(nr * 32, 256), 256, 0, st>>>((const Tout*)Wv, nr, L, D, info);
   sort_desc_kernel<double><<<grid1d(nr, 128), 128, 0, st>>>(D, nr, order, S);
   return launch_status(4 + launched);
