@@ -378,17 +378,29 @@ static int launch_panel(T* P, int64_t ld, int m, int nb, T* tau, T* Tout, int* i
                                                                                                          : TNC_ERR_CUDA;
 }
 
-// Rows of a CTA by the panel's length: FP32 panels stay within the portable
-// cluster of 8 as long as they can (a step's barrier and reduction take 1160
-// cycles over 8 CTAs and 1700 over 16, measured); FP64 panels spread over 16
-// as soon as possible, their arithmetic being the longer part.
+// Rows of a lane (R; a CTA holds 32 R) by the panel's length.  FP32: a step's
+// arithmetic grows with R, its exchange with the CTAs, and empty rows cost as
+// much as full ones.  So R goes in steps of one for complex types (real ones
+// pack rows in pairs and gain nothing from an odd R beyond 3), on 4 CTAs up to
+// 512 rows (1024 for real types) and else on 8, the portable cluster (16 CTAs of
+// half the rows: 3.30 ms for 1536 x 768 complex64, 2.84 on 8).  Against R of 2,
+// 4, 6 and 8 on 8 CTAs: 1536 x 768 complex64 2.83 -> 2.78 ms, 768 x 512 1.47 ->
+// 1.43, 1280 x 64 0.238 -> 0.225; float32 512 x 256 0.606 -> 0.559, 768 x 64
+// 0.186 -> 0.177.  FP64 panels spread over 16 CTAs as soon as possible, their
+// arithmetic being the longer part.
 template <typename T>
 static int qr_panel(T* P, int64_t ld, int64_t m, int64_t nb, T* tau, T* Tout, int* info, cudaStream_t st) {
   const int rows = (int)m, n = (int)nb;
+  constexpr bool cplx = traits<T>::is_complex;
   if constexpr (sizeof(typename traits<T>::real) == 4) {
-    if (m <= 512) return launch_panel<T, 2>(P, ld, rows, n, tau, Tout, info, st);
-    if (m <= 1024) return launch_panel<T, 4>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= (cplx ? 256 : 128)) return launch_panel<T, 2>(P, ld, rows, n, tau, Tout, info, st);
+    if (m > 256 && m <= 384) return launch_panel<T, 3>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 512) return launch_panel<T, 4>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 768) return launch_panel<T, cplx ? 3 : 6>(P, ld, rows, n, tau, Tout, info, st);
+    if (m <= 1024) return launch_panel<T, cplx ? 4 : 8>(P, ld, rows, n, tau, Tout, info, st);
+    if (cplx && m <= 1280) return launch_panel<T, cplx ? 5 : 6>(P, ld, rows, n, tau, Tout, info, st);
     if (m <= 1536) return launch_panel<T, 6>(P, ld, rows, n, tau, Tout, info, st);
+    if (cplx && m <= 1792) return launch_panel<T, cplx ? 7 : 8>(P, ld, rows, n, tau, Tout, info, st);
   } else {
     if (m <= 512) return launch_panel<T, 1>(P, ld, rows, n, tau, Tout, info, st);
     if (m <= 1024) return launch_panel<T, 2>(P, ld, rows, n, tau, Tout, info, st);
