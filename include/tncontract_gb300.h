@@ -438,7 +438,7 @@ int tnc_sweep_compress(int dtype, int n_sites, int64_t d,
 /* <bra|ket> of two states (ladder_contract, onedim_core.py:1587-1607): site i
  * (d[i], bonds[i], bonds[i+1]), bonds[0] = 1; conj_bra conjugates the bra.
  * scaled: the norms of the sites and of the environment are taken out as powers
- * of two.  out (HOST): the first element of the last environment (its real and
+ * of two; they may lie anywhere in the type's range.  out (HOST): the first element of the last environment (its real and
  * imaginary part), and the natural log of what was taken out.  d, the bonds and
  * the pointer lists are HOST arrays. */
 int tnc_mps_overlap_workspace_size(int dtype, int n_sites, const int64_t *d,

@@ -417,6 +417,29 @@ __global__ void sumsq_kernel(int64_t n, const T* __restrict__ x, double* out) {
 
 __global__ void sqrt_inplace(double* v) { v[0] = sqrt(v[0]); }
 
+__device__ __forceinline__ double max_part(float x) { return fabsf(x); }
+__device__ __forceinline__ double max_part(double x) { return fabs(x); }
+template <typename R> __device__ __forceinline__ double max_part(cplx<R> x) {
+  const double a = max_part(x.re), b = max_part(x.im);
+  return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+}
+// the largest |real or imaginary part|, as the integer of its bits (out zeroed; a NaN
+// ranks above every number)
+template <typename T>
+__global__ void max_part_kernel(int64_t n, const T* __restrict__ x, double* out) {
+  long long m = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const long long b = __double_as_longlong(max_part(x[i]));
+    m = b > m ? b : m;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long b = __shfl_xor_sync(0xffffffffu, m, o);
+    m = b > m ? b : m;
+  }
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<long long*>(out), m);
+}
+
 template <typename T>
 __global__ void dot_kernel(int64_t n, const T* __restrict__ x, const T* __restrict__ y, int conj_x, double* out) {
   __shared__ double red[32];
@@ -591,6 +614,13 @@ __global__ void diag_matrix_kernel(int64_t n, const typename traits<T>::real* __
     int64_t i = e / n, j = e - i * n;
     out[e] = (i == j) ? from_real<T>(d[i]) : zero_<T>();
   }
+}
+
+int max_part_launch(int dtype, int64_t n, const void* x, double* out, cudaStream_t st) {
+  if (cudaMemsetAsync(out, 0, sizeof(double), st) != cudaSuccess) return TNC_ERR_CUDA;
+  if (n <= 0) return TNC_OK;
+  TNC_DISPATCH(dtype, T, max_part_kernel<T><<<grid1d(n, 256, 152 * 4), 256, 0, st>>>(n, (const T*)x, out));
+  return launch_status();
 }
 
 }  // namespace tnc

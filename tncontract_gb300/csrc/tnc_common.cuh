@@ -178,6 +178,8 @@ inline unsigned grid1d(int64_t n, int threads, int64_t cap = 152 * 32) {
 }
 
 // -------- internal (C++) entry points shared between translation units
+// out[0] (device) = the largest |real or imaginary part| of n elements (NaN if one is).
+int max_part_launch(int dtype, int64_t n, const void* x, double* out, cudaStream_t st);
 template <typename T>
 int gemm_launch(int opA, int opB, int64_t m, int64_t n, int64_t k, T alpha,
                 const T* A, int64_t lda, int64_t sA, const T* B, int64_t ldb,

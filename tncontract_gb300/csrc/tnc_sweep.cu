@@ -42,6 +42,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <new>
 #include <vector>
 
@@ -584,7 +585,9 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
 // rows (ra, p, lb), so that the next product contracts p and lb at once),
 // E' = X b.  With scaling, the sites' norms are read once at the start and the
 // environment's after every site, and powers of two are taken out in the
-// products' factors.
+// products' factors; a factor near the ends of the type's range in two steps, half
+// of it on the product's other operand, so that the products before the factor stay
+// in range too (a sweep in FP64 leaves up to e^600 in its first site).
 struct OverlapPlan {
   size_t norms, x, e[2], tc, total, tcb;
 };
@@ -625,10 +628,11 @@ int overlap_impl(int dt, int n, const int64_t* d, const void* const* bra, const 
   if (wb < P.total) return TNC_ERR_WORKSPACE;
   char* w = (char*)work;
   double* norms = (double*)(w + P.norms);
-  const int lim = fp32_class(dt) ? 100 : 1000;  // exponents that a factor may have in the type
+  const int far = fp32_class(dt) ? 40 : 400;  // exponents beyond which a factor goes in two steps
   const double ln2 = 0.69314718055994530942;
   double logs = 0.0;
   std::vector<double> h((size_t)(2 * n));
+  std::vector<int> ex((size_t)(2 * n), 0);  // of the sites' norms
   if (scaled) {
     for (int i = 0; i < n; ++i) {
       if (int rc = tnc_nrm2(dt, d[i] * ba[i] * ba[i + 1], bra[i], norms + i, st)) return rc;
@@ -637,14 +641,28 @@ int overlap_impl(int dt, int n, const int64_t* d, const void* const* bra, const 
     if (cudaMemcpyAsync(h.data(), norms, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
       return TNC_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return TNC_ERR_CUDA;
+    for (int i = 0; i < 2 * n; ++i) {
+      double& x = h[(size_t)i];
+      if (!(x > 1e-150 && x < 1e150)) {  // the sum of squares left the range of a double: by the largest part
+        const int q = i < n ? i : i - n;
+        const int64_t* bonds = i < n ? ba : bb;
+        if (int rc = max_part_launch(dt, d[q] * bonds[q] * bonds[q + 1], i < n ? bra[q] : ket[q], norms + 2 * n, st))
+          return rc;
+        if (cudaMemcpyAsync(&x, norms + 2 * n, sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+          return TNC_ERR_CUDA;
+        if (cudaStreamSynchronize(st) != cudaSuccess) return TNC_ERR_CUDA;
+      }
+      if (x > 0 && std::isfinite(x)) ex[(size_t)i] = std::ilogb(x);
+    }
   }
-  // the factor 2^-e for a norm, its logarithm kept
-  auto take_out = [&](double x, int extra) {
-    if (!scaled) return 1.0;
-    int e = extra + (x > 0 && std::isfinite(x) ? std::ilogb(x) : 0);
-    e = e > lim ? lim : e < -lim ? -lim : e;
+  // 2^-e, its logarithm kept: `pre` on the operand beside the site, `post` on the product
+  struct Factor {
+    double pre, post;
+  };
+  auto take_out = [&](int e) {
     logs += e * ln2;
-    return std::ldexp(1.0, -e);
+    const int p = e > far || e < -far ? e / 2 : 0;
+    return Factor{std::ldexp(1.0, -p), std::ldexp(1.0, p - e)};
   };
   const int opa = conj_bra ? TNC_OP_C : TNC_OP_T;
   T* X = (T*)(w + P.x);
@@ -653,23 +671,28 @@ int overlap_impl(int dt, int n, const int64_t* d, const void* const* bra, const 
     const int64_t la = ba[i], ra = ba[i + 1], lb = bb[i], rb = bb[i + 1];
     T* E = (T*)(w + P.e[cur]);
     T* E2 = (T*)(w + P.e[cur ^ 1]);
-    const double fa = take_out(h[(size_t)i], 0), fb = take_out(h[(size_t)(n + i)], left);
+    const Factor fa = take_out(ex[(size_t)i]), fb = take_out(ex[(size_t)(n + i)] + left);
     if (i == 0) {  // (d x ra)^H (d x rb); the bra's factor before the product, in which the two norms could leave the
                    // type's range
       const void* a = bra[i];
-      if (fa != 1.0) {
-        const double f[2] = {fa, 0.0};
-        if (int rc = tnc_scale(dt, d[i] * ra, f, bra[i], X, 0, st)) return rc;
+      for (const double f : {fa.pre, fa.post, fb.pre}) {
+        if (f == 1.0) continue;
+        const double s[2] = {f, 0.0};
+        if (int rc = tnc_scale(dt, d[i] * ra, s, a, X, 0, st)) return rc;
         a = X;
       }
-      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, rb, d[i], fb, a, ra, 0, ket[i], rb, 0, E2, rb, 0, 1, w + P.tc, P.tcb,
-                            st))
+      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, rb, d[i], fb.post, a, ra, 0, ket[i], rb, 0, E2, rb, 0, 1, w + P.tc,
+                            P.tcb, st))
         return rc;
     } else {
-      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, lb, la, fa, bra[i], ra, la * ra, E, lb, 0, X, d[i] * lb, lb, d[i],
+      if (fa.pre != 1.0)
+        if (int rc = scale(dt, la * lb, fa.pre, E, st)) return rc;
+      if (int rc = gemm_any(dt, opa, TNC_OP_N, ra, lb, la, fa.post, bra[i], ra, la * ra, E, lb, 0, X, d[i] * lb, lb, d[i],
                             w + P.tc, P.tcb, st))
         return rc;
-      if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_N, ra, rb, d[i] * lb, fb, X, d[i] * lb, 0, ket[i], rb, 0, E2, rb, 0, 1,
+      if (fb.pre != 1.0)
+        if (int rc = scale(dt, d[i] * ra * lb, fb.pre, X, st)) return rc;
+      if (int rc = gemm_any(dt, TNC_OP_N, TNC_OP_N, ra, rb, d[i] * lb, fb.post, X, d[i] * lb, 0, ket[i], rb, 0, E2, rb, 0, 1,
                             w + P.tc, P.tcb, st))
         return rc;
     }
