@@ -45,7 +45,8 @@ enum {
   TNC_ERR_CUDA = 4,          /* a CUDA launch or API call failed           */
   TNC_ERR_WORKSPACE = 5,     /* workspace smaller than *_workspace_size    */
   TNC_ERR_TIMEOUT = 6,       /* a bounded device-side wait gave up         */
-  TNC_ERR_TOO_LARGE = 7      /* problem exceeds tnc_svd_noalloc's scratch  */
+  TNC_ERR_TOO_LARGE = 7,     /* problem exceeds tnc_svd_noalloc's scratch  */
+  TNC_ERR_ZERO_STATE = 8     /* a state of norm zero cannot be compressed  */
 };
 
 /* matrix operation applied to a row-major operand */
@@ -406,7 +407,8 @@ int tnc_gather_rows(int dtype, const void *src, int64_t L, const int64_t *order,
  * the last, checking one, n rows of length L, complex; a third of that
  * real; for TNC_CORE_DF the FP32 operations of the double-float Jacobi:
  * 44 n^2 L per rotating sweep and 24 n^2 L for the checking one, complex;
- * 15 and 6 real).  Returns TNC_ERR_ARG for a zero state. */
+ * 15 and 6 real).  Returns TNC_ERR_ARG for a zero state, TNC_ERR_NONFINITE for
+ * one whose norm is not finite. */
 enum { TNC_CORE_STORAGE = 0, TNC_CORE_FP64 = 1, TNC_CORE_DF = 2 };
 int tnc_sweep_workspace_size(int dtype, int n_sites, int64_t d,
                              const int64_t *mps_bonds, const int64_t *mpo_bonds,
@@ -427,7 +429,8 @@ int tnc_sweep_apply_compress(int dtype, int n_sites, int64_t d,
  * aligned).  Each bond's largest singular value is divided out of the returned
  * sites; *log_norm: in, the log of the input's norm factor, out, that of the
  * output.  out_discarded[i]: the discarded squared values over the squared largest
- * one, bond between sites i and i+1. */
+ * one, bond between sites i and i+1.  Returns TNC_ERR_ZERO_STATE for a zero state,
+ * TNC_ERR_NONFINITE for one whose norm is not finite. */
 int tnc_sweep_compress(int dtype, int n_sites, int64_t d,
                        const void *const *sites, const int64_t *mps_bonds,
                        int64_t chi, double threshold, void *work,

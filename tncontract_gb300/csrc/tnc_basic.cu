@@ -643,6 +643,7 @@ const char* tnc_status_string(int s) {
     case TNC_ERR_WORKSPACE: return "workspace too small";
     case TNC_ERR_TIMEOUT: return "device-side wait timed out";
     case TNC_ERR_TOO_LARGE: return "problem needs more than the fixed scratch of tnc_svd_noalloc (16 MiB)";
+    case TNC_ERR_ZERO_STATE: return "zero state";
     default: return "unknown status";
   }
 }

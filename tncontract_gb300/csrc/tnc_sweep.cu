@@ -368,6 +368,7 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     if (int rc = host_norm(dt, k * r, B.rbuf, B.dnorm, &rn, st)) return rc;
     if (int stq = device_status(B.info, st)) return stq;
     prof.add(0, qr_flops(rows, r, cplx));
+    if (!std::isfinite(rn)) return TNC_ERR_NONFINITE;
     rn = pow2_of(rn);
     if (rn > 0) lnorm += std::log(rn);
     const int64_t r2 = sr[i + 1];  // sl[i + 1] == r
@@ -384,7 +385,8 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     const int i = n_sites - 1;
     double last = 0.0;
     if (int rc = host_norm(dt, d * sl[i] * sr[i], B.slot[i], B.dnorm, &last, st)) return rc;
-    if (!(last > 0.0)) return TNC_ERR_ARG;  // zero state
+    if (!std::isfinite(last)) return TNC_ERR_NONFINITE;
+    if (!(last > 0.0)) return TNC_ERR_ZERO_STATE;
     if (int rc = scale(dt, d * sl[i] * sr[i], 1.0 / last, B.slot[i], st)) return rc;
     lnorm += std::log(last);
   }
@@ -510,7 +512,8 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
     // storage type's rounding-noise floor
     const int64_t k = rank_rule<double>(sd, chi, threshold, eps);
     const double smax = sd.empty() ? 0.0 : sd[0];
-    if (!(smax > 0.0) || k < 1) return TNC_ERR_ARG;  // zero state
+    if (!(smax > 0.0)) return TNC_ERR_ZERO_STATE;
+    if (k < 1) return TNC_ERR_ARG;  // the threshold keeps nothing
     if (out_discarded) {
       double tot = 0.0, dis = 0.0;
       for (int64_t j = 0; j < kmin; ++j) {
@@ -741,11 +744,12 @@ extern "C" int tnc_sweep_apply_compress(int dtype, int n_sites, int64_t d, const
       !log_norm || !folded || chi < 0)
     return TNC_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
+  int rc = TNC_ERR_ARG;
   TNC_DISPATCH(dtype, T,
-               return sweep_impl<T>(dtype, n_sites, d, sites, mps_bonds, mpo, mpo_bonds, chi, threshold, block_rows,
-                                    core, core_tol, work, work_bytes, out_bonds, out_offsets, out_discarded, log_norm,
-                                    folded, profile, st));
-  return TNC_ERR_ARG;
+               rc = sweep_impl<T>(dtype, n_sites, d, sites, mps_bonds, mpo, mpo_bonds, chi, threshold, block_rows, core,
+                                  core_tol, work, work_bytes, out_bonds, out_offsets, out_discarded, log_norm, folded,
+                                  profile, st));
+  return rc == TNC_ERR_ZERO_STATE ? TNC_ERR_ARG : rc;
 }
 
 extern "C" int tnc_sweep_compress(int dtype, int n_sites, int64_t d, const void* const* sites, const int64_t* mps_bonds,

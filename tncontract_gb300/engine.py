@@ -541,8 +541,10 @@ def _compress_native(P, chi, threshold, stats, log_norm_in):
     log_norm = C.c_double(float(log_norm_in))
     st = L.lib().tnc_sweep_compress(code, N, d, ptrs, bonds, int(chi or 0), float(threshold), _ops._p(ws), sz.value, out_b,
                                     out_o, out_d, C.byref(log_norm), _ops._stream())
-    if st == L.ERR_ARG:
+    if st == L.ERR_ZERO_STATE:
         raise ValueError("zero state in the sweep")
+    if st == L.ERR_ARG:
+        raise ValueError("the sweep refused its arguments (or host memory ran out)")
     if st == L.ERR_NONFINITE:
         raise ValueError("array must not contain infs or NaNs")
     if st == L.ERR_NOT_CONVERGED:
