@@ -441,9 +441,10 @@ extern "C" int tnc_svd(int dtype, int64_t m, int64_t n, const void* A, int64_t l
 // (cudaGetSymbolAddress) on the first call made on a device, and looked up
 // again when that device's context is no longer the one the address was
 // taken in (after cudaDeviceReset, or a primary context released and
-// re-created, the library image is loaded anew at another address); make the
-// first call on a device, and the first after such a reset, before any
-// stream capture.
+// re-created, the library image is loaded anew at another address).  Contexts
+// are told apart by their id: a re-created primary context keeps its handle.
+// Make the first call on a device, and the first after such a reset, before
+// any stream capture.
 // ---------------------------------------------------------------------------
 #include <cuda.h>
 
@@ -454,25 +455,27 @@ namespace tnc {
 static constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_svd_scratch[kNoAllocScratchBytes];
 
-typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
+typedef CUresult (*CtxGetIdFn)(CUcontext, unsigned long long*);
 
-// cuCtxGetCurrent through the runtime's driver entry point (no link-time
-// dependency on the driver library)
-static CtxGetCurrentFn ctx_get_current() {
+// Id of the calling thread's current context, never used twice in a process; 0
+// when there is none or it was destroyed.  cuCtxGetId through the runtime's
+// driver entry point (no link-time dependency on the driver library).
+static unsigned long long context_id() {
   static std::once_flag once;
-  static CtxGetCurrentFn fn = nullptr;
+  static CtxGetIdFn fn = nullptr;
   std::call_once(once, [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
         q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<CtxGetCurrentFn>(p);
+      fn = reinterpret_cast<CtxGetIdFn>(p);
   });
-  return fn;
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 struct NoallocSlot {
-  CUcontext ctx;  // the context the address was looked up in
+  unsigned long long ctx;  // the id of the context the address was looked up in
   void* ptr;
 };
 static std::mutex g_noalloc_mu;
@@ -482,15 +485,13 @@ static int noalloc_scratch(void** out) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return TNC_ERR_CUDA;
   if (dev < 0 || dev >= 128) return TNC_ERR_ARG;
-  CtxGetCurrentFn get = ctx_get_current();
-  if (!get) return TNC_ERR_CUDA;
-  CUcontext ctx = nullptr;
-  if (get(&ctx) != CUDA_SUCCESS) return TNC_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_noalloc_mu);
-  if (ctx == nullptr || g_noalloc[dev].ptr == nullptr || g_noalloc[dev].ctx != ctx) {
+  unsigned long long ctx = context_id();
+  if (ctx == 0 || g_noalloc[dev].ptr == nullptr || g_noalloc[dev].ctx != ctx) {
     void* p = nullptr;  // the lookup also makes the device's primary context current
     if (cudaGetSymbolAddress(&p, g_noalloc_svd_scratch) != cudaSuccess || p == nullptr) return TNC_ERR_CUDA;
-    if (get(&ctx) != CUDA_SUCCESS || ctx == nullptr) return TNC_ERR_CUDA;
+    ctx = context_id();
+    if (ctx == 0) return TNC_ERR_CUDA;
     g_noalloc[dev] = NoallocSlot{ctx, p};
   }
   *out = g_noalloc[dev].ptr;
