@@ -75,3 +75,17 @@ def test_two_rows(gpu, dt):
     assert worst_r <= 2 and worst_q <= (16 if cplx else 8), (worst_r, worst_q)
     # unbiased: the mean of 400 errors of at most 2 eps, uniform or better, stays within 4 deviations
     assert abs(np.mean(mean)) <= 4 * 2 / np.sqrt(3) / np.sqrt(400), np.mean(mean)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_real_norm_is_rounded_once_a_step(gpu, dt):
+    """R of one real column of two entries.  Bound, in u = eps / 2: two squares and their sum, 2 u, halved by the root,
+    which is rounded correctly: 2 u of the result, that is u of 2^k where the result lies in [2^k, 2^(k+1))."""
+    rng = np.random.default_rng(12)
+    eps = np.finfo(dt).eps
+    for _ in range(1500):
+        a = (rng.standard_normal(2) * np.array([1.0, 2.0 ** rng.integers(-3, 4)])).astype(dt)
+        _, R = _qr(a.reshape(2, 1))
+        x = a.astype(np.float64 if dt == np.float32 else np.longdouble)
+        n = np.sqrt((x * x).sum())
+        assert abs(abs(x.dtype.type(R[0, 0])) - n) <= eps * n * 1.0001, a
