@@ -1,0 +1,51 @@
+"""Clustered spectra in the refined FP64 SVD (24 to 512 rows): what its steps leave to the FP64 Jacobi starts from a
+unitary J, and pairs that already meet the tolerance are not left to it."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(n, s, dt, seed):
+    rng = np.random.default_rng(seed)
+
+    def unitary():
+        a = rng.standard_normal((n, n))
+        if np.issubdtype(dt, np.complexfloating):
+            a = a + 1j * rng.standard_normal((n, n))
+        return np.linalg.qr(a)[0]
+    return ((unitary() * s) @ unitary().conj().T).astype(dt)
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("n,size,gap", [(40, 5, 1e-4), (64, 16, 1e-6), (97, 30, 1e-5), (130, 130, 1e-6), (64, 64, 1e-12)])
+def test_cluster(gpu, dt, n, size, gap):
+    """`size` values within `gap` of one another beside generic ones.  Bounds: 8 n eps, as for other spectra."""
+    from tncontract_gb300 import _ops
+    s = np.sort(np.concatenate([1.0 + gap * np.linspace(0, 1, size), np.linspace(0.2, 0.9, n - size)]))[::-1]
+    A = _matrix(n, s, dt, n)
+    U, S, V = (t.cpu().numpy() for t in _ops.svd(torch.from_numpy(A).cuda()))
+    tol = 8 * n * np.finfo(dt).eps
+    assert np.max(np.abs(S - np.linalg.svd(A, compute_uv=False))) <= tol
+    assert np.max(np.abs(U.conj().T @ U - np.eye(n))) <= tol
+    assert np.max(np.abs(V @ V.conj().T - np.eye(n))) <= tol
+    assert np.linalg.norm((U * S) @ V - A) <= tol * np.linalg.norm(A)
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("tol", [1e-8, 3e-8, 1e-7])
+def test_equal_pair_below_the_tolerance(gpu, dt, tol):
+    """Two equal values whose rows meet a caller's tolerance while others do not: their angle is large but nothing has to
+    be rotated, so the steps finish the work.  info[1] counts the sweeps of the Jacobi that ended it: the
+    single-precision one's (five or more from a random matrix), not the FP64 one's (one or two after the steps)."""
+    from tncontract_gb300 import _ops
+    n = 48
+    s = np.linspace(0.1, 2.0, n)[::-1].copy()
+    s[1] = s[0]
+    for seed in range(12):
+        infos = []
+        A = _matrix(n, s, dt, 100 + seed)
+        _ops.svd(torch.from_numpy(A).cuda(), tol=tol, info_out=infos)
+        assert infos[0].cpu().tolist()[0] == 0
+        assert infos[0].cpu().tolist()[1] >= 4, (seed, infos[0].cpu().tolist())

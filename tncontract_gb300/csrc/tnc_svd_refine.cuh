@@ -209,6 +209,12 @@ __device__ __forceinline__ float refine_skip(int step, double tol) {
   return HASJ && step == 0 ? 1e-9f : 0.5f * (float)tol;
 }
 
+// Whether a pair is above the tolerance (scaled squared norms and product).
+template <typename T>
+__device__ __forceinline__ bool refine_above(T g, double a, double b, double noise2, double tol2) {
+  return a > noise2 && b > noise2 && abs2_(g) > tol2 * (a * b);
+}
+
 // Counts of the pairs above the tolerances, and for every row its pairs with a
 // large angle (and its partner in the last).  A thread takes a pair i < k.  Without J, delta is nothing and d is
 // not read.  Pairs of two rows from nkeep on are left alone.
@@ -232,7 +238,7 @@ __global__ void refine_test_kernel(int64_t n, const T* __restrict__ GF, const ty
     const T g = GF[i * n + k] * sc, dl = HASJ ? GF[k * n + i] : zero_<T>();
     const double ai = a[i] * sc, ak = a[k] * sc, di = HASJ ? d[i] : 0.0, dk = HASJ ? d[k] : 0.0;
     if (HASJ) unit += abs2_(dl) > utol2;
-    if (ai > noise2 && ak > noise2 && abs2_(g) > tol2 * (ai * ak)) {
+    if (refine_above<T>(g, ai, ak, noise2, tol2)) {
       ++rot;
       if (refine_pair<T>(g, dl, ai - ai * di, ak - ak * dk, noise2, skip).large) {
         // two in a row: the simultaneous rotations do not hold for them
@@ -250,8 +256,8 @@ __global__ void refine_test_kernel(int64_t n, const T* __restrict__ GF, const ty
 }
 
 // F^T in single precision, Ft[k][i] = F(i, k).  A pair takes its first-order
-// rotation, or, when its angle is large and neither row has another such pair,
-// the full one (with its part of the diagonal; without J, refine_pairs_kernel does
+// rotation, or, when its angle is large, it is above the tolerance and neither row
+// has another such pair, the full one (with its part of the diagonal; without J, refine_pairs_kernel does
 // it in FP64).  Late steps take small angles only, so that what they leave of J's
 // defect is below rounding.
 template <typename T, bool HASJ>
@@ -282,7 +288,9 @@ __global__ void refine_f_kernel(int64_t n, const T* __restrict__ GF, const typen
       S f = zero_<S>();
       if (rotate && (i < nkeep || k < nkeep)) {
         RefinePair<S> r = refine_pair<T>(g, dl, up ? ai : ak, up ? ak : ai, noise2, skip);
-        if (!HASJ && r.large && li == 1 && rows_large[k] == 1) {
+        if ((r.large || (HASJ && r.t >= top)) && !refine_above<T>(g, raw, rk, noise2, tol * tol)) {
+          r.f = zero_<S>();  // two nearly equal norms that meet the tolerance: the test has not counted the pair
+        } else if (!HASJ && r.large && li == 1 && rows_large[k] == 1) {
           r.f = zero_<S>();
           fmax2 = 1.f;  // another look
         } else if (HASJ && r.large && li == 1 && rows_large[k] == 1 && r.t < top) {
