@@ -49,3 +49,25 @@ def test_equal_pair_below_the_tolerance(gpu, dt, tol):
         _ops.svd(torch.from_numpy(A).cuda(), tol=tol, info_out=infos)
         assert infos[0].cpu().tolist()[0] == 0
         assert infos[0].cpu().tolist()[1] >= 4, (seed, infos[0].cpu().tolist())
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("tol", [1e-10, 1e-8, 3e-8, 1e-7])
+@pytest.mark.parametrize("n", [24, 48, 100])
+def test_loose_tolerance(gpu, dt, tol, n):
+    """A caller's loose tolerance is one on the rows' orthogonality: the accumulated factor stays unitary to rounding, and
+    the singular values are second order in the tolerance (8 n tol^2 beside the usual 8 n eps)."""
+    from tncontract_gb300 import _ops
+    s = np.linspace(0.1, 2.0, n)[::-1].copy()
+    s[1] = s[0]
+    for shape in ("square", "tall"):
+        A = _matrix(n, s, dt, n)
+        if shape == "tall":
+            A = np.linalg.qr(_matrix(2 * n, np.ones(2 * n), dt, 1)[:, :n])[0] @ A
+        U, S, V = (t.cpu().numpy() for t in _ops.svd(torch.from_numpy(A).cuda(), tol=tol))
+        assert np.max(np.abs(S - s)) <= 8 * n * (np.finfo(dt).eps + tol * tol)
+        # the accumulated side: VH of a tall or square matrix is normalised rows or J, U the other
+        both = [np.max(np.abs(U.conj().T @ U - np.eye(n))), np.max(np.abs(V @ V.conj().T - np.eye(n)))]
+        assert min(both) <= 8 * n * np.finfo(dt).eps, both
+        assert max(both) <= 2 * tol + 8 * n * np.finfo(dt).eps, both
+        assert np.linalg.norm((U * S) @ V - A) <= 16 * n * np.finfo(dt).eps * np.linalg.norm(A)

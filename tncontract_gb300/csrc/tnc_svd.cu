@@ -264,11 +264,11 @@ static int svd_refine(int64_t nr, const T* R, T* J, T* Wb, T* GF, char* scratch,
   typedef TileS<T> G;
   const int64_t rows = (nr + G::BM - 1) / G::BM, cols = (nr + G::BN - 1) / G::BN;
   const unsigned half = refine_half_tiles(nr);
-  const double eps = traits<T>::eps;
+  const double eps = traits<T>::eps, utol = fmin(tol, sqrt((double)nr) * eps);
   refine_product_kernel<T><<<(unsigned)(rows * cols), G::THR, 0, st>>>(nr, J, R, Wb, rs, 0);
   for (int s = 0; s <= kRefineSteps; ++s) {
     refine_gram_kernel<T><<<dim3(half, 2), G::THR, 0, st>>>(nr, Wb, J, GF, a, d, rs, s, js.rows_large);
-    refine_test_kernel<T, true><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, eps, nr, rs, s, -1.f, js.rows_large,
+    refine_test_kernel<T, true><<<g, 256, 0, st>>>(nr, GF, a, d, frob2, tol, utol, eps, nr, rs, s, -1.f, js.rows_large,
                                                      nullptr);
     if (s == kRefineSteps) break;
     refine_f_kernel<T, true><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, GF, a, d, frob2, tol, eps, nr, rs, s, -1.f,

@@ -216,15 +216,17 @@ __device__ __forceinline__ bool refine_above(T g, double a, double b, double noi
 }
 
 // Counts of the pairs above the tolerances, and for every row its pairs with a
-// large angle (and its partner in the last).  A thread takes a pair i < k.  Without J, delta is nothing and d is
-// not read.  Pairs of two rows from nkeep on are left alone.
+// large angle (and its partner in the last).  A thread takes a pair i < k.  J is held to
+// utol, rounding, whatever the caller's tolerance: U and VH are as unitary as J, and
+// the singular values are second order in tol only if it is.  Without J, delta is
+// nothing and d is not read.  Pairs of two rows from nkeep on are left alone.
 template <typename T, bool HASJ>
 __global__ void refine_test_kernel(int64_t n, const T* __restrict__ GF, const typename traits<T>::real* __restrict__ a,
                                    const typename traits<T>::real* __restrict__ d, const double* frob2, double tol,
-                                   double eps, int64_t nkeep, RefineState* st, int step, float accept,
+                                   double utol, double eps, int64_t nkeep, RefineState* st, int step, float accept,
                                    unsigned* rows_large, unsigned* partner) {
   if (refine_done(st, step, accept) || (!HASJ && refine_hard(st, step))) return;
-  const double sc = refine_scale2(frob2), noise2 = eps * eps * frob2[0] * sc, tol2 = tol * tol, utol2 = 16.0 * tol2;
+  const double sc = refine_scale2(frob2), noise2 = eps * eps * frob2[0] * sc, tol2 = tol * tol, utol2 = 16.0 * utol * utol;
   const float skip = refine_skip<HASJ>(step, tol);
   unsigned rot = 0, unit = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * n; e += (int64_t)gridDim.x * blockDim.x) {

@@ -1184,7 +1184,7 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
     if (cudaMemsetAsync(rs, 0, (kDfSteps + 1) * sizeof(RefineState), st) != cudaSuccess) return TNC_ERR_CUDA;
     for (int s = 0; s <= kDfSteps; ++s) {
       df_gram_kernel<Tdf><<<(unsigned)(tiles * (tiles + 1) / 2), 256, 0, st>>>(nr, L, W, G, D, rs, s, accept, large);
-      refine_test_kernel<Tout, false><<<g, 256, 0, st>>>(nr, G, D, nullptr, f2, tol, eps, keep, rs, s, accept, large,
+      refine_test_kernel<Tout, false><<<g, 256, 0, st>>>(nr, G, D, nullptr, f2, tol, 0.0, eps, keep, rs, s, accept, large,
                                                          large + nr);
       if (s == kDfSteps) break;
       refine_f_kernel<Tout, false><<<grid1d(nr * 32, 128), 128, 0, st>>>(nr, G, D, nullptr, f2, tol, eps, keep, rs, s,
