@@ -71,3 +71,26 @@ def test_loose_tolerance(gpu, dt, tol, n):
         assert min(both) <= 8 * n * np.finfo(dt).eps, both
         assert max(both) <= 2 * tol + 8 * n * np.finfo(dt).eps, both
         assert np.linalg.norm((U * S) @ V - A) <= 16 * n * np.finfo(dt).eps * np.linalg.norm(A)
+
+
+@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("tol", [1e-8, 1e-7])
+@pytest.mark.parametrize("below", [0.3, 0.9])
+def test_rule_of_the_steps(gpu, dt, tol, below):
+    """A triangular matrix (its QR changes nothing) with one pair of rows of equal norm below the tolerance and one of unequal
+    norms above it, all too nearly orthogonal for the single-precision Jacobi to rotate: one step ends the work, and info[1]
+    is that Jacobi's one sweep.  The FP64 Jacobi would have counted two, one that rotates and one that finds nothing."""
+    from tncontract_gb300 import _ops
+    n = 40
+    phase = np.exp(0.7j) if np.issubdtype(dt, np.complexfloating) else 1.0
+    R = np.diag(np.linspace(2.0, 0.5, n)).astype(dt)
+    g = below * tol * R[0, 0].real ** 2
+    R[0, 1] = phase * g / R[0, 0].real
+    R[1, 1] = np.sqrt(abs(R[0, 0]) ** 2 + abs(R[0, 1]) ** 2)
+    R[2, 3] = phase * 3 * tol * abs(R[2, 2])
+    infos = []
+    U, S, V = (t.cpu().numpy() for t in _ops.svd(torch.from_numpy(np.ascontiguousarray(R.conj().T)).cuda(), tol=tol,
+                                                 info_out=infos))
+    assert infos[0].cpu().tolist()[:3] == [0, 1, 0]
+    assert np.max(np.abs(S - np.linalg.svd(R, compute_uv=False))) <= 8 * n * np.finfo(dt).eps + 2 * below * tol
+    assert np.linalg.norm((U * S) @ V - R.conj().T) <= 16 * n * np.finfo(dt).eps * np.linalg.norm(R)
