@@ -74,20 +74,22 @@ def test_loose_tolerance(gpu, dt, tol, n):
 
 
 @pytest.mark.parametrize("dt", [np.float64, np.complex128])
-@pytest.mark.parametrize("tol", [1e-8, 1e-7])
-@pytest.mark.parametrize("below", [0.3, 0.9])
-def test_rule_of_the_steps(gpu, dt, tol, below):
-    """A triangular matrix (its QR changes nothing) with one pair of rows of equal norm below the tolerance and one of unequal
-    norms above it, all too nearly orthogonal for the single-precision Jacobi to rotate: one step ends the work, and info[1]
-    is that Jacobi's one sweep.  The FP64 Jacobi would have counted two, one that rotates and one that finds nothing."""
+@pytest.mark.parametrize("tol", [1.5e-9, 3e-9])
+def test_rule_of_the_steps(gpu, dt, tol):
+    """A triangular matrix (its QR changes nothing) with one pair of rows of equal norm just below the tolerance, whose angle
+    is large, and a dozen rows of nearly equal norms above it, whose angles (up to 8.5e-4) take a second step; all too
+    nearly orthogonal for the single-precision Jacobi to rotate.  The steps end the work, and info[1] is that Jacobi's one
+    sweep; the FP64 Jacobi would have counted two, one that rotates and one that finds nothing."""
     from tncontract_gb300 import _ops
-    n = 40
+    n, m, below = 40, 12, 0.9
     phase = np.exp(0.7j) if np.issubdtype(dt, np.complexfloating) else 1.0
     R = np.diag(np.linspace(2.0, 0.5, n)).astype(dt)
-    g = below * tol * R[0, 0].real ** 2
-    R[0, 1] = phase * g / R[0, 0].real
+    R[0, 1] = phase * below * tol * abs(R[0, 0])
     R[1, 1] = np.sqrt(abs(R[0, 0]) ** 2 + abs(R[0, 1]) ** 2)
-    R[2, 3] = phase * 3 * tol * abs(R[2, 2])
+    size, g, t = abs(R[2, 2]), 2.772e-6, 8.5e-4
+    for i in range(m):
+        R[2 + i, 2 + i] = size * np.sqrt(1 - g / t * i)
+        R[2 + i, 3 + i:2 + m] = phase * g * R[2 + i, 2 + i]
     infos = []
     U, S, V = (t.cpu().numpy() for t in _ops.svd(torch.from_numpy(np.ascontiguousarray(R.conj().T)).cuda(), tol=tol,
                                                  info_out=infos))
