@@ -81,4 +81,14 @@ template int jacobi32_rows<c64>(c64*, c64*, int64_t, int64_t, int, int, double, 
 
 TNC_DEFINE_SPIN_SETTER(spin_limit_set_j32)
 
+// Self-test: a warp waits for a row nobody gives.
+__global__ void j32_selftest_kernel(const unsigned* counter, SyncWords* sw, int* info) {
+  j32_wait_row(counter, 1u, sw);
+  if (threadIdx.x == 0) info[0] = ld_volatile(&sw->err);
+}
+int j32_wait_selftest(const unsigned* counter, SyncWords* sw, int* info, cudaStream_t st) {
+  j32_selftest_kernel<<<1, 32, 0, st>>>(counter, sw, info);
+  return launch_status(1);
+}
+
 }  // namespace tnc

@@ -19,8 +19,9 @@
 //
 // Lanes hold 16-byte pieces (V elements) of a row; rows are padded to 32 E
 // elements with zeros, which rotations keep, so the inner loops test nothing.
-// Every wait is bounded; a wait that gives up records TNC_ERR_TIMEOUT, and the
-// CTAs leave together at the sweep's grid barrier.
+// Every wait is bounded; a CTA whose wait gives up (or finds that another's has)
+// records TNC_ERR_TIMEOUT, goes through the sweep without waiting again and leaves
+// before its grid barrier, at which the others then leave too.
 #pragma once
 #include "tnc_persist.cuh"
 #include "tnc_rot.cuh"
@@ -173,6 +174,21 @@ __device__ __forceinline__ unsigned j32_acquire(const unsigned* p) {
   return v;
 }
 
+// A warp waits until a row's counter has reached `step`; false on error / timeout.
+__device__ __forceinline__ bool j32_wait_row(const unsigned* counter, unsigned step, SyncWords* sw) {
+  int good = 1;
+  if ((threadIdx.x & 31) == 0) {
+    const long long limit = spin_limit();
+    for (long long spins = 0; j32_acquire(counter) < step; ++spins) {
+      if (ld_volatile(&sw->err)) { good = 0; break; }
+      if (spins > limit) { atomicCAS(&sw->err, 0, TNC_ERR_TIMEOUT); good = 0; break; }
+    }
+  }
+  good = __shfl_sync(0xffffffffu, good, 0);
+  __syncwarp();
+  return good != 0;
+}
+
 struct J32Args {
   void *W, *J;  // rows of L elements each (J: ACC only)
   int nr, L, h, N, kb, max_sweeps, vec;  // N: half-blocks, padded to even; kb: half-blocks with kept rows
@@ -221,20 +237,7 @@ jacobi32_kernel(const J32Args p) {
     __syncwarp();
     if (lane == 0) j32_publish(p.ver + row, step);
   };
-  auto take_row = [&](int row, unsigned step) {
-    if (ok) {
-      int good = 1;
-      if (lane == 0) {
-        const long long limit = spin_limit();
-        for (long long spins = 0; j32_acquire(p.ver + row) < step; ++spins) {
-          if (ld_volatile(&p.sw->err)) { good = 0; break; }
-          if (spins > limit) { atomicCAS(&p.sw->err, 0, TNC_ERR_TIMEOUT); good = 0; break; }
-        }
-      }
-      ok = __shfl_sync(0xffffffffu, good, 0) != 0;
-      __syncwarp();
-    }
-  };
+  auto take_row = [&](int row, unsigned step) { ok = ok && j32_wait_row(p.ver + row, step, p.sw); };
   // rotate the pair (x, y); returns 0, 1 or 3 (above stol), the norms moved by *th
   auto rotate = [&](float a, float b, float2 (&xx)[P], float2 (&yy)[P], float& th) -> int {
     float re, im;
@@ -381,7 +384,7 @@ jacobi32_kernel(const J32Args p) {
     }
     if (lane == 0 && rot) atomicAdd(&p.counters[sweep], rot);
     if (lane == 0 && rotb) atomicAdd(&p.counters[kJ32MaxSweeps + sweep], rotb);
-    if (!grid_barrier(p.sw, gridDim.x)) return;
+    if (!__syncthreads_and(ok) || !grid_barrier(p.sw, gridDim.x)) return;
     last_rot = ld_volatile(&p.counters[sweep]);
     if (last_rot == 0) { converged = true; ++sweep; break; }
     if (p.staged && ld_volatile(&p.counters[kJ32MaxSweeps + sweep]) == 0) { staged = true; ++sweep; break; }

@@ -268,5 +268,7 @@ template <typename T>
 int jacobi32_rows(T* W, T* J, int64_t nr, int64_t L, int h, int max_sweeps, double tol, double stop_tol,
                   const double* frob2, float* Dn, unsigned* counters, SyncWords* sw, int* info, int64_t nkeep,
                   cudaStream_t st);
+// tnc_wait_selftest's kind 3: its wait for a row (counter and words zeroed by the caller).
+int j32_wait_selftest(const unsigned* counter, SyncWords* sw, int* info, cudaStream_t st);
 
 }  // namespace tnc
