@@ -64,8 +64,10 @@ const char *tnc_status_string(int status);
 int tnc_set_spin_limit(long long polls);
 /* One CTA waits on something nothing completes -- kind 0: a grid barrier
  * expecting two CTAs, 1: a step counter nobody publishes, 2: a flag nobody
- * sets, 3: a row that nobody gives (the single-precision Jacobi) -- until the wait limit runs out; info[0] (device int) receives the
- * error word, TNC_ERR_TIMEOUT when the bounded wait gave up as designed.
+ * sets, 3: a row that nobody gives (the single-precision Jacobi), 4: bytes that
+ * nobody sends (the QR's panels) -- until the wait limit runs out; info[0]
+ * (device int) receives the error word, TNC_ERR_TIMEOUT when the bounded wait
+ * gave up as designed.
  * work: 256 bytes of device memory.  A self-test of the failure path the
  * factorisations share; the reference's counterpart of that path is
  * tensor_svd's retry and re-raise (tncontract/tensor.py:914-929). */

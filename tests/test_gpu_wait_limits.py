@@ -1,4 +1,4 @@
-"""The bounded waits of the single-precision Jacobi (a row's step counter): one that nothing completes gives up after the
+"""The bounded waits of the single-precision Jacobi (a row's step counter) and of the QR's panels (a step's bytes): one that nothing completes gives up after the
 limit and reports it, its own kernel's limit being the one that counts; factorisations right after are correct."""
 import numpy as np
 import pytest
@@ -19,7 +19,7 @@ def _check():
         assert np.linalg.norm(Q @ R - A) <= 400 * np.finfo(dt).eps * np.linalg.norm(A)
 
 
-@pytest.mark.parametrize("kind", [3])
+@pytest.mark.parametrize("kind", [3, 4])
 def test_wait_runs_out(gpu, kind):
     from tncontract_gb300 import _lib as L
     from tncontract_gb300 import _ops

@@ -578,7 +578,8 @@ def set_spin_limit(polls=0):
 
 def wait_selftest(kind):
     """Run one CTA whose bounded wait nothing completes (0 grid barrier,
-    1 step counter, 2 flag, 3 a row of the single-precision Jacobi) and return its error word (``TNC_ERR_TIMEOUT``
+    1 step counter, 2 flag, 3 a row of the single-precision Jacobi, 4 bytes of
+    a QR panel's step) and return its error word (``TNC_ERR_TIMEOUT``
     when the wait gave up as designed)."""
     ws = workspace(256)
     info = torch.zeros(1, dtype=torch.int32, device=device())

@@ -270,5 +270,7 @@ int jacobi32_rows(T* W, T* J, int64_t nr, int64_t L, int h, int max_sweeps, doub
                   cudaStream_t st);
 // tnc_wait_selftest's kind 3: its wait for a row (counter and words zeroed by the caller).
 int j32_wait_selftest(const unsigned* counter, SyncWords* sw, int* info, cudaStream_t st);
+// Its kind 4: the QR panel's wait for a step's bytes (info zeroed by the caller).
+int qr_wait_selftest(int* info, cudaStream_t st);
 
 }  // namespace tnc

@@ -631,6 +631,23 @@ template int qr_qt<c128>(int64_t, int64_t, const c128*, int, bool, c128*, void*,
 
 TNC_DEFINE_SPIN_SETTER(spin_limit_set_qr)
 
+// Self-test: the panel's wait for bytes that never come.
+__global__ void qr_selftest_kernel(int* info) {
+  __shared__ __align__(8) unsigned long long bar;
+  if (threadIdx.x == 0) {
+    qr_bar_init(qr_smem(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    qr_bar_expect(qr_smem(&bar), 16);
+  }
+  __syncthreads();
+  const bool here = qr_bar_wait(qr_smem(&bar), 0, qr_wait_limit());
+  if (!__syncthreads_and(here) && threadIdx.x == 0) info[0] = TNC_ERR_TIMEOUT;
+}
+int qr_wait_selftest(int* info, cudaStream_t st) {
+  qr_selftest_kernel<<<1, 64, 0, st>>>(info);
+  return launch_status(1);
+}
+
 }  // namespace tnc
 
 using namespace tnc;

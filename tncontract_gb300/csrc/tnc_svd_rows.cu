@@ -1313,7 +1313,7 @@ extern "C" int tnc_set_spin_limit(long long polls) {
 }
 
 extern "C" int tnc_wait_selftest(int kind, void* work, size_t work_bytes, int* info, void* stream) {
-  if (kind < 0 || kind > 3 || !work || !info || work_bytes < 256) return TNC_ERR_ARG;
+  if (kind < 0 || kind > 4 || !work || !info || work_bytes < 256) return TNC_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   char* w = (char*)work;
   SyncWords* sw = (SyncWords*)w;
@@ -1321,6 +1321,7 @@ extern "C" int tnc_wait_selftest(int kind, void* work, size_t work_bytes, int* i
   int* flag = (int*)(w + 128);
   if (cudaMemsetAsync(work, 0, 256, st) != cudaSuccess) return TNC_ERR_CUDA;
   if (cudaMemsetAsync(info, 0, sizeof(int), st) != cudaSuccess) return TNC_ERR_CUDA;
+  if (kind == 4) return qr_wait_selftest(info, st);
   if (kind == 3) return j32_wait_selftest(ver, sw, info, st);
   wait_selftest_kernel<<<1, 64, 0, st>>>(kind, sw, ver, flag, info);
   return launch_status(1);
