@@ -47,8 +47,9 @@ __device__ __forceinline__ Rot<T> make_rot_ieee(typename traits<T>::real a, type
 // c = 1 / sqrt(1 + |g|^2 w^2).  w may carry the hardware estimates' error (the
 // angle is off by 1e-7 of itself, and the next sweep sees that), c may not: a
 // rotation with a biased c^2 + s^2 drifts the norms.  c is the estimate y of
-// 1 / sqrt(q) and one step with the residual 1 - q y^2 from fused products, whose
-// last operation rounds to nearest, so its error is unbiased and half an ulp.
+// 1 / sqrt(q) and one step of Newton's method for y^-2 = q, y + y (1 - q y^2) / 2
+// (q y rounded, the residual and the last operation fused): below an ulp off, its
+// mean about zero.
 // Operands whose squares or products leave the comfortable FP32 range take the
 // IEEE formula.
 __device__ __forceinline__ float fast_rsqrt(float x) {
