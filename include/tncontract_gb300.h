@@ -407,9 +407,10 @@ int tnc_gather_rows(int dtype, const void *src, int64_t L, const int64_t *order,
  * [3o+1] += calls, [3o+2] += the op's fixed algorithmic flops (for op 3 the
  * flops the FP64 Jacobi executed: 14 n^2 L per rotating sweep and 4 n^2 L for
  * the last, checking one, n rows of length L, complex; a third of that
- * real; for TNC_CORE_DF the FP32 operations of the double-float Jacobi:
- * 44 n^2 L per rotating sweep and 24 n^2 L for the checking one, complex;
- * 15 and 6 real).  Returns TNC_ERR_ARG for a zero state, TNC_ERR_NONFINITE for
+ * real; for TNC_CORE_DF the FP32 operations: 24 n^2 L a Gram matrix and
+ * 48 n^2 L a rotation of all rows at once, complex, 6 and 12 real; and where the
+ * double-float Jacobi ran after them 44 n^2 L per rotating sweep and 24 n^2 L
+ * for the checking one, complex; 15 and 6 real).  Returns TNC_ERR_ARG for a zero state, TNC_ERR_NONFINITE for
  * one whose norm is not finite. */
 enum { TNC_CORE_STORAGE = 0, TNC_CORE_FP64 = 1, TNC_CORE_DF = 2 };
 int tnc_sweep_workspace_size(int dtype, int n_sites, int64_t d,

@@ -196,4 +196,15 @@ template <typename T>
 int qr_qt(int64_t fm, int64_t fn, const T* A, int adjoint, bool want_qt, T* R, void* work, size_t wb, T* tf, int* info,
           cudaStream_t st, T** qt);
 
+// What the whole-matrix steps of tnc_svd_rows_df did, from a host copy of their state
+// (kFinishStateBytes at that offset of its workspace; offset 0: the size takes none):
+// Gram matrices and rotations of all rows, and whether the Jacobi ran after them.
+constexpr size_t kFinishStateBytes = 64;
+struct FinishWork {
+  int grams, rotations;
+  bool jacobi;
+};
+size_t finish_state_offset(int dtype, int64_t m);
+FinishWork finish_work(const void* state, double tol);
+
 }  // namespace tnc

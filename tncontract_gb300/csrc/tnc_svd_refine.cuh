@@ -42,7 +42,7 @@ struct RefineState {
 // Whether a step before `upto` found nothing to do.  Without J (accept >= 0), also
 // whether one took an F below `accept`; a hard one is the last then, and the steps
 // after it have not run.
-__device__ __forceinline__ bool refine_done(const RefineState* st, int upto, float accept = -1.f) {
+__host__ __device__ __forceinline__ bool refine_done(const RefineState* st, int upto, float accept = -1.f) {
   for (int s = 0; s < upto; ++s) {
     if (st[s].rot == 0 && st[s].unit == 0) return true;
     if (accept >= 0.f && st[s].hard) return false;
@@ -51,13 +51,13 @@ __device__ __forceinline__ bool refine_done(const RefineState* st, int upto, flo
   return false;
 }
 // The same from inside step `step`, after its test.
-__device__ __forceinline__ bool refine_idle(const RefineState* st, int step, float accept = -1.f) {
+__host__ __device__ __forceinline__ bool refine_idle(const RefineState* st, int step, float accept = -1.f) {
   return refine_done(st, step, accept) || (st[step].rot == 0 && st[step].unit == 0);
 }
 // A step with pairs that it cannot rotate leaves them to the FP64 Jacobi: the
 // steps after it make J unitary and rotate nothing; without J such a step does
 // nothing and is the last.
-__device__ __forceinline__ bool refine_hard(const RefineState* st, int upto) {
+__host__ __device__ __forceinline__ bool refine_hard(const RefineState* st, int upto) {
   for (int s = 0; s < upto; ++s)
     if (st[s].hard) return true;
   return false;

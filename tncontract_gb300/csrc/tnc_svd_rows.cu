@@ -1136,6 +1136,24 @@ static bool df_refine_fits(int64_t nr, size_t es) {
   return nr >= kDfRefineMin && nr <= 1024 && 8 * (size_t)nr * (es / 2) <= 48 * 1024;
 }
 
+static float df_accept(double tol) { return tol >= 1e-8 ? (float)kDfStopTol : 0.f; }
+
+size_t finish_state_offset(int dtype, int64_t m) {
+  const size_t es = dtype == TNC_C64 ? 16 : 8;
+  return df_refine_fits(m, es) ? rows_layout(m, sizeof(double)).total + df_refine_layout(m, es).state : 0;
+}
+static_assert((kDfSteps + 1) * sizeof(RefineState) == kFinishStateBytes, "what callers copy");
+FinishWork finish_work(const void* state, double tol) {
+  const RefineState* st = (const RefineState*)state;
+  const float accept = df_accept(tol);
+  FinishWork w = {0, 0, !refine_done(st, kDfSteps + 1, accept)};
+  for (int s = 0; s <= kDfSteps; ++s) {  // as the kernels decide whether to run
+    w.grams += !(refine_done(st, s, accept) || refine_hard(st, s));
+    if (s < kDfSteps) w.rotations += !(refine_idle(st, s, accept) || refine_hard(st, s + 1));
+  }
+  return w;
+}
+
 // The finish of single-precision rows in double-float: A (m x n, m <= n,
 // FP32 or complex64) -> W (m x n, FP64 / complex128 elements), S (FP64), order.
 template <typename Tin, typename Tdf, typename Tout>
@@ -1176,7 +1194,7 @@ static int svd_rows_df_impl(int64_t m, int64_t n, const Tin* A, void* Wv, double
     unsigned* large = (unsigned*)(x + X.large);
     RefineState* rs = (RefineState*)(x + X.state);
     const double* f2 = frob2 + 1;  // of the scaled rows
-    accept = tol >= 1e-8 ? (float)kDfStopTol : 0.f;
+    accept = df_accept(tol);
     const double eps = traits<Tdf>::eps;
     const int64_t keep = nkeep < nr ? (nkeep + 7) / 8 * 8 : nr;  // whole half-blocks, as below
     const int64_t tiles = (nr + kDfTile - 1) / kDfTile;

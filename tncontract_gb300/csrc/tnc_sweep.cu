@@ -482,16 +482,26 @@ int sweep_impl(int dt, int n_sites, int64_t d, const void* const* sites, const i
         int hinfo[4] = {0, 0, 0, 0};
         if (cudaMemcpyAsync(hinfo, B.info, sizeof(hinfo), cudaMemcpyDeviceToHost, st) != cudaSuccess)
           return TNC_ERR_CUDA;
+        alignas(8) char steps[kFinishStateBytes] = {};
+        const size_t steps_at = prof.ok && P.core_df ? finish_state_offset(dt, kmin) : 0;
+        if (steps_at &&
+            cudaMemcpyAsync(steps, (char*)B.fact + steps_at, kFinishStateBytes, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+          return TNC_ERR_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return TNC_ERR_CUDA;
         if (hinfo[0]) return hinfo[0];
-        {  // executed arithmetic: rotating sweeps, then the checking one unless the finish
-           // stopped without it (info[3]) (pairs of kept rows); FP64 flops, or the FP32
-           // operations of the double-float finish
+        {  // executed arithmetic: whole-matrix steps (all rows, kept or not), then the Jacobi's rotating sweeps and
+           // the checking one unless it stopped without it (info[3]) (pairs of kept rows); FP64 flops, or the
+           // FP32 operations of the double-float finish
           const double pairs = (double)kmin * kmin - (double)(kmin - nkeep) * (kmin - nkeep);
           const double nn = pairs * m, sweeps = hinfo[1] > 0 ? hinfo[1] : 1;
           const double rotating = hinfo[3] ? sweeps : sweeps - 1.0, checking = hinfo[3] ? 0.0 : 1.0;
-          if (P.core_df) fp64_flops += (rotating * (cplx ? 44.0 : 15.0) + checking * (cplx ? 24.0 : 6.0)) * nn;
-          else fp64_flops += (rotating * 14.0 + checking * 4.0) * nn / (cplx ? 1.0 : 3.0);
+          const FinishWork w = steps_at ? finish_work(steps, tol64) : FinishWork{0, 0, true};
+          if (P.core_df) {
+            fp64_flops += (w.grams * (cplx ? 24.0 : 6.0) + w.rotations * (cplx ? 48.0 : 12.0)) * kmin * kmin * m;
+            if (w.jacobi) fp64_flops += (rotating * (cplx ? 44.0 : 15.0) + checking * (cplx ? 24.0 : 6.0)) * nn;
+          } else {
+            fp64_flops += (rotating * 14.0 + checking * 4.0) * nn / (cplx ? 1.0 : 3.0);
+          }
         }
         // the FP64 decision must retain only rows the FP64 stage finished
         const int64_t k64 = rank_rule<double>(sd, chi, threshold, eps);
