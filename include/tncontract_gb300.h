@@ -174,10 +174,11 @@ typedef struct {
 int tnc_gemm_grouped(int dtype, int count, const tnc_gemm_problem *problems,
                      void *stream);
 
-/* tnc_gemm on the tcgen05 tensor cores for F32 / C64: TF32 split products
- * (hi*hi + hi*lo + lo*hi, FP32 accumulation in tensor memory) give
- * FP32-class accuracy; operands are split into planar K-major TF32 planes in
- * the workspace and streamed by TMA.  Same operands and ops as tnc_gemm;
+/* tnc_gemm on the tcgen05 tensor cores for F32 / C64: every row of op(A) and
+ * column of op(B) is scaled by a power of two and cut into three 8-bit digits,
+ * exact in BF16, whose products' sums in tensor memory are exact: FP32-class
+ * accuracy without a bias.  The digit planes lie K-major in the workspace and
+ * are streamed by TMA.  Same operands and ops as tnc_gemm;
  * batch <= 65535.  The product np.tensordot performs (tensor.py:735) for
  * single-precision tensors, and the absorption products of the sweep. */
 int tnc_gemm_tc_workspace_size(int dtype, int64_t m, int64_t n, int64_t k,
@@ -287,7 +288,7 @@ int tnc_svd_noalloc(int dtype, int64_t m, int64_t n, const void *A,
  * run on its 16 x 16 Gram matrix and are applied to the rows as one 16 x 16
  * product (same rotations, GEMM-shaped work; 8-row half-blocks, the
  * row-by-row kernel where fewer rows need smaller ones).
- * max(m,n) <= 1024 (512 for F64/C128).  info as for tnc_svd. */
+ * max(m,n) <= 1024 (512 for C128).  info as for tnc_svd. */
 enum { TNC_ROWS_GRAM = 32 };
 int tnc_svd_rows_workspace_size(int dtype, int64_t m, int64_t n, size_t *bytes);
 int tnc_svd_rows(int dtype, int64_t m, int64_t n, const void *A, void *W,

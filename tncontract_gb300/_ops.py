@@ -81,7 +81,9 @@ def _arr(ctype, seq):
 
 # When set to a dict, every C-ABI call is bracketed by CUDA events on the
 # current stream: PROFILE[name] -> list of (start, end, algorithmic flops).
-# PROFILE_ONLY (a set of names) restricts the bracketing to those calls.
+# PROFILE_ONLY (a set of names) restricts the bracketing to those calls.  While it is
+# set, engine.compress, inner_product and fidelity run op by op, so that each op shows;
+# otherwise they are one native call of the same algorithm.
 PROFILE = None
 PROFILE_ONLY = None
 
@@ -407,7 +409,7 @@ def dot_device(x, y, conj_x=False):
 
 
 # FP32-class GEMMs at least this large (m*n*k*batch) run on the tcgen05
-# tensor-core kernel (TF32 split products); smaller ones and FP64 use the
+# tensor-core kernel (products of BF16 digits); smaller ones and FP64 use the
 # CUDA-core kernel.
 USE_TC = True
 TC_MIN_WORK = 1 << 21

@@ -490,12 +490,12 @@ jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double t
 // O(h^2 L) products are GEMM-shaped (FMA-pipe bound, not latency bound).
 // Single-precision rows (FP32, complex64), half-blocks of 8 rows, 256
 // threads, both tiles of the product in shared memory with a row stride
-// padded so the 16 rows fall in distinct banks.  Measured against the
-// row-by-row kernel on a 512 x 512 complex64 core (same 11-12 sweeps): 14.5
-// against 9.7 ms -- the products are 2.7x the row-by-row kernel's FMAs (Gram
-// plus application against inner products plus updates) and every task
-// still moves its rows through L2, so it is an option (TNC_ROWS_GRAM, an
-// autotuner candidate), not the default.
+// padded so the 16 rows fall in distinct banks.  The products are 2.7x the
+// FMAs of rotating row by row (Gram plus application against inner products
+// plus updates) and every task still moves its rows through L2: 14.5 ms for a
+// 512 x 512 complex64 core, where the single-precision kernel
+// (tnc_jacobi32.cuh) takes 5.2.  It wins none of the tuning table's 86
+// buckets and runs on request only (TNC_ROWS_GRAM).
 constexpr int kGramH = 8;
 constexpr int kGramRows = 2 * kGramH;  // rows of a task
 constexpr int kGramWarps = 8;          // 256 threads = one per Gram entry
@@ -957,9 +957,7 @@ static int svd_rows_impl(int64_t m, int64_t n, const T* A, T* W, typename traits
     if (block_rows == 2 || block_rows == 4 || block_rows == 8) h = block_rows;
     int rc;
     if constexpr (sizeof(R) == 4) {
-      // single-precision rows: the Gram-form block update on request (measured
-      // slower than the row-by-row kernel; it executes 2.7x the FMAs and keeps
-      // the per-task L2 round trip)
+      // single-precision rows: the Gram-form block update on request only
       if (block_rows == TNC_ROWS_GRAM && (nr > kGramH / 2) && gram_smem_bytes<T>(L) <= kMaxHalfBlockBytes)
         rc = launch_gram<T>(W, nr, L, max_sweeps, tol, frob2, counters, sw, info, nkeep, st, stop_tol);
       else

@@ -568,7 +568,8 @@ def compress(sites, chi, threshold=1e-15, stats=None, log_norm_in=0.0, fold_norm
     folded into the first site when it is representable (log_norm is then 0).
     Device sites of one dtype and physical dimension run as one native call
     (``tnc_sweep_compress``), so that instances on concurrent threads do not
-    contend for the interpreter at every operation."""
+    contend for the interpreter at every operation; while ``_ops.PROFILE`` is
+    set they run op by op."""
     P = [s for s in sites]
     if _native_chain(P):
         P, log_norm = _compress_native(P, chi, threshold, stats, log_norm_in)
@@ -816,9 +817,11 @@ def inner_product(bra, ket, conj_bra=True, log_scale=False):
     """<bra|ket> of two (phys, left, right) site lists on the device, by the
     left-to-right environment sweep of ladder_contract (onedim_core.py:1587-1607).
     Returns a Python complex; with ``log_scale`` every site and the
-    environment after every site are rescaled to unit norm and (mantissa,
-    natural log of the scale) is returned, for states whose overlaps leave
-    the FP64 range."""
+    environment after every site are rescaled (by powers of two in the native
+    call, to unit norm op by op) and (mantissa, natural log of the scale) is
+    returned, for states whose overlaps leave the FP64 range.  Closed chains
+    of device sites are one native call (``tnc_mps_overlap``), op by op while
+    ``_ops.PROFILE`` is set."""
     dt = torch.promote_types(bra[0].dtype, ket[0].dtype)
     n = min(len(bra), len(ket))
     if _native_overlap(bra[:n], ket[:n]):
