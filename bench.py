@@ -479,9 +479,9 @@ def run_ours(args):
     df_op = name == FINISH_OP["df"]
     if df_op:
         pipe = ("FP32 (double-float operations)", round(FP32_OPS_T, 1))
-        fp_note = ("CUDA-core arithmetic; achieved counts the FP32 operations the double-float Jacobi executed "
-                   "(44 n^2 L per rotating sweep and 24 n^2 L for the checking one: 12 per Dot2 step, 7 per "
-                   "compensated update), frac is against the measured bf16 tensor peak, frac_of_pipe_nominal "
+        fp_note = ("CUDA-core arithmetic; achieved counts the FP32 operations the finish executed (24 n^2 L a Gram "
+                   "matrix and 48 n^2 L a rotation of all rows at once; where the double-float Jacobi ran too, 44 "
+                   "n^2 L per rotating sweep and 24 n^2 L for the checking one; complex), frac is against the measured bf16 tensor peak, frac_of_pipe_nominal "
                    "against the FP32 pipe's operation rate (152 SMs x 128 lanes x 2.07 GHz = %.1f T ops/s)"
                    % FP32_OPS_T)
     else:

@@ -492,9 +492,9 @@ jacobi_block_kernel(T* W, int64_t nr, int64_t L, int h, int max_sweeps, double t
 // threads, both tiles of the product in shared memory with a row stride
 // padded so the 16 rows fall in distinct banks.  The products are 2.7x the
 // FMAs of rotating row by row (Gram plus application against inner products
-// plus updates) and every task still moves its rows through L2: 14.5 ms for a
-// 512 x 512 complex64 core, where the single-precision kernel
-// (tnc_jacobi32.cuh) takes 5.2.  It wins none of the tuning table's 86
+// plus updates) and every task still moves its rows through L2: 15.5 ms for a
+// Gaussian 512 x 512 complex64 core, where the single-precision kernel
+// (tnc_jacobi32.cuh) takes 6.6.  It wins none of the tuning table's 86
 // buckets and runs on request only (TNC_ROWS_GRAM).
 constexpr int kGramH = 8;
 constexpr int kGramRows = 2 * kGramH;  // rows of a task
